@@ -689,6 +689,8 @@ int run_transport(ptg_handle* h, const Transport& T) {
       int tbps = 0;
       CU(ptg::tail_occupancy(block, smem, &tbps, T.mode, h->g32.has_ext != 0, h->g32.stage_smem != 0));
       tgrid = h->num_sms * (tbps < 1 ? 1 : tbps);
+      if (T.mode == ptg::MODE_FORWARD)
+        r.grace_steps = ptg::grace_passes(norder * T.np_local, (int64_t)tgrid * (block / 32));
     }
     const bool work = (T.mode == ptg::MODE_ADJOINT || T.mode == ptg::MODE_TRACE) ? T.alist_n > 0
                                                                                    : r.nchunk > 0;

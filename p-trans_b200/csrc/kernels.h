@@ -138,6 +138,9 @@ struct RunF32 {
                                  live phonons moves them to the tail list, where
                                  each gets a warp of its own that advances it 32
                                  flights a round (0: off)                         */
+  int32_t grace_steps;        /* passes a warp's long-MFP phonons (no fast path) get
+                                 after the queue is dry before they go to the list
+                                 too (grace_passes)                               */
   float4* tail;               /* tail list: kTailUnits float4 per phonon           */
   int32_t tail_cap;           /* its capacity in phonons                           */
   int32_t* tail_order;        /* the tail phase takes list slots in this order
@@ -196,6 +199,26 @@ constexpr int kDefaultFastStepsPlain = 4;
 constexpr int kDefaultFastStepsExt = 20;
 inline int default_fast_steps(const GeoF32& g) {
   return g.has_ext ? kDefaultFastStepsExt : kDefaultFastStepsPlain;
+}
+
+/* Passes (one full flight per lane each) that the drain phase gives its
+   long-MFP phonons once the queue is dry, before it hands them to the tail
+   phase like the diffusive ones.  Most of them leave the box within a few
+   dozen flights, most flights ending at a surface, and a round of the tail
+   phase then advances one phonon by a single flight: a warp that takes them
+   one after the other needs about 2000 cycles a flight, a drain pass about
+   3500 for 32 of them.  So they stay where the tail phase would get many per
+   warp (120 000 phonons, MFP 150 nm in a 200 nm cube: 432 -> 209 us; 3.6e6
+   ballistic ones among spheres: 1107 -> 710 us) and go at once where it gets
+   few (2400 phonons in a porous film, MFP 100 nm: 229 us against 248 with 16
+   passes, 260 with 32).  The two are equal at 4 to 8 phonons per warp, and
+   16 and 32 passes at about 40; behind a BVH too (64 spheres and 16 capped
+   cylinders, 2e5 phonons, MFP 150 nm: 6.0 -> 3.1 ms).  The adjoint's two
+   passes hand over at once: their tail is a few long trajectories, which the
+   passes only delay (9.9 ms against 10.5 with 16). */
+inline int grace_passes(int64_t samples, int64_t tail_warps) {
+  if (samples < 6 * tail_warps) return 0;
+  return samples < 40 * tail_warps ? 16 : 32;
 }
 
 /* Replays are split in this many interleaved batches (sample % kAdjBatches)

@@ -1222,6 +1222,7 @@ __global__ void __launch_bounds__(kBlock,
   int ch_task = -1, ch_next = 0, ch_left = 0;
   bool queue_done = false;
   bool tail_full = false;  /* the tail list refused this warp: stop asking */
+  int grace = r.grace_steps;  /* passes its long-MFP phonons get before a hand-over */
 
   /* lane state */
   bool alive = false;
@@ -1411,12 +1412,15 @@ __global__ void __launch_bounds__(kBlock,
       if (queue_done) break;
       continue;
     }
-    /* ---- drain phase, queue dry: live phonons go to the tail list (the
-       diffusive ones and, as well, the few long-MFP ones, which would
-       otherwise hold their warp, and the drain launch, to the end) */
+    /* ---- drain phase, queue dry: live phonons go to the tail list: the
+       diffusive ones at once, the long-MFP ones after the passes in which
+       most of them end (grace_passes), lest the last few hold their warp,
+       and the drain launch, to the end */
     if (PH == PH_DRAIN && !BATCH && MODE != MODE_TRACE && queue_done && r.coop_lanes > 0 &&
         !tail_full && __popc(__ballot_sync(FULL, alive)) <= r.coop_lanes) {
-      const unsigned mw = __ballot_sync(FULL, alive);
+      const unsigned mw =
+          __ballot_sync(FULL, alive && (lam < flmax || r.fast_steps <= 0 || grace == 0));
+      grace -= grace > 0 ? 1 : 0;
       if (mw) {
         /* a slot is reserved from one counter of all requests (queue[5])
            before the phonon picks its end of the list: the phonons admitted

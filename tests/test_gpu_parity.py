@@ -246,6 +246,29 @@ def test_cooperative_tail_takes_the_same_trajectories(name, cap):
 
 
 
+@pytest.mark.parametrize("name", ["film_periodic", "brick_tris", "capped"])
+@pytest.mark.parametrize("np_", [3, 355, 356, 2400])
+@pytest.mark.parametrize("cap", [0, 17])
+def test_long_mfp_phonons_end_alike_in_either_phase(name, np_, cap):
+    """Phonons without a fast path stay in the drain phase for some passes
+    once the queue is dry, or go to the tail phase at once, by how many of
+    them each tail warp would get (kernels.h: grace_passes; 40 tasks, so 355
+    and 356 particles lie on either side of its line at 2368 warps): counts,
+    lost counts and flight totals equal the one-lane path's."""
+    m = geometries()[name]
+    spec = synth.spectrum(10, seed=8)
+    gb = A.GeomBuf(m)
+    run = A.make_run(kind_mfp=A.MFP_GRID, nangle=5, np_=np_, seed=31, mfp_grid=[90.0], precision=A.PREC_FP32)
+    got = []
+    for flags in (2, 0):
+        with A.Handle(gb.view, spec, max_flights=cap, tune_flags=flags) as h:
+            k = h.kappa(run, want_counts=True)
+            st = h.stats()
+            got.append((k["counts"], k["lost"], st["flights"], st["max_traj_flights"]))
+    np.testing.assert_array_equal(got[1][0], got[0][0])
+    assert got[1][1:] == got[0][1:]
+
+
 def _many_spheres(n=40, l=400.0, seed=0):
     rng = np.random.default_rng(seed)
     c, r = [], []

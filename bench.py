@@ -40,6 +40,7 @@ METRIC = "phonon free-flights/s on 1 B200, batched FP32 vs plain FP64, at ≤1% 
 UNIT = "free-flights/s"
 BYTES_PER_FLIGHT = 64       # FP32 SoA state: 32 B read + 32 B written per free flight
 FLOPS_PER_FLIGHT_C2 = 702   # 6 box quads x 95 + 3 z-cylinders x 24 + 60 per event
+PLAIN_FP64 = 8              # ptg_options.tune_flags bit 3: the plain kernel for FP64 runs
 FP32_PEAK_NOMINAL = 148 * 128 * 2 * 1.965e9 / 1e12   # TFLOP/s, 148 SMs x 128 lanes x FMA
 
 
@@ -379,7 +380,7 @@ def run_c5(args):
     idx = list(range(0, 256, max(1, 256 // args.fp64_subset)))[: args.fp64_subset]
     f64_ms = f64_fl = 0.0
     for i in idx:
-        with A.Handle(bufs[i].view, spec) as h:
+        with A.Handle(bufs[i].view, spec, tune_flags=PLAIN_FP64) as h:
             r64 = A.make_run(kind_mfp=A.MFP_PER_MODE, nangle=11, np_=nps[i], seed=i, precision=A.PREC_FP64,
                              temperature=300.0, nbins=64, bin_omega=(0.0, 15.0 * 2 * math.pi * 1e12))
             h.kappa(r64)
@@ -479,7 +480,7 @@ def run_structure(args):
     else:
         sample = f"all modes, {np64} particles per (mode, angle) task"
         vb, _, _, _, _ = timed({}, np64, A.PREC_FP32, 1, 1)
-    v64, ms64, fl64, _, _ = timed({}, np64, A.PREC_FP64, 1, 0)
+    v64, ms64, fl64, _, _ = timed({"tune_flags": PLAIN_FP64}, np64, A.PREC_FP64, 1, 0)
     line["plain_fp64"] = {"value": v64, "unit": UNIT, "sample": sample, "ms": ms64,
                           "fp32_same_sample": vb, "speedup_fp32_over_fp64_same_sample": vb / v64}
     print(json.dumps(line))
@@ -506,7 +507,9 @@ def run_c1(args):
     flush = torch.empty(256 * 1024 * 1024 // 4, dtype=torch.float32, device="cuda:0")
     res = {}
     with A.Handle(gb.view, spec) as h:
-        for name, prec in (("fp64", A.PREC_FP64), ("fp32", A.PREC_FP32)):
+        for name, prec, flags in (("plain", A.PREC_FP64, PLAIN_FP64), ("fp64", A.PREC_FP64, 0),
+                                  ("fp32", A.PREC_FP32, 0)):
+            h.set_options(tune_flags=flags)
             run = A.make_run(kind_mfp=A.MFP_PER_MODE, nangle=11, np_=5, seed=0, precision=prec, **bins)
             for _ in range(args.warmup):
                 h.kappa(run)
@@ -529,7 +532,7 @@ def run_c1(args):
         raise RuntimeError(p.stderr[-2000:])
     orc = json.loads(p.stdout.strip().splitlines()[-1])
     counts_equal = orc["counts_sha"] == _sha(res["fp64"]["counts"])
-    line = {"metric": "phonon free-flights/s, C1 square nanowire (plain method, FP64)",
+    line = {"metric": "phonon free-flights/s, C1 square nanowire, FP64",
             "value": res["fp64"]["value"], "unit": UNIT, "n_gpus": 1, "steps": args.steps,
             "warmup": args.warmup, "ms_per_step": res["fp64"]["ms_per_step"], "higher_is_better": True,
             "dtype": "f64", "data": "synthetic",
@@ -538,6 +541,8 @@ def run_c1(args):
                        "l2": "256 MiB written between timed steps"},
             "flights_per_step": res["fp64"]["flights"], "kappa": res["fp64"]["kappa"],
             "kappa_stderr": res["fp64"]["kappa_stderr"],
+            "plain_fp64": {"value": res["plain"]["value"], "unit": UNIT, "ms_per_step": res["plain"]["ms_per_step"],
+                           "counts_equal": bool(np.array_equal(res["plain"]["counts"], res["fp64"]["counts"]))},
             "persistent_fp32": {"value": res["fp32"]["value"], "unit": UNIT,
                                 "ms_per_step": res["fp32"]["ms_per_step"], "kappa": res["fp32"]["kappa"],
                                 "kappa_stderr": res["fp32"]["kappa_stderr"]},
@@ -607,8 +612,10 @@ def run_c3(args):
         t0 = time.perf_counter()
         adj = h.adjoint(run)
         adj_s = time.perf_counter() - t0
+        h.set_options(tune_flags=PLAIN_FP64)
         h.kappa(A.make_run(kind_mfp=A.MFP_PER_MODE, nangle=11, np_=2, seed=12345, precision=A.PREC_FP64, **bins))
         s64 = h.stats()
+        h.set_options(tune_flags=0)
         h.kappa(A.make_run(kind_mfp=A.MFP_PER_MODE, nangle=11, np_=2, seed=12345, precision=A.PREC_FP32, **bins))
         s32 = h.stats()
     v = fl / (ms * 1e-3)
@@ -755,6 +762,7 @@ def main():
 
     # plain FP64 one-phonon-per-thread comparator on the same workload
     run64 = make_run(pkg, spec, args.np * world, rank, world, A.PREC_FP64)
+    h.set_options(tune_flags=PLAIN_FP64)
     if args.fp64_steps > 0:
         h.kappa(run64)
     barrier()
@@ -766,6 +774,7 @@ def main():
         s64 = h.stats()
         f64_ms += s64["kernel_ms"] + s64["reduce_ms"]
         f64_flights += s64["flights"]
+    h.set_options(tune_flags=0)
     barrier()
     f64_ms = maxall(f64_ms)
     f64_flights = sumall(f64_flights)

@@ -78,7 +78,8 @@ extern "C" {
 #define PTG_FACE_PERIODIC   1
 /* kernel selection */
 #define PTG_PREC_FP32       0   /* persistent FP32 kernel, FP64 tallies       */
-#define PTG_PREC_FP64       1   /* plain FP64 one-phonon-per-thread kernel    */
+#define PTG_PREC_FP64       1   /* FP64 throughout: the CPU solver's          */
+                                /* trajectories, bit for bit                  */
 
 /* material_to codes in ptg_model.surf_material_to */
 #define PTG_MATERIAL_INTERNAL  0   /* "Internal": connects to the fill grain */
@@ -196,6 +197,9 @@ typedef struct ptg_options {
                             /*          copy is not issued, so its bounded wait */
                             /*          runs out and the call returns           */
                             /*          PTG_ERR_TIMEOUT                         */
+                            /*   bit 3: FP64 runs with the plain kernel, one    */
+                            /*          phonon per thread (the comparator; the  */
+                            /*          same trajectories)                      */
   int32_t fast_steps;       /* fast p-p flights per iteration before a warp     */
                             /* goes on only while half its lanes still can      */
                             /* (at most 4x; 0 = 4 for structures without BVH or */
@@ -560,7 +564,7 @@ int ptg_autotune(ptg_handle* h, const ptg_run* run, int32_t reps, ptg_options* b
 int ptg_transmission_noalloc(ptg_handle* h, double mfp_nm, int32_t nangle, int64_t np,
                              int32_t rank, int32_t nranks, uint64_t seed, double* transmit);
 
-/* Debug / replay: runs the FP64 kernel for one task and writes, per particle,
+/* Debug / replay: runs the plain FP64 kernel for one task and writes, per particle,
    the exit side (0 lost, 1 x-, 2 x+) and the number of free flights. */
 int ptg_replay_task(ptg_handle* h, const ptg_run* run, int64_t task,
                     int32_t* end_side, uint32_t* flights, double* final_pos);

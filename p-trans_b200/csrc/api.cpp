@@ -452,6 +452,33 @@ int build_blob(ptg_handle* h) {
   return PTG_OK;
 }
 
+/* Whether grain 0 is the box as setupBoxGrain builds it: six internal
+   rectangles x-, x+, y-, y+, z-, z+ with outward unit normals, the vertices
+   exactly at the corners.  (A caller's own geometry may differ.) */
+bool box_is_axis_aligned(const ptg::GeomSoA& G) {
+  if (G.grain_begin[0] != 0 || G.grain_begin[1] != 6) return false;
+  for (int k = 0; k < 6; ++k) {
+    const int ax = k >> 1;
+    if (G.shape[k] != PTG_SHAPE_POLYGON || G.nvertex[k] != 4 || !G.internal[k]) return false;
+    const double* v = &G.vertex[3 * (size_t)G.vertex_begin[k]];
+    for (int d = 0; d < 3; ++d)
+      if (G.normal[3 * k + d] != (d == ax ? ((k & 1) ? 1.0 : -1.0) : 0.0)) return false;
+    for (int i = 0; i < 5; ++i) {
+      if (v[3 * i + ax] != ((k & 1) ? G.box[ax] : 0.0)) return false;
+      int steps = 0;
+      for (int d = 0; d < 3; ++d) {
+        if (v[3 * i + d] != 0.0 && v[3 * i + d] != G.box[d]) return false;
+        if (i > 0 && v[3 * i + d] != v[3 * (i - 1) + d]) ++steps;
+      }
+      if (i > 0 && steps != 1) return false;
+    }
+    /* opposite corners: a rectangle, not a fold */
+    for (int d = 0; d < 3; ++d)
+      if (d != ax && (v[d] == v[6 + d] || v[3 + d] == v[9 + d])) return false;
+  }
+  return true;
+}
+
 int build_geo64(ptg_handle* h) {
   const ptg::GeomSoA& G = h->geom;
   ptg::Geo64& g = h->g64;
@@ -482,6 +509,7 @@ int build_geo64(ptg_handle* h) {
   g.igrain_fill = G.igrain_fill;
   g.nmaterial = G.nmaterial;
   g.max_omega = h->spec.max_omega;
+  g.box_axis = box_is_axis_aligned(G) ? 1 : 0;
   return PTG_OK;
 }
 
@@ -533,17 +561,85 @@ int run_transport(ptg_handle* h, const Transport& T) {
   CU(cudaMemsetAsync(h->queue.p, 0, sizeof(int) * 8, h->stream));
   const int64_t maxf = h->opt.max_flights > 0 ? h->opt.max_flights : 10000000LL;
   memset(&h->last, 0, sizeof(h->last));
-  if (T.precision == PTG_PREC_FP64) {
-    std::vector<ptg::Task64> t64(ntask);
-    for (int64_t i = 0; i < ntask; ++i) {
-      const ptg::TaskHost& th = (*T.tasks)[i];
-      t64[i] = {th.lambda, th.cth, th.sth, th.omega};
+  const bool fp64 = T.precision == PTG_PREC_FP64;
+  const bool plain = fp64 && (h->opt.tune_flags & 8);
+  /* the task table and the queue order (longest expected trajectories first:
+     ascending MFP) are written to pinned staging and copied without a host
+     wait; the chunk table (task, first local particle, count) is expanded
+     from the order on the device.  The MFP depends on (mode, grid point)
+     only, so those pairs are sorted and every angle's task follows its pair;
+     equal MFPs keep index order. */
+  if (h->h2d_pending) {
+    CU(cudaEventSynchronize(h->h2d_done));
+    h->h2d_pending = false;
+  }
+  const size_t task_bytes = (fp64 ? sizeof(ptg::Task64) : sizeof(float4)) * (size_t)ntask;
+  CU(h->pin_task.ensure(task_bytes > 0 ? task_bytes : 1));
+  CU(h->pin_order.ensure(sizeof(int) * (ntask > 0 ? ntask : 1)));
+  int* order = h->pin_order.as<int>();
+  const int64_t npair = T.npair > 0 ? std::min<int64_t>(ntask, T.npair) : ntask;
+  std::vector<int64_t> pairs;
+  pairs.reserve(npair);
+  for (int64_t i = 0; i < ntask; ++i) {
+    const ptg::TaskHost& th = (*T.tasks)[i];
+    if (fp64) {
+      h->pin_task.as<ptg::Task64>()[i] = {th.lambda, th.cth, th.sth, th.omega};
+    } else {
+      float lam = th.lambda == 1.0e10 ? INFINITY : (float)th.lambda;
+      if (!(th.lambda > 0.0)) lam = 0.0f;
+      h->pin_task.as<float4>()[i] = make_float4(lam, (float)th.cth, (float)th.sth,
+                                                (float)(th.omega / h->spec.max_omega));
     }
-    CU(h->task.ensure(sizeof(ptg::Task64) * ntask));
-    CU(cudaMemcpyAsync(h->task.p, t64.data(), sizeof(ptg::Task64) * ntask, cudaMemcpyHostToDevice,
-                       h->stream));
-    CU(cudaStreamSynchronize(h->stream));  /* t64 is a local buffer */
-    h->last.h2d_bytes += sizeof(ptg::Task64) * ntask;
+    if (i < npair && th.lambda > 0.0) pairs.push_back(i);
+  }
+  std::stable_sort(pairs.begin(), pairs.end(), [&](int64_t a, int64_t b) {
+    return (*T.tasks)[a].lambda < (*T.tasks)[b].lambda;
+  });
+  int64_t norder = 0;
+  const int64_t nrep = npair > 0 ? (ntask + npair - 1) / npair : 0;
+  for (int64_t pi : pairs)
+    for (int64_t k = 0; k < nrep; ++k) {
+      const int64_t t = pi + k * npair;
+      if (t < ntask) order[norder++] = (int)t;
+    }
+  int64_t csz = h->opt.chunk > 0 ? h->opt.chunk : 64;
+  int64_t per_task = T.np_local > 0 ? (T.np_local + csz - 1) / csz : 0;
+  /* FP64 runs take any size: larger chunks past a table of 1 GB */
+  while (fp64 && norder * per_task > (1LL << 26) && per_task > 1) {
+    csz *= 2;
+    per_task = (T.np_local + csz - 1) / csz;
+  }
+  const int64_t nchunk = plain ? 0 : norder * per_task;
+  if (nchunk > 2147483647LL) { h->last_error = "too many chunks"; return PTG_ERR_INVALID; }
+  CU(h->task.ensure(task_bytes));
+  CU(h->order.ensure(sizeof(int) * (norder > 0 ? norder : 1)));
+  CU(h->chunk.ensure(sizeof(int4) * (nchunk + 1)));
+  CU(cudaMemcpyAsync(h->task.p, h->pin_task.p, task_bytes, cudaMemcpyHostToDevice, h->stream));
+  if (norder > 0)
+    CU(cudaMemcpyAsync(h->order.p, order, sizeof(int) * norder, cudaMemcpyHostToDevice, h->stream));
+  CU(cudaEventRecord(h->h2d_done, h->stream));
+  h->h2d_pending = true;
+  /* the timed transport starts here, with the tables resident: the chunk
+     expansion is part of it */
+  CU(cudaEventRecord(h->ev[0], h->stream));
+  if (nchunk > 0)
+    CU(ptg::launch_expand_chunks(h->order.as<const int>(), (int)norder, (int)per_task, (int)csz,
+                                 (int)T.np_local, h->chunk.as<int4>(), h->stream));
+  h->last.h2d_bytes += task_bytes + sizeof(int) * norder;
+  /* scheduling of both persistent kernels.  A lane that loops longer on the
+     fast path holds its warp's other lanes: 16 steps cost 13.6 ms of drain on
+     the thin film against 11.1 ms for 8. */
+  const int rt = h->opt.regen_threshold > 0 ? h->opt.regen_threshold : ptg::kDefaultRegen;
+  const int regen_threshold = rt > 32 ? 32 : rt;
+  const int fast_steps = (h->opt.tune_flags & 1) ? 0 : (h->opt.fast_steps > 0 ? h->opt.fast_steps : ptg::default_fast_steps(h->g32));
+  const double lmin = std::min(h->geom.box[0], std::min(h->geom.box[1], h->geom.box[2]));
+  const float fast_lambda_max = (float)(0.1 * lmin);
+  /* tune_flags bit 1 turns the tail phase off; 0 selects 32 lanes (every
+     diffusive phonon still alive when a warp finds the queue dry) */
+  const int coop_lanes = (h->opt.tune_flags & 2) ? 0 : (h->opt.coop_lanes > 0 ? std::min(h->opt.coop_lanes, 32) : 32);
+  const int bs = h->opt.block_size;
+  const int block = (bs >= 32 && bs <= 256 && bs % 32 == 0) ? bs : 256;
+  if (fp64) {
     ptg::Run64 r;
     memset(&r, 0, sizeof(r));
     r.task = h->task.as<const ptg::Task64>();
@@ -561,69 +657,48 @@ int run_transport(ptg_handle* h, const Transport& T) {
     r.lost = h->lost.as<unsigned long long>();
     r.stats = h->stats.as<unsigned long long>();
     r.replay_task = -1;
-    CU(cudaEventRecord(h->ev[0], h->stream));
-    int grid = 0, block = 0;
-    CU(ptg::launch_plain_fp64(h->g64, r, h->stream, &grid, &block));
+    int grid = 0, pblock = block;
+    h->last.launches = 0;
+    if (plain) {
+      CU(ptg::launch_plain_fp64(h->g64, r, h->stream, &grid, &pblock));
+      h->last.launches = 1;
+    } else if (nchunk > 0) {
+      r.chunk = h->chunk.as<const int4>();
+      r.nchunk = (int32_t)nchunk;
+      r.queue = h->queue.as<int>();
+      r.regen_threshold = regen_threshold;
+      r.fast_steps = fast_steps;
+      r.fast_lambda_max = fast_lambda_max;
+      r.round_lambda_max = (float)lmin;
+      r.coop_lanes = coop_lanes;
+      r.max_flights = std::min<int64_t>(maxf, 4294967295LL);
+      int bps = 0, tbps = 0;
+      CU(ptg::drain64_occupancy(block, &bps));
+      if (h->opt.blocks_per_sm > 0 && h->opt.blocks_per_sm < bps) bps = h->opt.blocks_per_sm;
+      CU(ptg::tail64_occupancy(block, &tbps));
+      grid = h->num_sms * std::max(bps, 1);
+      const int tgrid = h->num_sms * std::max(tbps, 1);
+      if (coop_lanes > 0) {
+        r.tail_cap = grid * block;
+        CU(h->tail.ensure((sizeof(float4) * ptg::kTail64Units + sizeof(int)) * (size_t)r.tail_cap +
+                          sizeof(int) * ptg::kTailOrderExtra));
+        r.tail = h->tail.as<float4>();
+        r.tail_order = reinterpret_cast<int*>(r.tail + (size_t)ptg::kTail64Units * r.tail_cap);
+        r.grace_steps = ptg::grace_passes(norder * T.np_local, (int64_t)tgrid * (block / 32));
+      }
+      CU(ptg::launch_drain64(h->g64, h->g32, r, grid, block, h->stream));
+      if (coop_lanes > 0) {
+        CU(ptg::launch_tail_order(r.tail, ptg::kTail64Units, r.tail_cap, r.queue, r.tail_order,
+                                  h->g32.box[0], h->stream));
+        CU(ptg::launch_tail64(h->g64, h->g32, r, tgrid, block, h->stream));
+      }
+      h->last.launches = coop_lanes > 0 ? 5 : 2;
+    }
     CU(cudaEventRecord(h->ev[1], h->stream));
     h->last.grid = grid;
-    h->last.block = block;
-    h->last.launches = 1;
+    h->last.block = pblock;
     h->fp32_split = false;
   } else {
-    /* the FP32 task table and the queue order (longest expected
-       trajectories first: ascending MFP) are written to pinned staging and
-       copied without a host wait; the chunk table (task, first local
-       particle, count) is expanded from the order on the device.  The MFP
-       depends on (mode, grid point) only, so those pairs are sorted and
-       every angle's task follows its pair; equal MFPs keep index order. */
-    if (h->h2d_pending) {
-      CU(cudaEventSynchronize(h->h2d_done));
-      h->h2d_pending = false;
-    }
-    CU(h->pin_task.ensure(sizeof(float4) * (ntask > 0 ? ntask : 1)));
-    CU(h->pin_order.ensure(sizeof(int) * (ntask > 0 ? ntask : 1)));
-    float4* t32 = h->pin_task.as<float4>();
-    int* order = h->pin_order.as<int>();
-    const int64_t npair = T.npair > 0 ? std::min<int64_t>(ntask, T.npair) : ntask;
-    std::vector<int64_t> pairs;
-    pairs.reserve(npair);
-    for (int64_t i = 0; i < ntask; ++i) {
-      const ptg::TaskHost& th = (*T.tasks)[i];
-      float lam = th.lambda == 1.0e10 ? INFINITY : (float)th.lambda;
-      if (!(th.lambda > 0.0)) lam = 0.0f;
-      t32[i] = make_float4(lam, (float)th.cth, (float)th.sth,
-                           (float)(th.omega / h->spec.max_omega));
-      if (i < npair && th.lambda > 0.0) pairs.push_back(i);
-    }
-    std::stable_sort(pairs.begin(), pairs.end(), [&](int64_t a, int64_t b) {
-      return (*T.tasks)[a].lambda < (*T.tasks)[b].lambda;
-    });
-    int64_t norder = 0;
-    const int64_t nrep = npair > 0 ? (ntask + npair - 1) / npair : 0;
-    for (int64_t pi : pairs)
-      for (int64_t k = 0; k < nrep; ++k) {
-        const int64_t t = pi + k * npair;
-        if (t < ntask) order[norder++] = (int)t;
-      }
-    const int64_t csz = h->opt.chunk > 0 ? h->opt.chunk : 64;
-    const int64_t per_task = T.np_local > 0 ? (T.np_local + csz - 1) / csz : 0;
-    const int64_t nchunk = norder * per_task;
-    if (nchunk > 2147483647LL) { h->last_error = "too many chunks"; return PTG_ERR_INVALID; }
-    CU(h->task.ensure(sizeof(float4) * ntask));
-    CU(h->order.ensure(sizeof(int) * (norder > 0 ? norder : 1)));
-    CU(h->chunk.ensure(sizeof(int4) * (nchunk + 1)));
-    CU(cudaMemcpyAsync(h->task.p, t32, sizeof(float4) * ntask, cudaMemcpyHostToDevice, h->stream));
-    if (norder > 0)
-      CU(cudaMemcpyAsync(h->order.p, order, sizeof(int) * norder, cudaMemcpyHostToDevice, h->stream));
-    CU(cudaEventRecord(h->h2d_done, h->stream));
-    h->h2d_pending = true;
-    /* the timed transport starts here, with the tables resident: the chunk
-       expansion is part of it */
-    CU(cudaEventRecord(h->ev[0], h->stream));
-    if (nchunk > 0)
-      CU(ptg::launch_expand_chunks(h->order.as<const int>(), (int)norder, (int)per_task, (int)csz,
-                                   (int)T.np_local, h->chunk.as<int4>(), h->stream));
-    h->last.h2d_bytes += sizeof(float4) * ntask + sizeof(int) * norder;
     ptg::RunF32 r;
     memset(&r, 0, sizeof(r));
     r.task = h->task.as<const float4>();
@@ -637,18 +712,10 @@ int run_transport(ptg_handle* h, const Transport& T) {
     r.c1 = ((uint32_t)T.stream) << 8;
     r.max_flights = (uint32_t)std::min<int64_t>(maxf, 4294967295LL);
     r.ref_quirks = h->opt.ref_quirks;
-    /* defaults: refill once 2 lanes are idle; at most 8 fast-path flights
-       per lane and iteration (a lane that loops longer holds its warp's
-       other lanes: 16 fast steps cost 13.6 ms of drain on the thin film
-       against 11.1 ms for 8) */
-    int rt = h->opt.regen_threshold > 0 ? h->opt.regen_threshold : ptg::kDefaultRegen;
-    r.regen_threshold = rt > 32 ? 32 : rt;
-    r.fast_steps = (h->opt.tune_flags & 1) ? 0 : (h->opt.fast_steps > 0 ? h->opt.fast_steps : ptg::default_fast_steps(h->g32));
-    const double lmin = std::min(h->geom.box[0], std::min(h->geom.box[1], h->geom.box[2]));
-    r.fast_lambda_max = (float)(0.1 * lmin);
-    /* tune_flags bit 1 turns the tail phase off; 0 selects 32 lanes (every
-       diffusive phonon still alive when a warp finds the queue dry) */
-    r.coop_lanes = (h->opt.tune_flags & 2) ? 0 : (h->opt.coop_lanes > 0 ? std::min(h->opt.coop_lanes, 32) : 32);
+    r.regen_threshold = regen_threshold;
+    r.fast_steps = fast_steps;
+    r.fast_lambda_max = fast_lambda_max;
+    r.coop_lanes = coop_lanes;
     r.stage_test = (h->opt.tune_flags & 4) ? 1 : 0;
     r.counts = h->counts.as<unsigned long long>();
     r.lost = h->lost.as<unsigned long long>();
@@ -665,8 +732,6 @@ int run_transport(ptg_handle* h, const Transport& T) {
     r.trace_npos = T.trace_npos;
     r.trace_end = T.trace_end;
     r.nsurf = h->geom.nsurf();
-    const int bs = h->opt.block_size;
-    const int block = (bs >= 32 && bs <= 256 && bs % 32 == 0) ? bs : 256;
     const size_t smem = ptg::dynamic_smem_bytes(h->g32, h->blob_bytes);
     int bps = 0;
     CU(ptg::persistent_occupancy(block, smem, &bps, T.mode, h->g32.has_ext != 0, h->g32.stage_smem != 0));
@@ -698,7 +763,8 @@ int run_transport(ptg_handle* h, const Transport& T) {
       CU(ptg::launch_persistent_fp32(h->g32, r, grid, block, smem, h->stream, T.mode));
       CU(cudaEventRecord(h->ev[4], h->stream));
       if (tail) {
-        CU(ptg::launch_tail_order(r, h->g32.box[0], h->stream));
+        CU(ptg::launch_tail_order(r.tail, ptg::kTailUnits, r.tail_cap, r.queue, r.tail_order,
+                                  h->g32.box[0], h->stream));
         CU(ptg::launch_tail_fp32(h->g32, r, tgrid, block, smem, h->stream, T.mode));
       }
     }

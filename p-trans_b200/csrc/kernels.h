@@ -37,6 +37,8 @@ struct Geo64 {
   int face_kind[6];
   int kind_grain, ngrain, igrain_fill, nmaterial;
   double max_omega;
+  int box_axis;              /* grain 0 is the six axis-aligned rectangles of
+                                the box, every one internal                 */
 };
 
 /* Per task: lambda [nm] (1e10 ballistic, <= 0 skipped), cos/sin of the
@@ -62,6 +64,17 @@ struct Run64 {
   int* end_side;
   unsigned* flights;
   double* final_pos;
+  /* persistent kernels: the work queue, scheduling and tail list of RunF32
+     (kTail64Units float4 per phonon; queue[4] phonons on the list) */
+  const int4* chunk;
+  int32_t nchunk;
+  int* queue;
+  int32_t regen_threshold, fast_steps, coop_lanes, grace_steps;
+  float fast_lambda_max;
+  float round_lambda_max;    /* phonons with a longer MFP end in the drain     */
+  float4* tail;
+  int32_t tail_cap;
+  int32_t* tail_order;
 };
 
 cudaError_t launch_plain_fp64(const Geo64& g, const Run64& r, cudaStream_t st, int* grid,
@@ -238,7 +251,16 @@ cudaError_t launch_persistent_fp32(const GeoF32& g, const RunF32& r, int grid, i
    remaining walk first.  A memset and two kernels between the drain and the
    tail launch on the same stream; x_len is the box length along x. */
 constexpr int kTailOrderExtra = 256;
-cudaError_t launch_tail_order(const RunF32& r, float x_len, cudaStream_t st);
+cudaError_t launch_tail_order(float4* tail, int units, int tail_cap, const int* queue, int32_t* order,
+                              float x_len, cudaStream_t st);
+/* The FP64 pair: the same queue and list, FP64 flights; the blob of g32 gives
+   the bounds for balls and BVH walks. */
+cudaError_t drain64_occupancy(int block, int* blocks_per_sm);
+cudaError_t tail64_occupancy(int block, int* blocks_per_sm);
+cudaError_t launch_drain64(const Geo64& g, const GeoF32& g32, const Run64& r, int grid, int block,
+                           cudaStream_t st);
+cudaError_t launch_tail64(const Geo64& g, const GeoF32& g32, const Run64& r, int grid, int block,
+                          cudaStream_t st);
 cudaError_t launch_tail_fp32(const GeoF32& g, const RunF32& r, int grid, int block, size_t smem,
                              cudaStream_t st, int mode = MODE_FORWARD);
 cudaError_t tail_occupancy(int block, size_t smem, int* blocks_per_sm, int mode = MODE_FORWARD,
@@ -255,6 +277,11 @@ cudaError_t persistent_batch_occupancy(int block, int* blocks_per_sm, bool bvh,
    ball centre and radii, grain, last surface, task, omega, sample id,
    flight, adjoint terms, second ball). */
 constexpr int kTailUnits = 7;
+/* ... and in the FP64 one: (x, ball centre), (ball radii squared, -, MFP) in
+   FP32, then position, direction, free path and MFP in FP64, (grain and
+   surface last met, order bucket, grain), (task, sample id, flight).  Both
+   layouts hold x at word 0, the MFP at word 7 and the bucket at word 26. */
+constexpr int kTail64Units = 8;
 /* Shared memory for staged BVH nodes when the whole blob is not staged:
    64 KB, the top ten or so levels of the trees, small enough that two
    blocks of the tail kernel (28.5 KB of its own) still fit on an SM. */

@@ -57,6 +57,7 @@
 
 #include <type_traits>
 
+#include "geo_fp32.cuh"
 #include "kernels.h"
 #include "philox.cuh"
 
@@ -64,72 +65,9 @@ namespace ptg {
 
 namespace {
 
-constexpr unsigned FULL = 0xffffffffu;
 constexpr int kBlock = 256;
 constexpr float kTwoPi = 6.28318530717958648f;
 constexpr float kPi = 3.14159265358979323846f;
-
-extern __shared__ float4 sblob[];
-
-#ifdef PT_CHECK
-/* Bounds-checked build: [0] violations, [1] code of the first, [2] its
-   index.  A failed check is recorded and the access is redirected to a
-   valid element; the kernel never traps. */
-__device__ int g_check[3];
-__device__ __noinline__ void check_fail(int code, int index) {
-  if (atomicAdd(&g_check[0], 1) == 0) {
-    g_check[1] = code;
-    g_check[2] = index;
-  }
-}
-#endif
-
-/* Geometry blob accessor: SMEM = true reads the copy staged in shared
-   memory (shared-memory loads), false reads global memory through the
-   read-only path. */
-template <bool SMEM>
-struct Geo {
-  const float4* base;   /* global blob (SMEM = false) */
-  BlobLayout lay;
-  int nstage = 0;       /* SMEM = false: BVH node units staged in shared memory */
-  __device__ __forceinline__ float4 ld(int i) const {
-#ifdef PT_CHECK
-    if ((unsigned)i >= (unsigned)lay.total) { check_fail(1, i); i = 0; }
-#endif
-    if (SMEM) return sblob[i];
-    return __ldg(base + i);
-  }
-  __device__ __forceinline__ int ldi(int unit, int k) const {
-#ifdef PT_CHECK
-    if (k < 0 || (unsigned)(unit + k / 4) >= (unsigned)lay.total) { check_fail(1, unit + k / 4); unit = 0; k = 0; }
-#endif
-    if (SMEM) return reinterpret_cast<const int*>(sblob + unit)[k];
-    return __ldg(reinterpret_cast<const int*>(base + unit) + k);
-  }
-  __device__ __forceinline__ float4 hotA(int s) const { return ld(lay.hot + 2 * s); }
-  __device__ __forceinline__ int4 hotB(int s) const {
-    const float4 v = ld(lay.hot + 2 * s + 1);
-    return make_int4(__float_as_int(v.x), __float_as_int(v.y), __float_as_int(v.z),
-                     __float_as_int(v.w));
-  }
-  __device__ __forceinline__ float4 cold(int s, int i) const { return ld(lay.cold + 3 * s + i); }
-  __device__ __forceinline__ float4 edge(int e) const { return ld(lay.edge + e); }
-  __device__ __forceinline__ int cand_begin(int g) const { return ldi(lay.cand_begin, g); }
-  __device__ __forceinline__ int cand(int k) const { return ldi(lay.cand, k); }
-  __device__ __forceinline__ float4 start(int i) const { return ld(lay.start + i); }
-  __device__ __forceinline__ int bvh_root(int g) const { return ldi(lay.bvh_root, g); }
-  __device__ __forceinline__ float4 node(int i) const {
-    if (!SMEM && i < nstage) return sblob[i];  /* a top level, staged */
-    return ld(lay.bvh_node + i);
-  }
-};
-
-/* Square root from the hardware approximation (relative error ~2^-22). */
-__device__ __forceinline__ float sqrt_approx(float x) {
-  float y;
-  asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
 
 /* sin / cos of 2*pi*u, u in (0,1): hardware approximations on [-pi, pi). */
 __device__ __forceinline__ void sincos2pi(float u, float* s, float* c) {
@@ -356,25 +294,6 @@ __device__ __forceinline__ void test_surface(const G_t& G, int s, float px, floa
   }
 }
 
-/* Entry distance of the ray into a node box (+inf when it misses the box
-   or enters beyond tmax); inverse direction components are finite. */
-__device__ __forceinline__ float box_entry(float4 lo, float4 hi, float px, float py, float pz,
-                                           float ix, float iy, float iz, float tmax, float eps) {
-  const float ax = (lo.x - px) * ix, bx = (hi.x - px) * ix;
-  const float ay = (lo.y - py) * iy, by = (hi.y - py) * iy;
-  const float az = (lo.z - pz) * iz, bz = (hi.z - pz) * iz;
-  const float t0 = fmaxf(fmaxf(fminf(ax, bx), fminf(ay, by)), fminf(az, bz));
-  const float t1 = fminf(fminf(fmaxf(ax, bx), fmaxf(ay, by)), fmaxf(az, bz));
-  return (t0 <= t1 && t1 >= -eps && t0 <= tmax) ? t0 : 3.0e38f;
-}
-
-__device__ __forceinline__ float inv_dir(float d) {
-  return __fdividef(1.0f, fabsf(d) > 1.0e-20f ? d : copysignf(1.0e-20f, d));
-}
-
-/* Traversal depth bound: the builder limits the depth to 30. */
-constexpr int kBvhStack = 32;
-
 /* BVH traversal of a grain (root >= 0): ordered descent, the far child
    pushed with its entry distance and popped only while it can still hold a
    nearer hit.  Nodes entered beyond tcut (the flight's free path) are
@@ -479,140 +398,6 @@ __device__ __forceinline__ void slab_exit(float px, float py, float pz, float dx
   tb = hz ? tz : tb;
   sb = hz ? (dz > 0.0f ? 5 : 4) : sb;
   tb = fmaxf(tb, 0.0f);
-}
-
-/* Lower bound of the distance from p to one candidate surface (planes bound
-   polygons from below, the infinite cylinder bounds the clipped one).  The
-   square roots are the hardware approximation: its relative error (< 2^-22
-   of a distance below the box diagonal) is far inside the 4 eps the callers
-   take off, so the bound stays a bound. */
-template <bool EXT, class G_t>
-__device__ __forceinline__ float surface_lb(const G_t& G, int s, float px, float py, float pz) {
-  const float4 A = G.hotA(s);
-  const int4 B = G.hotB(s);
-  const int type = B.x & 0xff;
-  if (type == REC_POLY) return fabsf(A.w - fmaf(A.x, px, fmaf(A.y, py, A.z * pz)));
-  if (EXT && type == REC_CAP) {
-    /* inside: the nearer of mantle and caps; outside: the larger excess */
-    const float4 E = G.edge(B.y);
-    const float wx = px - A.x, wy = py - A.y, wz = pz - A.z;
-    const float sa = fmaf(wx, E.x, fmaf(wy, E.y, wz * E.z));
-    const float ux = fmaf(-sa, E.x, wx), uy = fmaf(-sa, E.y, wy), uz = fmaf(-sa, E.z, wz);
-    const float er = sqrt_approx(fmaf(ux, ux, fmaf(uy, uy, uz * uz))) - A.w;
-    const float ea = fabsf(sa) - E.w;
-    return (er <= 0.0f && ea <= 0.0f) ? fminf(-er, -ea) : fmaxf(er, ea);
-  }
-  if (type == REC_SPHERE) {
-    const float wx = px - A.x, wy = py - A.y, wz = pz - A.z;
-    return fabsf(sqrt_approx(fmaf(wx, wx, fmaf(wy, wy, wz * wz))) - A.w);
-  }
-  const float wx = px - A.x, wy = py - A.y;
-  return fabsf(sqrt_approx(fmaf(wx, wx, wy * wy)) - A.z);
-}
-
-/* Distance from p to a node box (0 inside; approximate square root, as in
-   surface_lb). */
-__device__ __forceinline__ float box_dist(float4 lo, float4 hi, float px, float py, float pz) {
-  const float ex = fmaxf(fmaxf(lo.x - px, px - hi.x), 0.0f);
-  const float ey = fmaxf(fmaxf(lo.y - py, py - hi.y), 0.0f);
-  const float ez = fmaxf(fmaxf(lo.z - pz, pz - hi.z), 0.0f);
-  return sqrt_approx(fmaf(ex, ex, fmaf(ey, ey, ez * ez)));
-}
-
-/* BVH range query for the safe ball: the smallest lower bound d of the
-   distance from p to a surface of the grain, the surface it belongs to
-   (near) and the smallest bound d2 of every other surface, searched below
-   the initial d (nodes no nearer than the second bound so far are pruned:
-   they cannot change either; a surface's bound is the larger of the
-   distance to its leaf's box and its own plane / quadric bound).  Out of
-   line, like scan_bvh. */
-template <bool EXT, class G_t>
-__device__ __noinline__ float safety_bvh(const G_t& G, int root, float px, float py, float pz,
-                                         float d, float& d2, int& near) {
-  int stk[kBvhStack];
-  float std_[kBvhStack];
-  int sp = 0;
-  int node = root;
-  d2 = d;
-  near = -1;
-  while (true) {
-    const float4 n0 = G.node(2 * node), n1 = G.node(2 * node + 1);
-    const int cnt = __float_as_int(n1.w);
-    const int a = __float_as_int(n0.w);
-    bool descended = false;
-    if (cnt > 0) {
-      const float bd = box_dist(n0, n1, px, py, pz);
-      for (int k = a; k < a + cnt; ++k) {
-        const int sk = G.cand(k);
-        const float e = fmaxf(bd, surface_lb<EXT>(G, sk, px, py, pz));
-        const bool nearer = e < d;
-        d2 = nearer ? d : fminf(d2, e);
-        near = nearer ? sk : near;
-        d = nearer ? e : d;
-      }
-    } else {
-      const float dl = box_dist(G.node(2 * a), G.node(2 * a + 1), px, py, pz);
-      const float dg = box_dist(G.node(2 * a + 2), G.node(2 * a + 3), px, py, pz);
-      const bool lf = dl <= dg;
-      const float dn = lf ? dl : dg, df = lf ? dg : dl;
-      if (dn < d2) {
-        if (df < d2 && sp < kBvhStack) {
-          stk[sp] = lf ? a + 1 : a;
-          std_[sp] = df;
-          ++sp;
-        }
-        node = lf ? a : a + 1;
-        descended = true;
-      }
-    }
-    if (descended) continue;
-    bool found = false;
-    while (sp > 0) {
-      --sp;
-      if (std_[sp] < d2) {
-        node = stk[sp];
-        found = true;
-        break;
-      }
-    }
-    if (!found) break;
-  }
-  return d;
-}
-
-/* Lower bound of the distance from p to every box face and to every
-   candidate surface of the grain, less 4 eps.  A grain with a BVH is
-   searched only within `cap` (the radius the safe ball needs).  dgrain
-   receives the bound over the candidate surfaces alone (the grain ball: a
-   flight inside it needs the box-face test only); for a BVH grain it is
-   searched no farther than the full bound, so it costs no extra nodes. */
-template <bool EXT, class G_t>
-__device__ __forceinline__ float safety(const G_t& G, int grain, float px, float py, float pz,
-                                        float X, float Y, float Z, float eps, float cap,
-                                        float& dgrain, float& dgrain2, int& near) {
-  const float dbox = fminf(fminf(fminf(px, X - px), fminf(py, Y - py)), fminf(pz, Z - pz));
-  float dc = 3.0e38f, dc2 = 3.0e38f;
-  near = -1;
-  if (grain > 0) {
-    const int root = EXT ? G.bvh_root(grain) : -1;
-    if (root < 0) {
-      /* the nearest candidate and the bound of all the others */
-      const int kb = G.cand_begin(grain), ke = G.cand_begin(grain + 1);
-      for (int k = kb; k < ke; ++k) {
-        const int sk = G.cand(k);
-        const float d = surface_lb<EXT>(G, sk, px, py, pz);
-        const bool nearer = d < dc;
-        dc2 = nearer ? dc : fminf(dc2, d);
-        near = nearer ? sk : near;
-        dc = nearer ? d : dc;
-      }
-    } else {
-      dc = safety_bvh<EXT>(G, root, px, py, pz, fminf(dbox, cap), dc2, near);
-    }
-  }
-  dgrain = dc - 4.0f * eps;
-  dgrain2 = dc2 - 4.0f * eps;
-  return fminf(dbox, dc) - 4.0f * eps;
 }
 
 /* One candidate surface, where the second ball has shown it to be the only
@@ -1023,12 +808,6 @@ __device__ __forceinline__ void rotate_dirs(const float* frow, int s, int lane, 
   const float r0 = frow[ri], r1 = frow[RS + ri];
   const float r2 = frow[2 * RS + ri], r3 = frow[3 * RS + ri];
   f = cur ? r0 : a0; x = cur ? r1 : a1; y = cur ? r2 : a2; z = cur ? r3 : a3;
-}
-
-__device__ __forceinline__ unsigned lanemask_lt() {
-  unsigned m;
-  asm volatile("mov.u32 %0, %%lanemask_lt;" : "=r"(m));
-  return m;
 }
 
 __device__ __forceinline__ unsigned long long globaltimer() {
@@ -2228,9 +2007,9 @@ static_assert(2 * kOrderBuckets == kTailOrderExtra, "tail order histogram and cu
    flights to leave (the exit time of a random walk whose flights move it
    by 2 MFP^2 / 3 squared along x); walls and holes stretch the walk, but the
    phonons the tail phase waits for are those that rank high on it. */
-__device__ __forceinline__ int order_bucket(const float4* tail, int slot, float x_len) {
-  const float4 e0 = tail[(size_t)kTailUnits * slot];
-  const float4 e1 = tail[(size_t)kTailUnits * slot + 1];
+__device__ __forceinline__ int order_bucket(const float4* tail, int units, int slot, float x_len) {
+  const float4 e0 = tail[(size_t)units * slot];
+  const float4 e1 = tail[(size_t)units * slot + 1];
   const float w = fmaxf(e0.x * (x_len - e0.x), 0.0f) / (e1.w * e1.w);
   return w > 1.0f ? min(kOrderBuckets - 1, (int)(4.0f * __log2f(w))) : 0;
 }
@@ -2242,21 +2021,21 @@ __device__ __forceinline__ int tail_slot(int c, int nlong, int tail_cap) {
 
 /* One thread per hand-over: its bucket, kept in the entry's spare word
    (float4 6, z), and the bucket histogram. */
-__global__ void k_order_hist(float4* __restrict__ tail, int tail_cap, const int* __restrict__ queue,
-                             float x_len, int* __restrict__ hist) {
+__global__ void k_order_hist(float4* __restrict__ tail, int units, int tail_cap,
+                             const int* __restrict__ queue, float x_len, int* __restrict__ hist) {
   const int nlong = min(queue[2], tail_cap);
   const int ntail = nlong + min(queue[4], tail_cap - nlong);
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= ntail) return;
   const int slot = tail_slot(c, nlong, tail_cap);
-  const int b = order_bucket(tail, slot, x_len);
-  reinterpret_cast<int*>(tail + (size_t)kTailUnits * slot + 6)[2] = b;
+  const int b = order_bucket(tail, units, slot, x_len);
+  reinterpret_cast<int*>(tail + (size_t)units * slot + 6)[2] = b;
   atomicAdd(&hist[b], 1);
 }
 
 /* One thread per hand-over: the bucket offsets from the top bucket down
    (every block from the histogram), then the slot to its bucket's range. */
-__global__ void k_order_scatter(const float4* __restrict__ tail, int tail_cap,
+__global__ void k_order_scatter(const float4* __restrict__ tail, int units, int tail_cap,
                                 const int* __restrict__ queue, const int* __restrict__ hist,
                                 int* __restrict__ cursor, int* __restrict__ order) {
   __shared__ int h[kOrderBuckets];
@@ -2277,20 +2056,21 @@ __global__ void k_order_scatter(const float4* __restrict__ tail, int tail_cap,
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= ntail) return;
   const int slot = tail_slot(c, nlong, tail_cap);
-  const int b = reinterpret_cast<const int*>(tail + (size_t)kTailUnits * slot + 6)[2];
+  const int b = reinterpret_cast<const int*>(tail + (size_t)units * slot + 6)[2];
   order[h[b] + atomicAdd(&cursor[b], 1)] = slot;
 }
 }  // namespace
 
-cudaError_t launch_tail_order(const RunF32& r, float x_len, cudaStream_t st) {
+cudaError_t launch_tail_order(float4* tail, int units, int tail_cap, const int* queue, int32_t* order,
+                              float x_len, cudaStream_t st) {
   /* the histogram and the bucket cursors follow the order array */
-  int* hist = r.tail_order + r.tail_cap;
+  int* hist = order + tail_cap;
   cudaError_t e = cudaMemsetAsync(hist, 0, sizeof(int) * 2 * kOrderBuckets, st);
   if (e != cudaSuccess) return e;
-  const unsigned blocks = (unsigned)((r.tail_cap + 255) / 256);
-  k_order_hist<<<blocks, 256, 0, st>>>(r.tail, r.tail_cap, r.queue, x_len, hist);
-  k_order_scatter<<<blocks, 256, 0, st>>>(r.tail, r.tail_cap, r.queue, hist, hist + kOrderBuckets,
-                                          r.tail_order);
+  const unsigned blocks = (unsigned)((tail_cap + 255) / 256);
+  k_order_hist<<<blocks, 256, 0, st>>>(tail, units, tail_cap, queue, x_len, hist);
+  k_order_scatter<<<blocks, 256, 0, st>>>(tail, units, tail_cap, queue, hist, hist + kOrderBuckets,
+                                          order);
   return cudaGetLastError();
 }
 

@@ -1,18 +1,22 @@
 /*
- * kernels_fp64.cu - the plain FP64 transport kernel: one phonon per thread,
- * the reference's linear scan of the box grain plus the current grain per
- * free flight, the reference's intersection / reflection / transmission
- * arithmetic in FP64, the 1e-7 nm nudge and the out-of-box check
- * (calcTransmit and helpers, src/RTMCphon.f90:1608-2414, 2883-3301).
+ * kernels_fp64.cu - FP64 transport: the reference's intersection, reflection
+ * and transmission arithmetic in FP64, its 1e-7 nm nudge and its out-of-box
+ * check (calcTransmit and helpers, src/RTMCphon.f90:1608-2414, 2883-3301),
+ * in two forms that take the same trajectories bit for bit:
+ *   - k_plain_fp64, one phonon per thread and the reference's linear scan of
+ *     the box grain plus the current grain at every flight: the comparator of
+ *     the persistent kernels and the replay target of the CPU oracle;
+ *   - k_drain64 / k_tail64, the two phases of the persistent FP32 kernels
+ *     (kernels_fp32.cu) with FP64 flights.
  *
- * It is the comparator of the persistent FP32 kernel and the replay target of
- * the CPU oracle: this file is compiled with --fmad=false so every a*b+c is
- * rounded twice, exactly as the host restatement computes it.
+ * Compiled with --fmad=false, so every a*b+c is rounded twice, exactly as the
+ * host restatement computes it.
  */
 #include <cuda_runtime.h>
 #include <stdint.h>
 
 #include "fp64_math.cuh"
+#include "geo_fp32.cuh"
 #include "kernels.h"
 #include "philox.cuh"
 
@@ -22,6 +26,8 @@ namespace {
 
 constexpr double kSmall = 1.0e-5;       /* SMALL_VAL, src/RTMCphon.f90:67 */
 constexpr double kBallistic = 1.0e10;   /* src/RTMCphon.f90:1686          */
+/* safe-ball radius searched in a grain with a BVH, in units of the MFP */
+constexpr float kBallCap64 = 32.0f;
 
 __device__ __forceinline__ double dot3(const double* a, const double* b) {
   return a[0] * b[0] + a[1] * b[1] + a[2] * b[2];
@@ -133,9 +139,12 @@ __device__ void capped_normal(const Geo64& g, int k, const double* R, double* N)
   }
 }
 
-/* calcSurfaceDistance dispatch, src/RTMCphon.f90:2883-3088 */
+/* calcSurfaceDistance dispatch, src/RTMCphon.f90:2883-3088.  CULL: a polygon
+   whose plane is crossed beyond lim is left before the division and the edge
+   test (the product's 1e-6 is far above the rounding of either side). */
+template <bool CULL>
 __device__ bool surface_distance(const Geo64& g, int k, const double* R0, const double* D,
-                                 double* L) {
+                                 double lim, double* L) {
   const int sh = g.shape[k];
   if (sh == 1) {
     const double* N = g.normal + 3 * k;
@@ -143,8 +152,11 @@ __device__ bool surface_distance(const Geo64& g, int k, const double* R0, const 
     if (cosangle <= 0.0) return false;
     const double* v = g.vertex + 3 * (size_t)g.vbegin[k];
     double w[3] = {v[0] - R0[0], v[1] - R0[1], v[2] - R0[2]};
-    const double Lh = dot3(w, N) / cosangle;
+    const double num = dot3(w, N);
+    if (CULL && num > lim * cosangle * 1.000001) return false;
+    const double Lh = num / cosangle;
     if (Lh < 0.0) return false;
+    if (CULL && Lh > lim) return false;
     double Rh[3];
     for (int d = 0; d < 3; ++d) Rh[d] = R0[d] + D[d] * Lh;
     if (!in_polygon(v, g.nvertex[k], Rh)) return false;
@@ -264,27 +276,34 @@ __device__ double threshold(const Geo64& g, int k, double omega, double od) {
   return 0.0;
 }
 
-/* One trajectory; returns EndSide (0 lost, 1 x-, 2 x+). */
-__device__ int trace(const Geo64& g, const Task64& t, const Draw& rng, int64_t max_flights,
-                     uint64_t* nflights, bool* capped, double* fpos) {
-  const double X = g.box[0], Y = g.box[1], Z = g.box[2];
+/* A phonon: position, direction, free path, the surface last met (grain and
+   its index there; -1 after an intrinsic event) and the grain it is in. */
+struct Ph64 {
+  double pos[3], dir[3], fp;
+  int igrain, isurf, which;
+};
+
+/* Emission; returns EndSide (1 when the direction points back out). */
+__device__ int emit64(const Geo64& g, const Task64& t, const Draw& rng, Ph64& p) {
+  const double Y = g.box[1], Z = g.box[2];
   double d0, d1, e0, e1;
   rng.block(0, 0, &d0, &d1);
-  double pos[3] = {0.0, d0 * Y * g.scope[0], d1 * Z * g.scope[1]};
+  p.pos[0] = 0.0; p.pos[1] = d0 * Y * g.scope[0]; p.pos[2] = d1 * Z * g.scope[1];
   rng.block(0, 1, &e0, &e1);
   double sphi, cphi;
   dsincos_2pi(e0, &sphi, &cphi);
-  double dir[3] = {t.cth, t.sth * cphi, t.sth * sphi};
-  int EndSide = (dir[0] <= 0.0) ? 1 : 0;
-  int igrain = 0, isurf = 0, whichV = 0;
+  p.dir[0] = t.cth; p.dir[1] = t.sth * cphi; p.dir[2] = t.sth * sphi;
+  p.igrain = 0;
+  p.isurf = 0;
+  p.which = 0;
   if (g.kind_grain == 1) {
     double dmin = 1.0e10;
     for (int ig = 1; ig <= g.ngrain; ++ig) {
       if (!g.grain_incident[ig]) continue;
       const double* G = g.grain_gen + 3 * ig;
-      const double a = pos[0] - G[0], b = pos[1] - G[1], c = pos[2] - G[2];
+      const double a = p.pos[0] - G[0], b = p.pos[1] - G[1], c = p.pos[2] - G[2];
       const double d2 = a * a + b * b + c * c;
-      if (dmin > d2) { dmin = d2; whichV = ig; }
+      if (dmin > d2) { dmin = d2; p.which = ig; }
     }
   } else {
     bool found = false;
@@ -292,135 +311,173 @@ __device__ int trace(const Geo64& g, const Task64& t, const Draw& rng, int64_t m
       if (!g.grain_incident[ig]) continue;
       for (int k = g.grain_begin[ig]; k < g.grain_begin[ig + 1]; ++k) {
         if (!g.incident[k]) continue;
-        if (in_polygon(g.vertex + 3 * (size_t)g.vbegin[k], g.nvertex[k], pos)) {
-          whichV = ig;
+        if (in_polygon(g.vertex + 3 * (size_t)g.vbegin[k], g.nvertex[k], p.pos)) {
+          p.which = ig;
           found = true;
           break;
         }
       }
     }
-    if (!found) whichV = g.igrain_fill;
+    if (!found) p.which = g.igrain_fill;
   }
-  const bool ballistic = (t.lambda == kBallistic);
-  double FreePath = ballistic ? kBallistic : -t.lambda * dlog_pos(e1);
+  p.fp = (t.lambda == kBallistic) ? kBallistic : -t.lambda * dlog_pos(e1);
+  return (p.dir[0] <= 0.0) ? 1 : 0;
+}
+
+__device__ __forceinline__ bool in_box64(const Geo64& g, const double* pos) {
+  return pos[0] >= 0.0 - kSmall && pos[0] <= g.box[0] + kSmall && pos[1] >= 0.0 - kSmall &&
+         pos[1] <= g.box[1] + kSmall && pos[2] >= 0.0 - kSmall && pos[2] <= g.box[2] + kSmall;
+}
+
+/* Isotropic direction and free path of an intrinsic event from flight fl's
+   blocks 0 and 1 (what a used-up free path draws). */
+__device__ __forceinline__ void pp_draw64(const Draw& rng, double lambda, uint32_t fl, double* dir,
+                                          double* fp) {
+  double d0, d1, r0, r1;
+  rng.block(fl, 0, &d0, &d1);
+  rng.block(fl, 1, &r0, &r1);
+  const double ct = d0 * 2.0 - 1.0;
+  double sp, cp;
+  dsincos_2pi(d1, &sp, &cp);
+  const double st = sqrt(1.0 - ct * ct);
+  dir[0] = ct; dir[1] = st * cp; dir[2] = st * sp;
+  *fp = -lambda * dlog_pos(r0);
+}
+
+/* Flight fl ends in an intrinsic event after its whole free path. */
+__device__ __forceinline__ void pp_event64(const Draw& rng, double lambda, uint32_t fl, Ph64& p) {
+  for (int d = 0; d < 3; ++d) p.pos[d] = p.pos[d] + p.fp * p.dir[d];
+  pp_draw64(rng, lambda, fl, p.dir, &p.fp);
+  for (int d = 0; d < 3; ++d) p.pos[d] = p.pos[d] + 1.0e-7 * p.dir[d];
+  p.igrain = 0;
+  p.isurf = -1;
+}
+
+/* Flight fl ends after `distance` at surface p.isurf of grain p.igrain:
+   bath, periodic face, reflection or transmission (src/RTMCphon.f90:1744-1792,
+   2225-2413).  Returns EndSide (0 lost, 1 x-, 2 x+), -1 while it goes on. */
+__device__ int surface_event64(const Geo64& g, double lambda, double omega, const Draw& rng,
+                               uint32_t fl, double distance, Ph64& p) {
+  double* const pos = p.pos;
+  double* const dir = p.dir;
+  int end_side = -1, Jreflect = 1;
+  double d0, d1;
+  for (int d = 0; d < 3; ++d) pos[d] = pos[d] + distance * dir[d];
+  if (p.isurf < 0) {
+    return 0;
+  } else if (p.igrain == 0 && p.isurf == 0) {
+    end_side = 1;
+  } else if (p.igrain == 0 && p.isurf == 1) {
+    end_side = 2;
+  } else if (p.igrain == 0 && g.face_kind[p.isurf] == 1) {
+    const int ax = p.isurf >> 1;
+    const double L = g.box[ax];
+    const double sg = (p.isurf & 1) == 0 ? L : -L;
+    if (ax == 1) pos[1] = pos[1] + sg;
+    else pos[2] = pos[2] + sg;
+  } else {
+    const int k = g.grain_begin[p.igrain] + p.isurf;
+    rng.block(fl, 0, &d0, &d1);
+    double od = 0.0;
+    if (g.nmaterial != 1 && (g.kind_trans[k] == 2 || g.kind_trans[k] == 3)) {
+      double x;
+      rng.block(fl, 2, &od, &x);
+    }
+    if (d0 <= g.spec[k]) {
+      const double thr = threshold(g, k, omega, od);
+      if (d1 <= thr) {
+        Jreflect = 0;
+      } else {
+        double N[3];
+        surface_normal(g, k, pos, N);
+        if (dot3(N, dir) < 0) for (int d = 0; d < 3; ++d) N[d] = -1.0 * N[d];
+        const double dn = dot3(N, dir);
+        for (int d = 0; d < 3; ++d) dir[d] = dir[d] - 2.0 * N[d] * dn;
+        Jreflect = 1;
+      }
+    } else {
+      double N[3], Rm[9];
+      surface_normal(g, k, pos, N);
+      if (dot3(N, dir) < 0.0) for (int d = 0; d < 3; ++d) N[d] = -1.0 * N[d];
+      surface_rotation(g, k, pos, Rm);
+      double f0, f1;
+      rng.block(fl, 1, &f0, &f1);
+      const double sint = sqrt(d1);
+      const double cost = sqrt(1.0 - sint * sint);
+      double sp, cp;
+      dsincos_2pi(f0, &sp, &cp);
+      const double td[3] = {sint * cp, sint * sp, cost};
+      double v[3];
+      for (int i = 0; i < 3; ++i) v[i] = Rm[i] * td[0] + Rm[3 + i] * td[1] + Rm[6 + i] * td[2];
+      if (dot3(dir, N) > 0.0) {
+        for (int i = 0; i < 3; ++i) dir[i] = -v[i];
+      } else {
+        for (int i = 0; i < 3; ++i) dir[i] = v[i];
+      }
+      if (dot3(dir, N) > 0.0) for (int i = 0; i < 3; ++i) dir[i] = -1.0 * dir[i];
+      const double thr = threshold(g, k, omega, od);
+      if (f1 <= thr) {
+        for (int i = 0; i < 3; ++i) dir[i] = -dir[i];
+        Jreflect = 0;
+      } else {
+        Jreflect = 1;
+      }
+    }
+  }
+  for (int d = 0; d < 3; ++d) pos[d] = pos[d] + 1.0e-7 * dir[d];
+  if (lambda == kBallistic) {
+    p.fp = kBallistic;
+  } else {
+    p.fp = p.fp - distance;
+    if (p.fp < 1.0e-10) {
+      double r0, r1;
+      rng.block(fl, 2, &r0, &r1);
+      p.fp = -lambda * dlog_pos(r1);
+    }
+  }
+  if (Jreflect == 0) p.which = g.gout[g.grain_begin[p.igrain] + p.isurf];
+  return end_side;
+}
+
+/* One trajectory; returns EndSide (0 lost, 1 x-, 2 x+). */
+__device__ int trace(const Geo64& g, const Task64& t, const Draw& rng, int64_t max_flights,
+                     uint64_t* nflights, bool* capped, double* fpos) {
+  Ph64 p;
+  int EndSide = emit64(g, t, rng, p);
   uint64_t flight = 0;
   *capped = false;
   while (EndSide == 0) {
-    if (!(pos[0] >= 0.0 - kSmall && pos[0] <= X + kSmall && pos[1] >= 0.0 - kSmall &&
-          pos[1] <= Y + kSmall && pos[2] >= 0.0 - kSmall && pos[2] <= Z + kSmall))
-      break;
+    if (!in_box64(g, p.pos)) break;
     if ((int64_t)flight >= max_flights) { *capped = true; break; }
     ++flight;
-    const uint32_t fl = (uint32_t)flight;
     double distance = 1.0e10;
-    int ig_min = igrain, is_min = isurf;
+    int ig_min = p.igrain, is_min = p.isurf;
     for (int pass = 0; pass < 2; ++pass) {
-      const int ig = pass == 0 ? 0 : whichV;
-      if (pass == 1 && whichV == 0) break;
+      const int ig = pass == 0 ? 0 : p.which;
+      if (pass == 1 && p.which == 0) break;
       const int kb = g.grain_begin[ig], ke = g.grain_begin[ig + 1];
       for (int k = kb; k < ke; ++k) {
         if (!g.internal[k]) continue;
         double L;
-        if (surface_distance(g, k, pos, dir, &L) && distance > L) {
+        if (surface_distance<false>(g, k, p.pos, p.dir, 0.0, &L) && distance > L) {
           distance = L;
           ig_min = ig;
           is_min = k - kb;
         }
       }
     }
-    igrain = ig_min;
-    isurf = is_min;
-    int Jreflect = 1;
-    bool pp = false;
-    if (FreePath < distance) {
-      distance = FreePath;
-      for (int d = 0; d < 3; ++d) pos[d] = pos[d] + distance * dir[d];
-      rng.block(fl, 0, &d0, &d1);
-      const double ct = d0 * 2.0 - 1.0;
-      double sp, cp;
-      dsincos_2pi(d1, &sp, &cp);
-      const double st = sqrt(1.0 - ct * ct);
-      dir[0] = ct; dir[1] = st * cp; dir[2] = st * sp;
-      igrain = 0;
-      isurf = -1;
-      pp = true;
+    if (p.fp < distance) {
+      pp_event64(rng, t.lambda, (uint32_t)flight, p);
     } else {
-      for (int d = 0; d < 3; ++d) pos[d] = pos[d] + distance * dir[d];
-      if (isurf < 0) {
-        break;
-      } else if (igrain == 0 && isurf == 0) {
-        EndSide = 1;
-      } else if (igrain == 0 && isurf == 1) {
-        EndSide = 2;
-      } else if (igrain == 0 && g.face_kind[isurf] == 1) {
-        const int ax = isurf >> 1;
-        if ((isurf & 1) == 0) pos[ax] = pos[ax] + g.box[ax];
-        else pos[ax] = pos[ax] - g.box[ax];
-      } else {
-        const int k = g.grain_begin[igrain] + isurf;
-        rng.block(fl, 0, &d0, &d1);
-        double od = 0.0;
-        if (g.nmaterial != 1 && (g.kind_trans[k] == 2 || g.kind_trans[k] == 3)) {
-          double x;
-          rng.block(fl, 2, &od, &x);
-        }
-        if (d0 <= g.spec[k]) {
-          const double thr = threshold(g, k, t.omega, od);
-          if (d1 <= thr) {
-            Jreflect = 0;
-          } else {
-            double N[3];
-            surface_normal(g, k, pos, N);
-            if (dot3(N, dir) < 0) for (int d = 0; d < 3; ++d) N[d] = -1.0 * N[d];
-            const double dn = dot3(N, dir);
-            for (int d = 0; d < 3; ++d) dir[d] = dir[d] - 2.0 * N[d] * dn;
-            Jreflect = 1;
-          }
-        } else {
-          double N[3], Rm[9];
-          surface_normal(g, k, pos, N);
-          if (dot3(N, dir) < 0.0) for (int d = 0; d < 3; ++d) N[d] = -1.0 * N[d];
-          surface_rotation(g, k, pos, Rm);
-          double f0, f1;
-          rng.block(fl, 1, &f0, &f1);
-          const double sint = sqrt(d1);
-          const double cost = sqrt(1.0 - sint * sint);
-          double sp, cp;
-          dsincos_2pi(f0, &sp, &cp);
-          const double td[3] = {sint * cp, sint * sp, cost};
-          double v[3];
-          for (int i = 0; i < 3; ++i) v[i] = Rm[i] * td[0] + Rm[3 + i] * td[1] + Rm[6 + i] * td[2];
-          if (dot3(dir, N) > 0.0) {
-            for (int i = 0; i < 3; ++i) dir[i] = -v[i];
-          } else {
-            for (int i = 0; i < 3; ++i) dir[i] = v[i];
-          }
-          if (dot3(dir, N) > 0.0) for (int i = 0; i < 3; ++i) dir[i] = -1.0 * dir[i];
-          const double thr = threshold(g, k, t.omega, od);
-          if (f1 <= thr) {
-            for (int i = 0; i < 3; ++i) dir[i] = -dir[i];
-            Jreflect = 0;
-          } else {
-            Jreflect = 1;
-          }
-        }
-      }
+      p.igrain = ig_min;
+      p.isurf = is_min;
+      const int e = surface_event64(g, t.lambda, t.omega, rng, (uint32_t)flight, distance, p);
+      if (e == 0) break;
+      if (e > 0) EndSide = e;
     }
-    for (int d = 0; d < 3; ++d) pos[d] = pos[d] + 1.0e-7 * dir[d];
-    if (ballistic) {
-      FreePath = kBallistic;
-    } else {
-      FreePath = FreePath - distance;
-      if (FreePath < 1.0e-10) {
-        double r0, r1;
-        if (pp) { rng.block(fl, 1, &r0, &r1); FreePath = -t.lambda * dlog_pos(r0); }
-        else { rng.block(fl, 2, &r0, &r1); FreePath = -t.lambda * dlog_pos(r1); }
-      }
-    }
-    if (Jreflect == 0) whichV = g.gout[g.grain_begin[igrain] + isurf];
   }
   *nflights = flight;
-  if (fpos) { fpos[0] = pos[0]; fpos[1] = pos[1]; fpos[2] = pos[2]; }
+  if (fpos) { fpos[0] = p.pos[0]; fpos[1] = p.pos[1]; fpos[2] = p.pos[2]; }
   return EndSide;
 }
 
@@ -496,6 +553,500 @@ __global__ void __launch_bounds__(128) k_plain_fp64(Geo64 g, Run64 r) {
   }
 }
 
+/* ---- persistent FP64 transport ------------------------------------------- */
+
+/* Nearest surface of the box and of grain `which` no farther than the
+   flight's free path (one beyond it cannot end the flight): the same surface,
+   distance and tie (box before grain, then the lower index) as the linear
+   scan.  What the scan does for every surface is left out where it cannot
+   matter:
+     - box faces that the host found to be the axis-aligned rectangles they
+       are meant to be (Geo64.box_axis) are met at (face - x) / d, which is
+       the general formula's value with a normal of +-1 and zeros, and a hit
+       well inside the rectangle needs no edge test;
+     - a plane crossed beyond the nearest hit so far is left early;
+     - a grain with a BVH is walked in FP32: the node boxes are padded by 4 eps
+       and positions rounded by 2^-24 of the box, so no node that holds the
+       hit is skipped.
+   Returns whether there is a hit; box_only leaves the grain's surfaces out. */
+__device__ bool nearest64(const Geo64& g, const Geo<false>& G, float eps, const double* pos,
+                          const double* dir, double fp, int which, bool box_only, double* dist,
+                          int* igrain, int* isurf) {
+  double best = fp < 1.0e10 ? __longlong_as_double(__double_as_longlong(fp) + 1) : 1.0e10;
+  bool hit = false;
+  if (g.box_axis) {
+    const double m = (double)eps;
+#pragma unroll
+    for (int ax = 0; ax < 3; ++ax) {
+      const double d = dir[ax];
+      const double w = (d > 0.0 ? g.box[ax] : 0.0) - pos[ax];
+      if (d == 0.0) continue;
+      if (d > 0.0 ? (w < 0.0 || w > best * d * 1.000001) : (w > 0.0 || w < best * d * 1.000001))
+        continue;
+      const double L = w / d;
+      if (!(best > L)) continue;
+      const int b = ax == 0 ? 1 : 0, c = ax == 2 ? 1 : 2;
+      const double hb = pos[b] + dir[b] * L, hc = pos[c] + dir[c] * L;
+      const int k = 2 * ax + (d > 0.0 ? 1 : 0);
+      bool in = hb > m && hb < g.box[b] - m && hc > m && hc < g.box[c] - m;
+      if (!in) {
+        const double Rh[3] = {pos[0] + dir[0] * L, pos[1] + dir[1] * L, pos[2] + dir[2] * L};
+        in = in_polygon(g.vertex + 3 * (size_t)g.vbegin[k], 4, Rh);
+      }
+      if (in) { best = L; *igrain = 0; *isurf = k; hit = true; }
+    }
+  } else {
+    for (int k = 0; k < g.grain_begin[1]; ++k) {
+      double L;
+      if (g.internal[k] && surface_distance<true>(g, k, pos, dir, best, &L) && best > L) {
+        best = L; *igrain = 0; *isurf = k; hit = true;
+      }
+    }
+  }
+  if (which > 0 && !box_only) {
+    const int kb0 = g.grain_begin[which];
+    const int root = G.bvh_root(which);
+    if (root < 0) {
+      const int kb = G.cand_begin(which), ke = G.cand_begin(which + 1);
+      for (int i = kb; i < ke; ++i) {
+        const int k = G.cand(i);
+        double L;
+        if (surface_distance<true>(g, k, pos, dir, best, &L) && best > L) {
+          best = L; *igrain = which; *isurf = k - kb0; hit = true;
+        }
+      }
+    } else {
+      const float px = (float)pos[0], py = (float)pos[1], pz = (float)pos[2];
+      const float ix = inv_dir((float)dir[0]), iy = inv_dir((float)dir[1]),
+                  iz = inv_dir((float)dir[2]);
+      int stk[kBvhStack];
+      float stt[kBvhStack];
+      int sp = 0, node = root;
+      bool mine = false;  /* the hit so far is one of this grain's */
+      while (true) {
+        const int cnt = __float_as_int(G.node(2 * node + 1).w);
+        const int a = __float_as_int(G.node(2 * node).w);
+        /* the nearest hit as an FP32 bound, rounded up by its tolerance */
+        float tm = fminf((float)best * 1.00001f + eps, 3.0e38f);
+        bool descended = false;
+        if (cnt > 0) {
+          for (int i = a; i < a + cnt; ++i) {
+            const int k = G.cand(i);
+            double L;
+            if (surface_distance<true>(g, k, pos, dir, best, &L) &&
+                (best > L || (mine && best == L && k - kb0 < *isurf))) {
+              best = L; *igrain = which; *isurf = k - kb0; hit = true; mine = true;
+            }
+          }
+          tm = fminf((float)best * 1.00001f + eps, 3.0e38f);
+        } else {
+          const float tl = box_entry(G.node(2 * a), G.node(2 * a + 1), px, py, pz, ix, iy, iz, tm, eps);
+          const float tg = box_entry(G.node(2 * a + 2), G.node(2 * a + 3), px, py, pz, ix, iy, iz, tm,
+                                     eps);
+          const bool hl = tl < 3.0e38f, hg = tg < 3.0e38f;
+          if (hl || hg) {
+            const bool lf = hl && (!hg || tl <= tg);
+            if (hl && hg && sp < kBvhStack) {
+              stk[sp] = lf ? a + 1 : a;
+              stt[sp] = lf ? tg : tl;
+              ++sp;
+            }
+            node = lf ? a : a + 1;
+            descended = true;
+          }
+        }
+        if (descended) continue;
+        bool found = false;
+        while (sp > 0) {
+          --sp;
+          if (stt[sp] <= tm) {
+            node = stk[sp];
+            found = true;
+            break;
+          }
+        }
+        if (!found) break;
+      }
+    }
+  }
+  *dist = hit ? best : 1.0e10;
+  return hit;
+}
+
+/* Safe ball and grain ball about pos from the FP32 bounds (kernels_fp32.cu),
+   less the rounding of the centre, the 1e-7 nudges and the few 1e-8 of the
+   box by which an FP64 root can be off: radius squared, 0 for none. */
+__device__ __forceinline__ void ball64(const Geo<false>& G, const GeoF32& gp, int which,
+                                       const double* pos, float lam, float* bx, float* by,
+                                       float* bz, float* br2, float* gr2) {
+  *bx = (float)pos[0]; *by = (float)pos[1]; *bz = (float)pos[2];
+  float dg, dg2;
+  int near;
+  const float d = safety<true>(G, which, *bx, *by, *bz, gp.box[0], gp.box[1], gp.box[2], gp.eps,
+                               kBallCap64 * lam, dg, dg2, near) - 1.0e-6f;
+  dg -= 1.0e-6f;
+  *br2 = d > 0.0f ? d * d : 0.0f;
+  *gr2 = dg > 0.0f ? dg * dg : 0.0f;
+}
+
+/* Squared distance of p from the ball's centre, in FP32. */
+__device__ __forceinline__ float off2(const double* p, float bx, float by, float bz) {
+  const float x = (float)p[0] - bx, y = (float)p[1] - by, z = (float)p[2] - bz;
+  return fmaf(x, x, fmaf(y, y, z * z));
+}
+
+__device__ __forceinline__ Draw sample_draw(const Run64& r, uint64_t sample) {
+  Draw rng;
+  rng.key.k0 = r.k0;
+  rng.key.k1 = r.k1;
+  rng.c1 = r.c1;
+  rng.slo = (uint32_t)sample;
+  rng.shi = (uint32_t)(sample >> 32);
+  return rng;
+}
+
+__device__ __forceinline__ float4 pack2(double a, double b) {
+  return make_float4(__int_as_float(__double2loint(a)), __int_as_float(__double2hiint(a)),
+                     __int_as_float(__double2loint(b)), __int_as_float(__double2hiint(b)));
+}
+__device__ __forceinline__ void unpack2(float4 v, double* a, double* b) {
+  *a = __hiloint2double(__float_as_int(v.y), __float_as_int(v.x));
+  *b = __hiloint2double(__float_as_int(v.w), __float_as_int(v.z));
+}
+
+/* ---- the two phases ---------------------------------------------------------
+   The plain kernel is bound by latency: one lane per phonon, every flight a
+   scan of all surfaces by divergent lanes (about 4 us a flight), to the end of
+   the longest trajectory.  Porous film, 2000 modes from 5 nm, 1e5 phonons:
+   plain 29.4 ms, here 3.4; wire 300 x 60 nm, MFPs from 2 nm, 1e5 phonons:
+   171 -> 7.9 ms; wire 1000 x 100 nm, gray MFP 150 nm, 3e4 phonons: 5.2 -> 2.9.
+   What bounds them now is the instructions of a round (about 2100 a warp, at
+   7 cycles each: fixed latencies of the FP64 chains, instruction fetch) times
+   the rounds of the longest walk. */
+
+/* Drain phase: the work queue, one phonon per lane, idle lanes refilled from
+   the warp's chunk; flights that stay in the safe ball are taken without a
+   scan; once the queue is dry the live phonons go to the tail list
+   (grace_passes). */
+__global__ void __launch_bounds__(256, 2) k_drain64(Geo64 g, GeoF32 gp, Run64 r) {
+  Geo<false> G;
+  G.base = gp.blob;
+  G.lay = gp.lay;
+  const int lane = threadIdx.x & 31;
+  int ch_task = -1, ch_next = 0, ch_left = 0;
+  bool queue_done = false;
+  int grace = r.grace_steps;
+  bool alive = false;
+  Ph64 p;
+  p.pos[0] = p.pos[1] = p.pos[2] = p.dir[0] = p.dir[1] = p.dir[2] = p.fp = 0.0;
+  p.igrain = p.isurf = p.which = 0;
+  double lambda = 1.0;
+  float bx = 0, by = 0, bz = 0, br2 = 0, gr2 = 0;
+  int task = 0;
+  uint32_t flight = 0;
+  uint64_t sample = 0;
+  unsigned long long my_flights = 0, my_samples = 0, my_capped = 0, my_lost = 0;
+  while (true) {
+    int end_side = -1;
+    unsigned idle = __ballot_sync(FULL, !alive);
+    if (!queue_done && idle && (__popc(idle) >= r.regen_threshold || idle == FULL)) {
+      while (idle && !queue_done) {
+        if (ch_left == 0) {
+          int c = 0;
+          if (lane == 0) c = atomicAdd(r.queue, 1);
+          c = __shfl_sync(FULL, c, 0);
+          if (c >= r.nchunk) { queue_done = true; break; }
+          const int4 q = r.chunk[c];
+          ch_task = q.x; ch_next = q.y; ch_left = q.z;
+        }
+        const int take = min(__popc(idle), ch_left);
+        const int rank = __popc(idle & lanemask_lt());
+        if (((idle >> lane) & 1u) && rank < take) {
+          const int64_t q = (int64_t)r.rank + (int64_t)(ch_next + rank) * r.nranks;
+          task = ch_task;
+          sample = (uint64_t)task * (uint64_t)r.np + (uint64_t)q;
+          const Task64 t = r.task[task];
+          lambda = t.lambda;
+          const int e = emit64(g, t, sample_draw(r, sample), p);
+          end_side = e > 0 ? e : -1;
+          br2 = gr2 = 0.0f;
+          flight = 0;
+          alive = true;
+          my_samples += 1;
+        }
+        ch_next += take;
+        ch_left -= take;
+        idle = __ballot_sync(FULL, !alive);
+      }
+    }
+    if (!__any_sync(FULL, alive)) {
+      if (queue_done) break;
+      continue;
+    }
+    if (queue_done && r.coop_lanes > 0 && __popc(__ballot_sync(FULL, alive)) <= r.coop_lanes) {
+      /* A round costs about as much as a pass of 32 lanes (2100 warp
+         instructions).  Where the MFP is the smallest box side or more nearly
+         every flight ends at a surface, so those phonons stay to the end
+         (wire 1000 x 100 nm, 1e5 phonons: MFP 1000 nm 4.39 -> 2.10 ms, 150 nm
+         5.39 -> 3.66; at 30 nm it would be 7.68 -> 12.2). */
+      const float lam = (float)lambda;
+      const bool give = alive && end_side < 0 &&
+                        (lam < r.fast_lambda_max || r.fast_steps <= 0 ||
+                         (grace == 0 && lam < r.round_lambda_max));
+      const unsigned mw = __ballot_sync(FULL, give);
+      grace -= grace > 0 ? 1 : 0;
+      if (mw) {
+        const int fw = __ffs(mw) - 1;
+        int base = 0;
+        if (lane == fw) base = atomicAdd(r.queue + 4, __popc(mw));
+        base = __shfl_sync(FULL, base, fw);
+        const int idx = base + __popc(mw & lanemask_lt());
+        /* the list has a slot for every lane of the grid */
+        if (give && idx < r.tail_cap) {
+          float4* e = r.tail + (size_t)kTail64Units * (r.tail_cap - 1 - idx);
+          e[0] = make_float4((float)p.pos[0], bx, by, bz);
+          e[1] = make_float4(br2, gr2, 0.0f, (float)lambda);
+          e[2] = pack2(p.pos[0], p.pos[1]);
+          e[3] = pack2(p.pos[2], p.dir[0]);
+          e[4] = pack2(p.dir[1], p.dir[2]);
+          e[5] = pack2(p.fp, lambda);
+          e[6] = make_float4(__int_as_float(p.igrain), __int_as_float(p.isurf), 0.0f,
+                             __int_as_float(p.which));
+          e[7] = make_float4(__int_as_float(task), __uint_as_float((uint32_t)sample),
+                             __uint_as_float((uint32_t)(sample >> 32)), __uint_as_float(flight));
+          alive = false;
+        }
+        if (!__any_sync(FULL, alive)) break;
+      }
+    }
+    const Draw rng = sample_draw(r, sample);
+    /* ---- flights inside the safe ball, one a pass: past fast_steps only
+       while half of the live lanes are still in theirs ---------------- */
+    bool paused = false;
+    {
+      const int nalive = __popc(__ballot_sync(FULL, alive));
+      bool fast = alive && end_side < 0 && br2 > 0.0f;
+      for (int n = 0;; ++n) {
+        if (fast) {
+          double q[3];
+          for (int d = 0; d < 3; ++d) q[d] = p.pos[d] + p.fp * p.dir[d];
+          fast = (int64_t)flight < r.max_flights && off2(q, bx, by, bz) < br2;
+        }
+        const unsigned gm = __ballot_sync(FULL, fast);
+        if (!gm) break;
+        if (n >= r.fast_steps && (n >= 4 * r.fast_steps || 2 * __popc(gm) < nalive)) {
+          paused = fast;
+          break;
+        }
+        if (fast) {
+          ++flight;
+          pp_event64(rng, lambda, flight, p);
+        }
+      }
+    }
+    if (alive && !paused && end_side < 0) {
+      if (!in_box64(g, p.pos)) {
+        end_side = 0;
+      } else if ((int64_t)flight >= r.max_flights) {
+        end_side = 0;
+        my_capped += 1;
+      } else {
+        ++flight;
+        double q[3], distance;
+        for (int d = 0; d < 3; ++d) q[d] = p.pos[d] + p.fp * p.dir[d];
+        const bool box_only = off2(q, bx, by, bz) < gr2 && off2(p.pos, bx, by, bz) < gr2;
+        const bool hit = nearest64(g, G, gp.eps, p.pos, p.dir, p.fp, p.which, box_only, &distance,
+                                   &p.igrain, &p.isurf);
+        if (!hit && p.fp < 1.0e10) {
+          pp_event64(rng, lambda, flight, p);
+          br2 = 0.0f;
+          if (r.fast_steps > 0 && (float)lambda < r.fast_lambda_max)
+            ball64(G, gp, p.which, p.pos, (float)lambda, &bx, &by, &bz, &br2, &gr2);
+        } else {
+          const int which = p.which;
+          end_side = surface_event64(g, lambda, r.task[task].omega, rng, flight, distance, p);
+          br2 = 0.0f;
+          if (p.which != which) gr2 = 0.0f;
+        }
+      }
+    }
+    const bool fin = alive && end_side >= 0;
+    warp_add_by_task(fin && (end_side == 2 || (end_side == 0 && r.ref_quirks)), task, r.counts);
+    warp_add_by_task(fin && end_side == 0, task, r.lost);
+    if (fin) {
+      my_flights += flight;
+      my_lost += end_side == 0 ? 1 : 0;
+      alive = false;
+    }
+  }
+  unsigned long long v0 = my_flights, v1 = my_lost, v2 = my_capped, v3 = my_samples;
+  for (int o = 16; o > 0; o >>= 1) {
+    v0 += __shfl_xor_sync(FULL, v0, o);
+    v1 += __shfl_xor_sync(FULL, v1, o);
+    v2 += __shfl_xor_sync(FULL, v2, o);
+    v3 += __shfl_xor_sync(FULL, v3, o);
+  }
+  if (lane == 0) {
+    if (v0) atomicAdd(r.stats + 0, v0);
+    if (v1) atomicAdd(r.stats + 1, v1);
+    if (v2) atomicAdd(r.stats + 2, v2);
+    if (v3) atomicAdd(r.stats + 3, v3);
+  }
+}
+
+/* flights a round tests from its first one that walks a BVH */
+constexpr int kTestWindow64 = 4;
+/* double2 between the rows of a warp's round */
+constexpr int kRow64 = 33;
+
+/* Tail phase: one phonon per warp, 32 flights a round, one per lane.  Every
+   lane holds the phonon.  Lane j draws what flight f+1+j ends with if it ends
+   in an intrinsic event (the blocks depend on the counter alone); the moves
+   fp d and the nudges are products of those draws, so only their sums run one
+   after the other: lane c < 3 adds coordinate c's, two additions a flight,
+   through shared memory.  The first flight that meets a surface, leaves the
+   box or reaches the cap ends the round, and every lane takes its event. */
+__global__ void __launch_bounds__(256, 2) k_tail64(Geo64 g, GeoF32 gp, Run64 r) {
+  __shared__ double2 rows[8][3 * kRow64];
+  double2* const row = rows[threadIdx.x >> 5];
+  Geo<false> G;
+  G.base = gp.blob;
+  G.lay = gp.lay;
+  const int lane = threadIdx.x & 31;
+  const int ntail = min(r.queue[4], r.tail_cap);
+  unsigned long long my_flights = 0, my_capped = 0, my_lost = 0;
+  while (true) {
+    int c = 0;
+    if (lane == 0) c = atomicAdd(r.queue + 3, 1);
+    c = __shfl_sync(FULL, c, 0);
+    if (c >= ntail) break;
+    const float4* e = r.tail + (size_t)kTail64Units * r.tail_order[c];
+    const float4 e0 = e[0], e1 = e[1], e6 = e[6], e7 = e[7];
+    float bx = e0.y, by = e0.z, bz = e0.w, br2 = e1.x, gr2 = e1.y;
+    Ph64 p;
+    double lambda;
+    unpack2(e[2], &p.pos[0], &p.pos[1]);
+    unpack2(e[3], &p.pos[2], &p.dir[0]);
+    unpack2(e[4], &p.dir[1], &p.dir[2]);
+    unpack2(e[5], &p.fp, &lambda);
+    p.igrain = __float_as_int(e6.x);
+    p.isurf = __float_as_int(e6.y);
+    p.which = __float_as_int(e6.w);
+    const int task = __float_as_int(e7.x);
+    const Draw rng = sample_draw(r, ((uint64_t)__float_as_uint(e7.z) << 32) | __float_as_uint(e7.y));
+    uint32_t flight = __float_as_uint(e7.w);
+    const double omega = r.task[task].omega;
+    int end_side = -1;
+    bool capped = false;
+    while (end_side < 0) {
+      double nd[3], nf;
+      pp_draw64(rng, lambda, flight + 1u + (uint32_t)lane, nd, &nf);
+      /* flight `lane` starts with what the previous one drew */
+      double sfp = __shfl_up_sync(FULL, nf, 1), sd[3];
+      if (lane == 0) sfp = p.fp;
+#pragma unroll
+      for (int d = 0; d < 3; ++d) {
+        sd[d] = __shfl_up_sync(FULL, nd[d], 1);
+        if (lane == 0) sd[d] = p.dir[d];
+        row[d * kRow64 + lane] = make_double2(sfp * sd[d], 1.0e-7 * nd[d]);
+      }
+      __syncwarp();
+      if (lane < 3) {
+        double2* const q = row + lane * kRow64;
+        double a = lane == 0 ? p.pos[0] : (lane == 1 ? p.pos[1] : p.pos[2]);
+#pragma unroll
+        for (int b = 0; b < 32; b += 8) {
+          double2 v[8];
+#pragma unroll
+          for (int j = 0; j < 8; ++j) v[j] = q[b + j];
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            v[j].x = a + v[j].x;
+            a = v[j].x + v[j].y;
+            v[j].y = a;
+          }
+#pragma unroll
+          for (int j = 0; j < 8; ++j) q[b + j] = v[j];
+        }
+      }
+      __syncwarp();
+      /* start point, end point before the nudge, and after it */
+      double sp[3], sq[3];
+#pragma unroll
+      for (int d = 0; d < 3; ++d) {
+        sq[d] = row[d * kRow64 + lane].x;
+        sp[d] = lane == 0 ? p.pos[d] : row[d * kRow64 + (lane > 0 ? lane - 1 : 0)].y;
+      }
+      const float se = off2(sq, bx, by, bz), ss = off2(sp, bx, by, bz);
+      const bool in_ball = se < br2 && ss < br2;
+      const bool in_gball = se < gr2 && ss < gr2;
+      const bool inbox = in_box64(g, sp);
+      const bool brk = !inbox || (int64_t)flight + lane >= r.max_flights;
+      const bool walks = !in_ball && !in_gball && p.which > 0 && G.bvh_root(p.which) >= 0;
+      const unsigned wm = __ballot_sync(FULL, walks);
+      const int jw = wm ? min(32, __ffs(wm) - 1 + kTestWindow64) : 32;
+      double distance = 1.0e10;
+      int ig = lane == 0 ? p.igrain : 0, is = lane == 0 ? p.isurf : -1;
+      bool stop = brk;
+      if (!brk && !in_ball && lane < jw) {
+        const bool hit = nearest64(g, G, gp.eps, sp, sd, sfp, p.which, in_gball, &distance, &ig, &is);
+        stop = hit || !(sfp < 1.0e10);
+      }
+      const unsigned sm = __ballot_sync(FULL, stop && lane < jw);
+      const int j = sm ? __ffs(sm) - 1 : jw;
+      flight += (uint32_t)j;
+      if (j < 32) {
+        /* the state at the start of flight j */
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+          p.pos[d] = __shfl_sync(FULL, sp[d], j);
+          p.dir[d] = __shfl_sync(FULL, sd[d], j);
+        }
+        p.fp = __shfl_sync(FULL, sfp, j);
+      } else {
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+          p.pos[d] = row[d * kRow64 + 31].y;
+          p.dir[d] = __shfl_sync(FULL, nd[d], 31);
+        }
+        p.fp = __shfl_sync(FULL, nf, 31);
+      }
+      __syncwarp();  /* the next round rewrites the rows */
+      if (j > 0) { p.igrain = 0; p.isurf = -1; }
+      if (sm) {
+        if (__shfl_sync(FULL, (int)brk, j)) {
+          capped = __shfl_sync(FULL, (int)inbox, j) != 0;
+          end_side = 0;
+          break;
+        }
+        const double L = __shfl_sync(FULL, distance, j);
+        p.igrain = __shfl_sync(FULL, ig, j);
+        p.isurf = __shfl_sync(FULL, is, j);
+        const int which = p.which;
+        ++flight;
+        end_side = surface_event64(g, lambda, omega, rng, flight, L, p);
+        br2 = 0.0f;
+        if (p.which != which) gr2 = 0.0f;
+      } else if (r.fast_steps > 0 && !__shfl_sync(FULL, (int)in_gball, j - 1)) {
+        /* a new ball where the walk left the grain ball */
+        ball64(G, gp, p.which, p.pos, (float)lambda, &bx, &by, &bz, &br2, &gr2);
+      }
+    }
+    my_flights += flight;
+    my_capped += capped ? 1 : 0;
+    my_lost += end_side == 0 ? 1 : 0;
+    if (lane == 0) {
+      if (end_side == 2 || (end_side == 0 && r.ref_quirks)) atomicAdd(r.counts + task, 1ull);
+      if (end_side == 0) atomicAdd(r.lost + task, 1ull);
+    }
+  }
+  if (lane == 0) {
+    if (my_flights) atomicAdd(r.stats + 0, my_flights);
+    if (my_lost) atomicAdd(r.stats + 1, my_lost);
+    if (my_capped) atomicAdd(r.stats + 2, my_capped);
+  }
+}
+
 }  // namespace
 
 cudaError_t launch_plain_fp64(const Geo64& g, const Run64& r, cudaStream_t st, int* grid_out,
@@ -508,6 +1059,28 @@ cudaError_t launch_plain_fp64(const Geo64& g, const Run64& r, cudaStream_t st, i
   k_plain_fp64<<<(unsigned)grid, block, 0, st>>>(g, r);
   if (grid_out) *grid_out = (int)grid;
   if (block_out) *block_out = block;
+  return cudaGetLastError();
+}
+
+cudaError_t drain64_occupancy(int block, int* bps) {
+  return cudaOccupancyMaxActiveBlocksPerMultiprocessor(bps, k_drain64, block, 0);
+}
+
+cudaError_t tail64_occupancy(int block, int* bps) {
+  return cudaOccupancyMaxActiveBlocksPerMultiprocessor(bps, k_tail64, block, 0);
+}
+
+cudaError_t launch_drain64(const Geo64& g, const GeoF32& gp, const Run64& r, int grid, int block,
+                           cudaStream_t st) {
+  if (block > 256 || block % 32) return cudaErrorInvalidConfiguration;
+  k_drain64<<<grid, block, 0, st>>>(g, gp, r);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_tail64(const Geo64& g, const GeoF32& gp, const Run64& r, int grid, int block,
+                          cudaStream_t st) {
+  if (block > 256 || block % 32) return cudaErrorInvalidConfiguration;
+  k_tail64<<<grid, block, 0, st>>>(g, gp, r);
   return cudaGetLastError();
 }
 

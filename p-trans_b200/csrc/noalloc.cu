@@ -208,7 +208,8 @@ extern "C" int ptg_transmission_noalloc(ptg_handle* h, double mfp_nm, int32_t na
   if (r.nchunk > 0) {
     if (ptg::launch_persistent_fp32(v.g32, r, grid, block, smem, s) != cudaSuccess)
       return PTG_ERR_CUDA;
-    if (tgrid > 0 && (ptg::launch_tail_order(r, v.g32.box[0], s) != cudaSuccess ||
+    if (tgrid > 0 && (ptg::launch_tail_order(r.tail, ptg::kTailUnits, r.tail_cap, r.queue, r.tail_order,
+                                             v.g32.box[0], s) != cudaSuccess ||
                       ptg::launch_tail_fp32(v.g32, r, tgrid, block, smem, s) != cudaSuccess))
       return PTG_ERR_CUDA;
   }

@@ -246,6 +246,44 @@ def test_cooperative_tail_takes_the_same_trajectories(name, cap):
 
 
 
+def _fp64_structures():
+    g = geometries()
+    g["wire_specular"] = synth.nanowire(length=250.0, width=40.0, height=40.0, p_side=1.0)
+    g["voronoi_mesh"] = synth.voronoi_box(4, box=(300.0, 250.0, 250.0), seed=5, trans=0.5, tri_levels=1)
+    g["many_spheres"] = _many_spheres()
+    return g
+
+
+_FP64_OPTIONS = [dict(max_flights=37, ref_quirks=1), dict(tune_flags=2), dict(tune_flags=1),
+                 dict(bvh_leaf=-1, coop_lanes=3)]
+
+
+@pytest.mark.parametrize("k", range(17))
+@pytest.mark.parametrize("mfp", [(1e-9, 3e-8), (2e-8, 2e-6), None])
+def test_persistent_fp64_takes_the_plain_kernels_trajectories(k, mfp):
+    """The persistent FP64 kernels (safe balls, cooperative rounds, early
+    rejection of planes, box faces as slabs, BVH walks in FP32) and the plain
+    one-phonon-per-thread kernel (tune_flags bit 3) give the same counts, lost
+    counts, flights and samples: every path moves a phonon with the same FP64
+    operations.  Diffusive, long and infinite (ballistic) mean free paths in
+    every structure; as they come, and in turn with a flight cap, without the
+    tail phase, without balls, without a BVH."""
+    name = list(_fp64_structures())[k]
+    spec = synth.spectrum(7, seed=6, **(dict(mfp_lo=mfp[0], mfp_hi=mfp[1]) if mfp else {}))
+    gb = A.GeomBuf(_fp64_structures()[name])
+    run = A.make_run(kind_mfp=A.MFP_PER_MODE if mfp else A.MFP_MATTHIESSEN, nangle=5, np_=41, seed=77, stream=2,
+                     precision=A.PREC_FP64)
+    for opts in (dict(), _FP64_OPTIONS[(k + (mfp is None)) % 4]):
+        got = []
+        for flags in (8, 0):
+            with A.Handle(gb.view, spec, **dict(opts, tune_flags=opts.get("tune_flags", 0) | flags)) as h:
+                r = h.kappa(run, want_counts=True)
+                st = h.stats()
+                got.append((r["counts"], r["lost"], r["samples"], st["flights"], st["capped"]))
+        np.testing.assert_array_equal(got[1][0], got[0][0], err_msg=f"{name} {opts}")
+        assert got[1][1:] == got[0][1:], (name, opts)
+
+
 @pytest.mark.parametrize("name", ["film_periodic", "brick_tris", "capped"])
 @pytest.mark.parametrize("np_", [3, 355, 356, 2400])
 @pytest.mark.parametrize("cap", [0, 17])

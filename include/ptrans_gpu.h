@@ -415,8 +415,8 @@ int ptg_adjoint(ptg_handle* h, const ptg_run* run, ptg_adjoint_out* out);
 /*
  * Batched screening: many structures (each a built geometry with its own
  * particle count, seed and stream) share one spectrum and run settings and
- * run in ONE persistent kernel launch, replayed as a CUDA graph by
- * ptg_batch_run.  Each geometry gets exactly the counts of its own ptg_kappa
+ * run in ONE persistent transport (a drain and a tail launch over all of
+ * them), replayed as a CUDA graph by ptg_batch_run.  Each geometry gets exactly the counts of its own ptg_kappa
  * run with the same np, seed and stream (the FP32 kernel), i.e. the
  * reference's RayTrace repeated per structure (src/RTMCphon.f90:3334-3433).
  * The run's np, seed and stream are ignored (per item instead); the tables

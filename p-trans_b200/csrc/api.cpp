@@ -684,15 +684,16 @@ int run_transport(ptg_handle* h, const Transport& T) {
                           sizeof(int) * ptg::kTailOrderExtra));
         r.tail = h->tail.as<float4>();
         r.tail_order = reinterpret_cast<int*>(r.tail + (size_t)ptg::kTail64Units * r.tail_cap);
+        CU(cudaMemsetAsync(r.tail_order + r.tail_cap, 0, sizeof(int) * ptg::kTailOrderExtra, h->stream));
         r.grace_steps = ptg::grace_passes(norder * T.np_local, (int64_t)tgrid * (block / 32));
       }
       CU(ptg::launch_drain64(h->g64, h->g32, r, grid, block, h->stream));
       if (coop_lanes > 0) {
         CU(ptg::launch_tail_order(r.tail, ptg::kTail64Units, r.tail_cap, r.queue, r.tail_order,
-                                  h->g32.box[0], h->stream));
+                                  h->stream));
         CU(ptg::launch_tail64(h->g64, h->g32, r, tgrid, block, h->stream));
       }
-      h->last.launches = coop_lanes > 0 ? 5 : 2;
+      h->last.launches = coop_lanes > 0 ? 4 : 2;
     }
     CU(cudaEventRecord(h->ev[1], h->stream));
     h->last.grid = grid;
@@ -748,6 +749,7 @@ int run_transport(ptg_handle* h, const Transport& T) {
       r.tail = h->tail.as<float4>();
       r.tail_cap = grid * block;
       r.tail_order = reinterpret_cast<int*>(r.tail + (size_t)ptg::kTailUnits * r.tail_cap);
+      CU(cudaMemsetAsync(r.tail_order + r.tail_cap, 0, sizeof(int) * ptg::kTailOrderExtra, h->stream));
     }
     int tgrid = 0;
     if (tail) {
@@ -764,14 +766,14 @@ int run_transport(ptg_handle* h, const Transport& T) {
       CU(cudaEventRecord(h->ev[4], h->stream));
       if (tail) {
         CU(ptg::launch_tail_order(r.tail, ptg::kTailUnits, r.tail_cap, r.queue, r.tail_order,
-                                  h->g32.box[0], h->stream));
+                                  h->stream));
         CU(ptg::launch_tail_fp32(h->g32, r, tgrid, block, smem, h->stream, T.mode));
       }
     }
     CU(cudaEventRecord(h->ev[1], h->stream));
     h->last.grid = grid;
     h->last.block = block;
-    h->last.launches = (work ? (tail ? 4 : 1) : 0) + (r.nchunk > 0 ? 1 : 0);
+    h->last.launches = (work ? (tail ? 3 : 1) : 0) + (r.nchunk > 0 ? 1 : 0);
     h->fp32_split = work;
     h->tail_cap = tail ? r.tail_cap : 0;
   }

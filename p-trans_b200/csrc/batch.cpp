@@ -10,7 +10,7 @@
  * geometries with very uneven sample counts and mean free paths share the
  * GPU without a tail per geometry.  Set-up builds every table once; each
  * ptg_batch_run replays one graph: clear the tallies, the batched transport
- * kernel, the batched FP64 kappa reduction (effectiveMFP + the kappa sum,
+ * (drain phase, order, tail phase), the batched FP64 kappa reduction (effectiveMFP + the kappa sum,
  * :2418-2451, :2645-2755) and the copy of the results to pinned memory.
  */
 #include <cuda_runtime.h>
@@ -53,7 +53,11 @@ struct ptg_batch {
   Dev coef, K, W, mfp, bin, grid, tc, kv, bw, bv, emfp, result, np_geo, dS_geo, tnorm_geo;
   double* host_result = nullptr;              /* pinned */
   unsigned long long* host_stats = nullptr;   /* pinned */
-  int launch_grid = 0;
+  /* grids of the drain and tail phases per kernel mode (forward, list,
+     adjoint; tail 0: none) and the tail list they share, with its order */
+  int drain_grid[3] = {0, 0, 0}, tail_grid[3] = {0, 0, 0};
+  Dev tail;
+  int64_t samples = 0;
   bool bvh = false;   /* a BVH or capped cylinders: the kernel built for them */
   /* what the per-geometry adjoint needs besides the forward's tables */
   ptg::SpecSoA spec;
@@ -87,6 +91,32 @@ struct ptg_batch {
       return e_ == cudaErrorMemoryAllocation ? PTG_ERR_NOMEM : PTG_ERR_CUDA;  \
     }                                                                         \
   } while (0)
+
+/* The transport of a batch on its stream: drain phase, order of the tail list,
+   tail phase (as for a single structure: api.cpp).  Without the tail the last
+   long walks of the strongly diffusive modes, up to 2e5 flights, ended one
+   lane each while the rest of the GPU was idle (64 films, 1e7 samples: 55 ->
+   20 ms). */
+static cudaError_t launch_phases(ptg_batch* b, ptg::RunF32 r, int mode) {
+  const int block = 256;
+  r.tail = b->tail.as<float4>();
+  r.tail_cap = b->drain_grid[mode] * block;
+  r.tail_order = reinterpret_cast<int*>(r.tail + (size_t)ptg::kTailUnits * r.tail_cap);
+  const int tgrid = r.coop_lanes > 0 ? b->tail_grid[mode] : 0;
+  if (tgrid == 0) r.coop_lanes = 0;
+  r.grace_steps =
+      mode == ptg::MODE_FORWARD ? ptg::grace_passes(b->samples, (int64_t)tgrid * (block / 32)) : 0;
+  cudaError_t e = cudaMemsetAsync(b->queue.p, 0, sizeof(int) * 8, b->stream);
+  if (e == cudaSuccess && tgrid > 0)
+    e = cudaMemsetAsync(r.tail_order + r.tail_cap, 0, sizeof(int) * ptg::kTailOrderExtra, b->stream);
+  if (e == cudaSuccess)
+    e = ptg::launch_persistent_batch(r, b->drain_grid[mode], block, b->stream, b->bvh, mode, false);
+  if (e == cudaSuccess && tgrid > 0)
+    e = ptg::launch_tail_order(r.tail, ptg::kTailUnits, r.tail_cap, r.queue, r.tail_order, b->stream);
+  if (e == cudaSuccess && tgrid > 0)
+    e = ptg::launch_persistent_batch(r, tgrid, block, b->stream, b->bvh, mode, true);
+  return e;
+}
 
 extern "C" int ptg_batch_create(const ptg_batch_item* items, int32_t nitems,
                                 const ptg_spectrum* spec, const ptg_run* run,
@@ -202,6 +232,7 @@ extern "C" int ptg_batch_create(const ptg_batch_item* items, int32_t nitems,
       const int g = task_geo[od.t];
       const int64_t npl = items[g].np > run->rank ? (items[g].np - run->rank + run->nranks - 1) / run->nranks : 0;
       if (npl > 2147483647LL) { delete b; return PTG_ERR_INVALID; }
+      b->samples += npl;
       for (int64_t j = 0; j < npl; j += csz)
         chunks.push_back(make_int4((int)od.t, (int)j, (int)std::min(csz, npl - j), 0));
     }
@@ -274,6 +305,7 @@ extern "C" int ptg_batch_create(const ptg_batch_item* items, int32_t nitems,
     const int rt = o.regen_threshold > 0 ? o.regen_threshold : ptg::kDefaultRegen;
     r.regen_threshold = rt > 32 ? 32 : rt;
     r.fast_steps = (o.tune_flags & 1) ? 0 : (o.fast_steps > 0 ? o.fast_steps : ptg::kDefaultFastSteps);
+    r.coop_lanes = (o.tune_flags & 2) ? 0 : (o.coop_lanes > 0 ? std::min(o.coop_lanes, 32) : 32);
     r.counts = b->counts.as<unsigned long long>();
     r.lost = b->lost.as<unsigned long long>();
     r.stats = b->stats.as<unsigned long long>();
@@ -310,12 +342,19 @@ extern "C" int ptg_batch_create(const ptg_batch_item* items, int32_t nitems,
     b->run = *run;
     if (run->kind_mfp == PTG_MFP_GRID) b->mfp_grid.assign(run->mfp_grid_nm, run->mfp_grid_nm + ns);
     b->run.mfp_grid_nm = b->mfp_grid.empty() ? nullptr : b->mfp_grid.data();
-    int bps = 0;
-    BCU(ptg::persistent_batch_occupancy(256, &bps, b->bvh));
-    if (o.blocks_per_sm > 0 && o.blocks_per_sm < bps) bps = o.blocks_per_sm;
-    if (bps < 1) bps = 1;
-    b->launch_grid = b->num_sms * bps;
-  
+    int most = 0;
+    for (int mode : {ptg::MODE_FORWARD, ptg::MODE_LIST, ptg::MODE_ADJOINT}) {
+      int bps = 0, tbps = 0;
+      BCU(ptg::persistent_batch_occupancy(256, &bps, b->bvh, mode, false));
+      BCU(ptg::persistent_batch_occupancy(256, &tbps, b->bvh, mode, true));
+      if (mode == ptg::MODE_FORWARD && o.blocks_per_sm > 0 && o.blocks_per_sm < bps) bps = o.blocks_per_sm;
+      b->drain_grid[mode] = b->num_sms * std::max(bps, 1);
+      b->tail_grid[mode] = b->num_sms * std::max(tbps, 1);
+      most = std::max(most, b->drain_grid[mode] * 256);
+    }
+    BCU(b->tail.alloc((sizeof(float4) * ptg::kTailUnits + sizeof(int)) * (size_t)most +
+                      sizeof(int) * ptg::kTailOrderExtra));
+
     /* capture: clear tallies, transport, reduction, results to pinned memory */
     const unsigned long long init[16] = {0, 0, 0, 0, 0, ~0ull, ~0ull, 0, 0, 0, 0, 0, 0, 0, 0, 0};
     static_assert(sizeof(init) == 16 * sizeof(unsigned long long), "stats layout");
@@ -327,8 +366,7 @@ extern "C" int ptg_batch_create(const ptg_batch_item* items, int32_t nitems,
     if (ce == cudaSuccess)
       ce = cudaMemsetAsync(dstats, 0, sizeof(unsigned long long) * ptg::kStatSlots, b->stream);
     if (ce == cudaSuccess) ce = cudaMemsetAsync(dstats + 5, 0xFF, sizeof(unsigned long long) * 2, b->stream);
-    if (ce == cudaSuccess) ce = cudaMemsetAsync(b->queue.p, 0, sizeof(int) * 8, b->stream);
-    if (ce == cudaSuccess && r.nchunk > 0) ce = ptg::launch_persistent_batch(r, b->launch_grid, 256, b->stream, b->bvh);
+    if (ce == cudaSuccess && r.nchunk > 0) ce = launch_phases(b, r, ptg::MODE_FORWARD);
     if (ce == cudaSuccess) ce = ptg::launch_kappa_reduce_batch(rb, b->stream);
     if (ce == cudaSuccess)
       ce = cudaMemcpyAsync(b->host_result, b->result.p, sizeof(double) * nres, cudaMemcpyDeviceToHost,
@@ -393,26 +431,21 @@ extern "C" int ptg_batch_run(ptg_batch* b, ptg_batch_out* out) {
   }
 }
 
-/* One batched transport launch outside the graph (list or adjoint mode):
+/* One batched transport outside the graph (list or adjoint mode):
    clears the tallies, statistics and queue, launches, waits; *ms receives
    its device time and st its statistics. */
 static int batch_launch(ptg_batch* b, const ptg::RunF32& r, int mode, unsigned long long* st,
                         float* ms) {
   const size_t ntot = (size_t)b->ngeo * (size_t)b->ntask_per_geo;
   unsigned long long* dstats = b->stats.as<unsigned long long>();
-  int bps = 0;
-  if (ptg::persistent_batch_occupancy(256, &bps, b->bvh, mode) != cudaSuccess) return PTG_ERR_CUDA;
-  if (bps < 1) bps = 1;
   if (cudaMemsetAsync(b->counts.p, 0, sizeof(unsigned long long) * ntot, b->stream) != cudaSuccess ||
       cudaMemsetAsync(b->lost.p, 0, sizeof(unsigned long long) * ntot, b->stream) != cudaSuccess ||
       cudaMemsetAsync(dstats, 0, sizeof(unsigned long long) * ptg::kStatSlots, b->stream) != cudaSuccess ||
       cudaMemsetAsync(dstats + 5, 0xFF, sizeof(unsigned long long) * 2, b->stream) != cudaSuccess ||
-      cudaMemsetAsync(b->queue.p, 0, sizeof(int) * 8, b->stream) != cudaSuccess ||
       cudaEventRecord(b->ev0, b->stream) != cudaSuccess)
     return PTG_ERR_CUDA;
   const bool work = mode == ptg::MODE_ADJOINT ? r.alist_n > 0 : r.nchunk > 0;
-  if (work && ptg::launch_persistent_batch(r, b->num_sms * bps, 256, b->stream, b->bvh, mode) != cudaSuccess)
-    return PTG_ERR_CUDA;
+  if (work && launch_phases(b, r, mode) != cudaSuccess) return PTG_ERR_CUDA;
   if (cudaEventRecord(b->ev1, b->stream) != cudaSuccess ||
       cudaMemcpyAsync(st, dstats, sizeof(unsigned long long) * ptg::kStatSlots, cudaMemcpyDeviceToHost,
                       b->stream) != cudaSuccess ||

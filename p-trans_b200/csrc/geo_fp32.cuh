@@ -232,6 +232,20 @@ __device__ __forceinline__ float safety(const G_t& G, int grain, float px, float
   return fminf(dbox, dc) - 4.0f * eps;
 }
 
+/* Buckets of the tail order: a quarter octave of the expected walk each. */
+constexpr int kOrderBuckets = 128;
+static_assert(2 * kOrderBuckets == kTailOrderExtra, "tail order histogram and cursors");
+
+/* Bucket of a phonon's expected remaining walk.  A diffusive phonon at x
+   between the baths at 0 and L takes about 1.5 x (L - x) / MFP^2 more flights
+   to leave (the exit time of a random walk whose flights move it by
+   2 MFP^2 / 3 squared along x); walls and holes stretch the walk, but the
+   phonons the tail phase waits for are those that rank high on it. */
+__device__ __forceinline__ int order_bucket(float x, float x_len, float lam) {
+  const float w = __fdividef(fmaxf(x * (x_len - x), 0.0f), lam * lam);
+  return w > 1.0f ? min(kOrderBuckets - 1, (int)(4.0f * __log2f(w))) : 0;
+}
+
 __device__ __forceinline__ unsigned lanemask_lt() {
   unsigned m;
   asm volatile("mov.u32 %0, %%lanemask_lt;" : "=r"(m));

@@ -246,13 +246,14 @@ cudaError_t launch_persistent_fp32(const GeoF32& g, const RunF32& r, int grid, i
                                    size_t smem, cudaStream_t st, int mode = MODE_FORWARD);
 /* The tail phase after it (forward, list and adjoint modes): the phonons
    the drain phase left in r.tail, one per warp. */
-/* Orders the tail list for the tail phase (r.tail_order: tail_cap ints and
-   kTailOrderExtra more for a histogram and cursors): longest expected
-   remaining walk first.  A memset and two kernels between the drain and the
-   tail launch on the same stream; x_len is the box length along x. */
+/* Orders the tail list for the tail phase, longest expected remaining walk
+   first: tail_cap ints, then kTailOrderExtra for the buckets' histogram, which
+   the drain phase fills as it hands phonons over, and their cursors (both
+   zeroed by the caller before the drain).  One kernel between the drain and
+   the tail launch on the same stream. */
 constexpr int kTailOrderExtra = 256;
-cudaError_t launch_tail_order(float4* tail, int units, int tail_cap, const int* queue, int32_t* order,
-                              float x_len, cudaStream_t st);
+cudaError_t launch_tail_order(const float4* tail, int units, int tail_cap, const int* queue,
+                              int32_t* order, cudaStream_t st);
 /* The FP64 pair: the same queue and list, FP64 flights; the blob of g32 gives
    the bounds for balls and BVH walks. */
 cudaError_t drain64_occupancy(int block, int* blocks_per_sm);
@@ -269,18 +270,17 @@ cudaError_t tail_occupancy(int block, size_t smem, int* blocks_per_sm, int mode 
    forward, list (ids of transmitted samples as (global task << 32) |
    particle) or adjoint replay of such a list. */
 cudaError_t launch_persistent_batch(const RunF32& r, int grid, int block, cudaStream_t st,
-                                    bool bvh, int mode = MODE_FORWARD);
-cudaError_t persistent_batch_occupancy(int block, int* blocks_per_sm, bool bvh,
-                                       int mode = MODE_FORWARD);
+                                    bool bvh, int mode, bool tail);
+cudaError_t persistent_batch_occupancy(int block, int* blocks_per_sm, bool bvh, int mode, bool tail);
 /* float4 per phonon in the tail list: the state of a phonon handed from the
    drain phase to the tail phase (position, direction, free path, MFP, the
    ball centre and radii, grain, last surface, task, omega, sample id,
    flight, adjoint terms, second ball). */
 constexpr int kTailUnits = 7;
-/* ... and in the FP64 one: (x, ball centre), (ball radii squared, -, MFP) in
-   FP32, then position, direction, free path and MFP in FP64, (grain and
-   surface last met, order bucket, grain), (task, sample id, flight).  Both
-   layouts hold x at word 0, the MFP at word 7 and the bucket at word 26. */
+/* ... and in the FP64 one: (ball centre, ball radii squared) in FP32, then
+   position, direction, free path and MFP in FP64, (grain and surface last
+   met, order bucket, grain), (task, sample id, flight).  Both layouts hold
+   the order bucket at word 26. */
 constexpr int kTail64Units = 8;
 /* Shared memory for staged BVH nodes when the whole blob is not staged:
    64 KB, the top ten or so levels of the trees, small enough that two

@@ -1028,11 +1028,34 @@ __global__ void __launch_bounds__(kBlock,
       int c = 0;
       if (lane == 0) c = atomicAdd(r.queue + 3, 1);
       c = __shfl_sync(FULL, c, 0);
+      const int slot =
+          c >= ntail ? 0
+                     : (r.tail_order ? r.tail_order[c] : (c < nlong ? c : r.tail_cap - 1 - (c - nlong)));
+      if (BATCH && c < ntail) {
+        /* the phonon's geometry, for every lane of its rounds; a local list
+           left by the last phonon may be another geometry's */
+        const GeoEntry* ge =
+            r.geos + __ldg(r.task_geo + __float_as_int(r.tail[(size_t)kTailUnits * slot + 3].z));
+        G.base = ge->blob;
+        G.lay = ge->lay;
+        X = ge->box[0]; Y = ge->box[1]; Z = ge->box[2];
+        eps = ge->eps;
+        key.k0 = ge->k0; key.k1 = ge->k1;
+        c1 = ge->c1;
+        pmask = ge->periodic_mask;
+        nmat = ge->nmaterial;
+        flmax = ge->fast_lambda_max;
+        adj_stride = ge->nsurf + 1;
+        adj_off = ge->adj_base;
+        if (kUseList) {
+          __syncwarp();
+          if (lane == 0) coop_lmeta[threadIdx.x >> 5] = make_int4(0, -1, 0, 0);
+          __syncwarp();
+        }
+      }
       if (c >= ntail) {
         queue_done = true;
       } else if (lane == 0) {
-        const int slot =
-            r.tail_order ? r.tail_order[c] : (c < nlong ? c : r.tail_cap - 1 - (c - nlong));
         const float4* e = r.tail + (size_t)kTailUnits * slot;
         const float4 e0 = e[0], e1 = e[1], e2 = e[2], e3 = e[3], e4 = e[4];
         px = e0.x; py = e0.y; pz = e0.z; dx = e0.w;
@@ -1195,7 +1218,7 @@ __global__ void __launch_bounds__(kBlock,
        diffusive ones at once, the long-MFP ones after the passes in which
        most of them end (grace_passes), lest the last few hold their warp,
        and the drain launch, to the end */
-    if (PH == PH_DRAIN && !BATCH && MODE != MODE_TRACE && queue_done && r.coop_lanes > 0 &&
+    if (PH == PH_DRAIN && MODE != MODE_TRACE && queue_done && r.coop_lanes > 0 &&
         !tail_full && __popc(__ballot_sync(FULL, alive)) <= r.coop_lanes) {
       const unsigned mw =
           __ballot_sync(FULL, alive && (lam < flmax || r.fast_steps <= 0 || grace == 0));
@@ -1234,7 +1257,9 @@ __global__ void __launch_bounds__(kBlock,
                              __int_as_float(task), omr);
           e[4] = make_float4(__uint_as_float(slo), __uint_as_float(shi), __uint_as_float(flight),
                              gr2);
-          e[6] = make_float4(g2r2, __int_as_float(gnear), 0.0f, 0.0f);
+          const int bucket = order_bucket(px, X, lam);
+          e[6] = make_float4(g2r2, __int_as_float(gnear), __int_as_float(bucket), 0.0f);
+          atomicAdd(r.tail_order + r.tail_cap + bucket, 1);
           if (MODE == MODE_ADJOINT)
             e[5] = make_float4(adj_w, adj_len, __uint_as_float(adj_npp), __int_as_float(adj_b));
           atomicAdd(r.stats + 16, (unsigned long long)flight);
@@ -1895,38 +1920,50 @@ cudaError_t launch_mode(const GeoF32& g, const RunF32& r, int grid, int block, s
   return cudaGetLastError();
 }
 
-template <int MODE>
+template <int MODE, int PH>
 cudaError_t batch_occupancy_mode(int block, int* bps, bool bvh) {
   return cudaOccupancyMaxActiveBlocksPerMultiprocessor(
       bps,
-      bvh ? k_persistent<false, MODE, true, true, PH_DRAIN>
-          : k_persistent<false, MODE, true, false, PH_DRAIN>,
+      bvh ? k_persistent<false, MODE, true, true, PH> : k_persistent<false, MODE, true, false, PH>,
       block, 0);
 }
 
-cudaError_t persistent_batch_occupancy(int block, int* bps, bool bvh, int mode) {
-  if (mode == MODE_LIST) return batch_occupancy_mode<MODE_LIST>(block, bps, bvh);
-  if (mode == MODE_ADJOINT) return batch_occupancy_mode<MODE_ADJOINT>(block, bps, bvh);
+template <int PH>
+cudaError_t batch_occupancy_phase(int block, int* bps, bool bvh, int mode) {
+  if (mode == MODE_LIST) return batch_occupancy_mode<MODE_LIST, PH>(block, bps, bvh);
+  if (mode == MODE_ADJOINT) return batch_occupancy_mode<MODE_ADJOINT, PH>(block, bps, bvh);
   if (mode != MODE_FORWARD) return cudaErrorInvalidValue;
-  return batch_occupancy_mode<MODE_FORWARD>(block, bps, bvh);
+  return batch_occupancy_mode<MODE_FORWARD, PH>(block, bps, bvh);
 }
 
-template <int MODE>
+cudaError_t persistent_batch_occupancy(int block, int* bps, bool bvh, int mode, bool tail) {
+  return tail ? batch_occupancy_phase<PH_TAIL>(block, bps, bvh, mode)
+              : batch_occupancy_phase<PH_DRAIN>(block, bps, bvh, mode);
+}
+
+template <int MODE, int PH>
 cudaError_t launch_batch_mode(const RunF32& r, int grid, int block, cudaStream_t st, bool bvh) {
   GeoF32 g;
   memset(&g, 0, sizeof(g));
-  if (bvh) k_persistent<false, MODE, true, true, PH_DRAIN><<<grid, block, 0, st>>>(g, r);
-  else k_persistent<false, MODE, true, false, PH_DRAIN><<<grid, block, 0, st>>>(g, r);
+  if (bvh) k_persistent<false, MODE, true, true, PH><<<grid, block, 0, st>>>(g, r);
+  else k_persistent<false, MODE, true, false, PH><<<grid, block, 0, st>>>(g, r);
   return cudaGetLastError();
 }
 
-cudaError_t launch_persistent_batch(const RunF32& r, int grid, int block, cudaStream_t st, bool bvh,
-                                    int mode) {
+template <int PH>
+cudaError_t launch_batch_phase(const RunF32& r, int grid, int block, cudaStream_t st, bool bvh,
+                               int mode) {
   if (block != kBlock) return cudaErrorInvalidConfiguration;
-  if (mode == MODE_LIST) return launch_batch_mode<MODE_LIST>(r, grid, block, st, bvh);
-  if (mode == MODE_ADJOINT) return launch_batch_mode<MODE_ADJOINT>(r, grid, block, st, bvh);
+  if (mode == MODE_LIST) return launch_batch_mode<MODE_LIST, PH>(r, grid, block, st, bvh);
+  if (mode == MODE_ADJOINT) return launch_batch_mode<MODE_ADJOINT, PH>(r, grid, block, st, bvh);
   if (mode != MODE_FORWARD) return cudaErrorInvalidValue;
-  return launch_batch_mode<MODE_FORWARD>(r, grid, block, st, bvh);
+  return launch_batch_mode<MODE_FORWARD, PH>(r, grid, block, st, bvh);
+}
+
+cudaError_t launch_persistent_batch(const RunF32& r, int grid, int block, cudaStream_t st, bool bvh,
+                                    int mode, bool tail) {
+  return tail ? launch_batch_phase<PH_TAIL>(r, grid, block, st, bvh, mode)
+              : launch_batch_phase<PH_DRAIN>(r, grid, block, st, bvh, mode);
 }
 
 /* The tail phase exists for the modes with cooperative rounds (forward,
@@ -1997,40 +2034,9 @@ __global__ void k_expand_chunks(const int* __restrict__ order, int norder, int p
   }
 }
 
-/* Buckets of the tail order: a quarter octave of the expected walk each. */
-constexpr int kOrderBuckets = 128;
-static_assert(2 * kOrderBuckets == kTailOrderExtra, "tail order histogram and cursors");
-
-/* Tail-list slot of hand-over c (front list, then back list) and the
-   bucket of its phonon's expected remaining walk.  A diffusive phonon at x
-   between the baths at 0 and L takes about 1.5 x (L - x) / MFP^2 more
-   flights to leave (the exit time of a random walk whose flights move it
-   by 2 MFP^2 / 3 squared along x); walls and holes stretch the walk, but the
-   phonons the tail phase waits for are those that rank high on it. */
-__device__ __forceinline__ int order_bucket(const float4* tail, int units, int slot, float x_len) {
-  const float4 e0 = tail[(size_t)units * slot];
-  const float4 e1 = tail[(size_t)units * slot + 1];
-  const float w = fmaxf(e0.x * (x_len - e0.x), 0.0f) / (e1.w * e1.w);
-  return w > 1.0f ? min(kOrderBuckets - 1, (int)(4.0f * __log2f(w))) : 0;
-}
-
 /* Hand-over c of the tail list: its slot (front list, then back list). */
 __device__ __forceinline__ int tail_slot(int c, int nlong, int tail_cap) {
   return c < nlong ? c : tail_cap - 1 - (c - nlong);
-}
-
-/* One thread per hand-over: its bucket, kept in the entry's spare word
-   (float4 6, z), and the bucket histogram. */
-__global__ void k_order_hist(float4* __restrict__ tail, int units, int tail_cap,
-                             const int* __restrict__ queue, float x_len, int* __restrict__ hist) {
-  const int nlong = min(queue[2], tail_cap);
-  const int ntail = nlong + min(queue[4], tail_cap - nlong);
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= ntail) return;
-  const int slot = tail_slot(c, nlong, tail_cap);
-  const int b = order_bucket(tail, units, slot, x_len);
-  reinterpret_cast<int*>(tail + (size_t)units * slot + 6)[2] = b;
-  atomicAdd(&hist[b], 1);
 }
 
 /* One thread per hand-over: the bucket offsets from the top bucket down
@@ -2061,14 +2067,10 @@ __global__ void k_order_scatter(const float4* __restrict__ tail, int units, int 
 }
 }  // namespace
 
-cudaError_t launch_tail_order(float4* tail, int units, int tail_cap, const int* queue, int32_t* order,
-                              float x_len, cudaStream_t st) {
-  /* the histogram and the bucket cursors follow the order array */
+cudaError_t launch_tail_order(const float4* tail, int units, int tail_cap, const int* queue,
+                              int32_t* order, cudaStream_t st) {
   int* hist = order + tail_cap;
-  cudaError_t e = cudaMemsetAsync(hist, 0, sizeof(int) * 2 * kOrderBuckets, st);
-  if (e != cudaSuccess) return e;
   const unsigned blocks = (unsigned)((tail_cap + 255) / 256);
-  k_order_hist<<<blocks, 256, 0, st>>>(tail, units, tail_cap, queue, x_len, hist);
   k_order_scatter<<<blocks, 256, 0, st>>>(tail, units, tail_cap, queue, hist, hist + kOrderBuckets,
                                           order);
   return cudaGetLastError();

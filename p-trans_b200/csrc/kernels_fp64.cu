@@ -804,14 +804,16 @@ __global__ void __launch_bounds__(256, 2) k_drain64(Geo64 g, GeoF32 gp, Run64 r)
         /* the list has a slot for every lane of the grid */
         if (give && idx < r.tail_cap) {
           float4* e = r.tail + (size_t)kTail64Units * (r.tail_cap - 1 - idx);
-          e[0] = make_float4((float)p.pos[0], bx, by, bz);
-          e[1] = make_float4(br2, gr2, 0.0f, (float)lambda);
+          e[0] = make_float4(bx, by, bz, br2);
+          e[1] = make_float4(gr2, 0.0f, 0.0f, 0.0f);
           e[2] = pack2(p.pos[0], p.pos[1]);
           e[3] = pack2(p.pos[2], p.dir[0]);
           e[4] = pack2(p.dir[1], p.dir[2]);
           e[5] = pack2(p.fp, lambda);
-          e[6] = make_float4(__int_as_float(p.igrain), __int_as_float(p.isurf), 0.0f,
-                             __int_as_float(p.which));
+          const int bucket = order_bucket((float)p.pos[0], gp.box[0], lam);
+          e[6] = make_float4(__int_as_float(p.igrain), __int_as_float(p.isurf),
+                             __int_as_float(bucket), __int_as_float(p.which));
+          atomicAdd(r.tail_order + r.tail_cap + bucket, 1);
           e[7] = make_float4(__int_as_float(task), __uint_as_float((uint32_t)sample),
                              __uint_as_float((uint32_t)(sample >> 32)), __uint_as_float(flight));
           alive = false;
@@ -922,7 +924,7 @@ __global__ void __launch_bounds__(256, 2) k_tail64(Geo64 g, GeoF32 gp, Run64 r) 
     if (c >= ntail) break;
     const float4* e = r.tail + (size_t)kTail64Units * r.tail_order[c];
     const float4 e0 = e[0], e1 = e[1], e6 = e[6], e7 = e[7];
-    float bx = e0.y, by = e0.z, bz = e0.w, br2 = e1.x, gr2 = e1.y;
+    float bx = e0.x, by = e0.y, bz = e0.z, br2 = e0.w, gr2 = e1.x;
     Ph64 p;
     double lambda;
     unpack2(e[2], &p.pos[0], &p.pos[1]);

@@ -199,6 +199,8 @@ extern "C" int ptg_transmission_noalloc(ptg_handle* h, double mfp_nm, int32_t na
     r.tail = reinterpret_cast<float4*>(base + kOffTail);
     r.tail_cap = std::min(kMaxTail, grid * block);
     r.tail_order = reinterpret_cast<int*>(base + kOffOrder);
+    if (cudaMemsetAsync(r.tail_order + r.tail_cap, 0, sizeof(int) * ptg::kTailOrderExtra, s) != cudaSuccess)
+      return PTG_ERR_CUDA;
     int tbps = 0;
     if (ptg::tail_occupancy(block, smem, &tbps, ptg::MODE_FORWARD, v.g32.has_ext != 0, v.g32.stage_smem != 0) != cudaSuccess)
       return PTG_ERR_CUDA;
@@ -208,8 +210,7 @@ extern "C" int ptg_transmission_noalloc(ptg_handle* h, double mfp_nm, int32_t na
   if (r.nchunk > 0) {
     if (ptg::launch_persistent_fp32(v.g32, r, grid, block, smem, s) != cudaSuccess)
       return PTG_ERR_CUDA;
-    if (tgrid > 0 && (ptg::launch_tail_order(r.tail, ptg::kTailUnits, r.tail_cap, r.queue, r.tail_order,
-                                             v.g32.box[0], s) != cudaSuccess ||
+    if (tgrid > 0 && (ptg::launch_tail_order(r.tail, ptg::kTailUnits, r.tail_cap, r.queue, r.tail_order, s) != cudaSuccess ||
                       ptg::launch_tail_fp32(v.g32, r, tgrid, block, smem, s) != cudaSuccess))
       return PTG_ERR_CUDA;
   }
@@ -241,7 +242,7 @@ extern "C" int ptg_transmission_noalloc(ptg_handle* h, double mfp_nm, int32_t na
   L->coop_flights = sv[13];
   L->box_tests = sv[14];
   L->surface_tests = sv[15];
-  L->launches = 1 + (r.nchunk > 0 ? (tgrid > 0 ? 4 : 1) : 0);
+  L->launches = 1 + (r.nchunk > 0 ? (tgrid > 0 ? 3 : 1) : 0);
   L->grid = grid;
   L->block = block;
   L->h2d_bytes = sizeof(double) * nmode;

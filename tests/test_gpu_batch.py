@@ -81,3 +81,36 @@ def test_batch_adjoint_equals_individual_adjoints():
         # where the single run's tail phase adds a round's flights by warp shuffles
         assert abs(ba["dk_dscale"][g] - sa["dk_dscale"]) <= 1e-3 * sa["dk_dscale_stderr"] + 1e-5 * abs(sa["dk_dscale"])
     assert ba["replayed"] == replayed
+
+
+@pytest.mark.parametrize("kind", ["films", "bvh"])
+@pytest.mark.parametrize("cap", [0, 40])
+def test_batched_tail_phase_takes_the_same_trajectories(kind, cap):
+    """A batch hands its last phonons to a tail phase whose warps switch
+    geometry from phonon to phonon; without it (tune_flags bit 1) every phonon
+    ends on one lane.  Counts, flights and lost phonons are equal, and so is
+    the replayed sample set of the adjoint, in films and where several
+    geometries with the same grain numbers keep a BVH and local lists."""
+    if kind == "films":
+        models, nps = synth.film_batch(7, seed=4, n_modes=12, nangle=5, samples_lo=500, samples_hi=9000)
+    else:
+        models = [synth.cube_lattice(n=n, l=300.0, fill=f, trans=0.3, spec=0.2, p_wall=0.3)
+                  for n, f in ((3, 0.5), (4, 0.4), (3, 0.3))]
+        models.append(synth.spheres_cylinders_box(n_spheres=4, n_cylinders=5, l=300.0, seed=3, r_sphere=(15.0, 35.0),
+                                                  r_cylinder=20.0, length=(50.0, 150.0), trans=0.3, p_wall=0.2))
+        nps = [37, 90, 61, 44]
+    spec = synth.spectrum(12, seed=5, mfp_lo=1e-9, mfp_hi=1e-7)
+    bufs = [A.GeomBuf(m) for m in models]
+    run = A.make_run(kind_mfp=A.MFP_PER_MODE, nangle=5, np_=1)
+    got = []
+    for flags in (2, 0):
+        with A.Batch([b.view for b in bufs], nps, [9 + i for i in range(len(bufs))], [0] * len(bufs), spec, run,
+                     max_flights=cap, tune_flags=flags) as bt:
+            r = bt.run(want_counts=True)
+            again = bt.run(want_counts=True)
+            a = bt.adjoint()
+        np.testing.assert_array_equal(again["counts"], r["counts"])
+        got.append((r["counts"], r["flights"], r["lost"], r["samples"], a["replayed"], a["mismatched"], a["flights"]))
+    np.testing.assert_array_equal(got[1][0], got[0][0])
+    assert got[1][1:] == got[0][1:]
+    assert got[0][5] == 0

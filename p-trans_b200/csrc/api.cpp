@@ -165,6 +165,44 @@ inline float4 i4(int a, int b, int c, int d) {
 
 namespace ptg {
 
+/* The facet planes of a convex grain given as a mesh: the distinct oriented
+   planes of its candidates when all of them are polygons, on at most
+   kMaxPlanes planes (within tol) that no vertex lies in front of, else none.
+   A polyhedral grain out of a mesher has thousands of triangles on a dozen
+   planes.  A plane's distance bounds that of every polygon on it (tightly, the
+   grain being convex), and a flight whose end lies behind all of them has met
+   none.  Other grains keep the tree searches: in a matrix around inclusions
+   the planes run through the space between them. */
+static void facet_planes(const GeomSoA& G, const std::vector<int>& cand, int cb, int ce, double tol,
+                         std::vector<float4>* out) {
+  std::vector<double> pl;
+  for (int i = cb; i < ce; ++i) {
+    const int s = cand[i];
+    if (G.shape[s] != PTG_SHAPE_POLYGON) return;
+    const double* n = &G.normal[3 * s];
+    const double* v = &G.vertex[3 * (size_t)G.vertex_begin[s]];
+    auto on = [&](const double* p) {
+      if (fabs(p[0] - n[0]) > 1e-6 || fabs(p[1] - n[1]) > 1e-6 || fabs(p[2] - n[2]) > 1e-6) return false;
+      for (int k = 0; k < G.nvertex[s]; ++k)
+        if (!(fabs(p[0] * v[3 * k] + p[1] * v[3 * k + 1] + p[2] * v[3 * k + 2] - p[3]) <= tol)) return false;
+      return true;
+    };
+    bool found = false;
+    for (size_t k = 0; k < pl.size() && !found; k += 4) found = on(&pl[k]);
+    if (found) continue;
+    const double own[4] = {n[0], n[1], n[2], n[0] * v[0] + n[1] * v[1] + n[2] * v[2]};
+    if ((int)pl.size() >= 4 * kMaxPlanes || !on(own)) return;
+    pl.insert(pl.end(), own, own + 4);
+  }
+  for (int i = cb; i < ce; ++i) {
+    const double* v = &G.vertex[3 * (size_t)G.vertex_begin[cand[i]]];
+    for (int j = 0; j < 3 * G.nvertex[cand[i]]; j += 3)
+      for (size_t k = 0; k < pl.size(); k += 4)
+        if (pl[k] * v[j] + pl[k + 1] * v[j + 1] + pl[k + 2] * v[j + 2] - pl[k + 3] > tol) return;
+  }
+  for (size_t k = 0; k < pl.size(); k += 4) out->push_back(f4(pl[k], pl[k + 1], pl[k + 2], pl[k + 3]));
+}
+
 /* The FP32 geometry blob of a built geometry (host copy) and its layout. */
 int blob_from_geometry(const GeomSoA& G, int bvh_leaf, std::vector<float4>* out,
                        BlobLayout* lay_out, std::string* why) {
@@ -266,8 +304,8 @@ int blob_from_geometry(const GeomSoA& G, int bvh_leaf, std::vector<float4>* out,
   cb[ngt] = (int)cand.size();
   /* BVH over the candidates of every large grain; its leaves reorder the
      grain's candidate list */
-  std::vector<int> root(ngt, -1);
-  std::vector<float4> nodes;
+  std::vector<int> root(ngt, -1), plane_begin(ngt + 1, 0);
+  std::vector<float4> nodes, planes;
   if (bvh_leaf >= 0) {
     const int leaf = bvh_leaf > 0 ? bvh_leaf : kBvhDefaultLeaf;
     const double S = std::max(G.box[0], std::max(G.box[1], G.box[2]));
@@ -321,6 +359,13 @@ int blob_from_geometry(const GeomSoA& G, int bvh_leaf, std::vector<float4>* out,
       nodes.insert(nodes.end(), gn.begin(), gn.end());
     }
   }
+  for (int g = 0; g < ngt; ++g) {
+    plane_begin[g] = (int)planes.size();
+    if (root[g] >= 0)
+      facet_planes(G, cand, cb[g], cb[g + 1],
+                   std::max(G.box[0], std::max(G.box[1], G.box[2])) / 1048576.0 * 0.25, &planes);
+  }
+  plane_begin[ngt] = (int)planes.size();
   if (!nodes.empty()) {
     /* breadth first over all grains' trees (every root first, then level
        by level): the front of the node region holds the top levels of
@@ -386,8 +431,11 @@ int blob_from_geometry(const GeomSoA& G, int bvh_leaf, std::vector<float4>* out,
   L.cand = L.cand_begin + units_of_ints(cb.size());
   L.start = L.cand + units_of_ints(cand.size() ? cand.size() : 1);
   L.bvh_root = L.start + (int)(start.size() ? start.size() : 1);
-  L.bvh_node = L.bvh_root + units_of_ints(root.size());
+  L.plane_begin = L.bvh_root + units_of_ints(root.size());
+  L.plane = L.plane_begin + units_of_ints(plane_begin.size());
+  L.bvh_node = L.plane + (int)(planes.size() ? planes.size() : 1);
   L.total = L.bvh_node + (int)(nodes.size() ? nodes.size() : 1);
+  L.nplane = (int)planes.size();
   L.nbvh = (int)(nodes.size() / 2);
   L.ncap = 0;
   for (int s = 0; s < ns; ++s) L.ncap += G.shape[s] == PTG_SHAPE_CAPPED ? 1 : 0;
@@ -400,6 +448,8 @@ int blob_from_geometry(const GeomSoA& G, int bvh_leaf, std::vector<float4>* out,
   if (!cand.empty()) memcpy(&blob[L.cand], cand.data(), cand.size() * 4);
   std::copy(start.begin(), start.end(), blob.begin() + L.start);
   memcpy(&blob[L.bvh_root], root.data(), root.size() * 4);
+  memcpy(&blob[L.plane_begin], plane_begin.data(), plane_begin.size() * 4);
+  std::copy(planes.begin(), planes.end(), blob.begin() + L.plane);
   std::copy(nodes.begin(), nodes.end(), blob.begin() + L.bvh_node);
   *out = std::move(blob);
   *lay_out = L;
@@ -445,7 +495,7 @@ int build_blob(ptg_handle* h) {
   g32.igrain_fill = G.igrain_fill;
   g32.nmaterial = G.nmaterial;
   g32.stage_smem = h->blob_bytes <= 96 * 1024 ? 1 : 0;
-  g32.has_ext = (L.nbvh > 0 || L.ncap > 0) ? 1 : 0;
+  g32.has_ext = L.nplane > 0 ? 2 : (L.nbvh > 0 || L.ncap > 0) ? 1 : 0;
   /* a blob too large to stage keeps the top levels of its BVHs (the front of
      the breadth-first node region) in shared memory */
   g32.node_stage = (!g32.stage_smem && L.nbvh > 0) ? std::min(2 * L.nbvh, ptg::kNodeStageUnits) : 0;
@@ -735,7 +785,7 @@ int run_transport(ptg_handle* h, const Transport& T) {
     r.nsurf = h->geom.nsurf();
     const size_t smem = ptg::dynamic_smem_bytes(h->g32, h->blob_bytes);
     int bps = 0;
-    CU(ptg::persistent_occupancy(block, smem, &bps, T.mode, h->g32.has_ext != 0, h->g32.stage_smem != 0));
+    CU(ptg::persistent_occupancy(block, smem, &bps, T.mode, h->g32.has_ext, h->g32.stage_smem != 0));
     if (h->opt.blocks_per_sm > 0 && h->opt.blocks_per_sm < bps) bps = h->opt.blocks_per_sm;
     if (bps < 1) bps = 1;
     const int grid = h->num_sms * bps;
@@ -754,7 +804,7 @@ int run_transport(ptg_handle* h, const Transport& T) {
     int tgrid = 0;
     if (tail) {
       int tbps = 0;
-      CU(ptg::tail_occupancy(block, smem, &tbps, T.mode, h->g32.has_ext != 0, h->g32.stage_smem != 0));
+      CU(ptg::tail_occupancy(block, smem, &tbps, T.mode, h->g32.has_ext, h->g32.stage_smem != 0));
       tgrid = h->num_sms * (tbps < 1 ? 1 : tbps);
       if (T.mode == ptg::MODE_FORWARD)
         r.grace_steps = ptg::grace_passes(norder * T.np_local, (int64_t)tgrid * (block / 32));

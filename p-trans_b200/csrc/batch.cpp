@@ -58,7 +58,7 @@ struct ptg_batch {
   int drain_grid[3] = {0, 0, 0}, tail_grid[3] = {0, 0, 0};
   Dev tail;
   int64_t samples = 0;
-  bool bvh = false;   /* a BVH or capped cylinders: the kernel built for them */
+  int ext = 0;   /* which kernels its geometries need (GeoF32.has_ext) */
   /* what the per-geometry adjoint needs besides the forward's tables */
   ptg::SpecSoA spec;
   ptg_run run;
@@ -110,11 +110,11 @@ static cudaError_t launch_phases(ptg_batch* b, ptg::RunF32 r, int mode) {
   if (e == cudaSuccess && tgrid > 0)
     e = cudaMemsetAsync(r.tail_order + r.tail_cap, 0, sizeof(int) * ptg::kTailOrderExtra, b->stream);
   if (e == cudaSuccess)
-    e = ptg::launch_persistent_batch(r, b->drain_grid[mode], block, b->stream, b->bvh, mode, false);
+    e = ptg::launch_persistent_batch(r, b->drain_grid[mode], block, b->stream, b->ext, mode, false);
   if (e == cudaSuccess && tgrid > 0)
     e = ptg::launch_tail_order(r.tail, ptg::kTailUnits, r.tail_cap, r.queue, r.tail_order, b->stream);
   if (e == cudaSuccess && tgrid > 0)
-    e = ptg::launch_persistent_batch(r, tgrid, block, b->stream, b->bvh, mode, true);
+    e = ptg::launch_persistent_batch(r, tgrid, block, b->stream, b->ext, mode, true);
   return e;
 }
 
@@ -176,7 +176,7 @@ extern "C" int ptg_batch_create(const ptg_batch_item* items, int32_t nitems,
       ptg::GeoEntry& e = entries[g];
       memset(&e, 0, sizeof(e));
       e.lay = L;
-      if (L.nbvh > 0 || L.ncap > 0) b->bvh = true;
+      if (L.nbvh > 0 || L.ncap > 0) b->ext = std::max(b->ext, L.nplane > 0 ? 2 : 1);
       for (int d = 0; d < 3; ++d) e.box[d] = (float)G.box[d];
       e.scope[0] = (float)G.scope[0];
       e.scope[1] = (float)G.scope[1];
@@ -345,8 +345,8 @@ extern "C" int ptg_batch_create(const ptg_batch_item* items, int32_t nitems,
     int most = 0;
     for (int mode : {ptg::MODE_FORWARD, ptg::MODE_LIST, ptg::MODE_ADJOINT}) {
       int bps = 0, tbps = 0;
-      BCU(ptg::persistent_batch_occupancy(256, &bps, b->bvh, mode, false));
-      BCU(ptg::persistent_batch_occupancy(256, &tbps, b->bvh, mode, true));
+      BCU(ptg::persistent_batch_occupancy(256, &bps, b->ext, mode, false));
+      BCU(ptg::persistent_batch_occupancy(256, &tbps, b->ext, mode, true));
       if (mode == ptg::MODE_FORWARD && o.blocks_per_sm > 0 && o.blocks_per_sm < bps) bps = o.blocks_per_sm;
       b->drain_grid[mode] = b->num_sms * std::max(bps, 1);
       b->tail_grid[mode] = b->num_sms * std::max(tbps, 1);

@@ -66,6 +66,8 @@ struct Geo {
   __device__ __forceinline__ int cand(int k) const { return ldi(lay.cand, k); }
   __device__ __forceinline__ float4 start(int i) const { return ld(lay.start + i); }
   __device__ __forceinline__ int bvh_root(int g) const { return ldi(lay.bvh_root, g); }
+  __device__ __forceinline__ int plane_begin(int g) const { return ldi(lay.plane_begin, g); }
+  __device__ __forceinline__ float4 plane(int i) const { return ld(lay.plane + i); }
   __device__ __forceinline__ float4 node(int i) const {
     if (!SMEM && i < nstage) return sblob[i];  /* a top level, staged */
     return ld(lay.bvh_node + i);
@@ -103,7 +105,7 @@ constexpr int kBvhStack = 32;
    square roots are the hardware approximation: its relative error (< 2^-22
    of a distance below the box diagonal) is far inside the 4 eps the callers
    take off, so the bound stays a bound. */
-template <bool EXT, class G_t>
+template <int EXT, class G_t>
 __device__ __forceinline__ float surface_lb(const G_t& G, int s, float px, float py, float pz) {
   const float4 A = G.hotA(s);
   const int4 B = G.hotB(s);
@@ -143,7 +145,7 @@ __device__ __forceinline__ float box_dist(float4 lo, float4 hi, float px, float 
    they cannot change either; a surface's bound is the larger of the
    distance to its leaf's box and its own plane / quadric bound).  Out of
    line, like scan_bvh. */
-template <bool EXT, class G_t>
+template <int EXT, class G_t>
 __device__ __noinline__ float safety_bvh(const G_t& G, int root, float px, float py, float pz,
                                          float d, float& d2, int& near) {
   int stk[kBvhStack];
@@ -203,7 +205,7 @@ __device__ __noinline__ float safety_bvh(const G_t& G, int root, float px, float
    receives the bound over the candidate surfaces alone (the grain ball: a
    flight inside it needs the box-face test only); for a BVH grain it is
    searched no farther than the full bound, so it costs no extra nodes. */
-template <bool EXT, class G_t>
+template <int EXT, class G_t>
 __device__ __forceinline__ float safety(const G_t& G, int grain, float px, float py, float pz,
                                         float X, float Y, float Z, float eps, float cap,
                                         float& dgrain, float& dgrain2, int& near) {
@@ -224,12 +226,43 @@ __device__ __forceinline__ float safety(const G_t& G, int grain, float px, float
         dc = nearer ? d : dc;
       }
     } else {
-      dc = safety_bvh<EXT>(G, root, px, py, pz, fminf(dbox, cap), dc2, near);
+      const int kb = EXT == 2 ? G.plane_begin(grain) : 0;
+      const int ke = EXT == 2 ? G.plane_begin(grain + 1) : 0;
+      if (ke > kb) {
+        for (int k = kb; k < ke; ++k) {
+          const float4 A = G.plane(k);
+          dc = fminf(dc, fabsf(fmaf(A.x, px, fmaf(A.y, py, A.z * pz)) - A.w));
+        }
+        dc2 = dc;
+      } else {
+        dc = safety_bvh<EXT>(G, root, px, py, pz, fminf(dbox, cap), dc2, near);
+      }
     }
   }
   dgrain = dc - 4.0f * eps;
   dgrain2 = dc2 - 4.0f * eps;
   return fminf(dbox, dc) - 4.0f * eps;
+}
+
+/* Whether a flight of length fp from p along d ends behind every facet plane
+   of a BVH grain that has them: a polygon is met only from behind (along its
+   outward normal), so none is met up to fp.  The margin covers the polygons'
+   distance from their plane (eps / 4), the tests' eps and the rounding of the
+   direction times fp.  This and the plane bounds of the balls replace nearly
+   every tree walk in a polyhedral grain: 5 Voronoi grains as 43 000 triangles,
+   2.5e6 phonons: 160 -> 54 ms (drain 60 -> 22, tail 93 -> 27). */
+template <class G_t>
+__device__ __forceinline__ bool behind_planes(const G_t& G, int grain, float px, float py, float pz,
+                                              float dx, float dy, float dz, float fp, float eps) {
+  const int kb = G.plane_begin(grain), ke = G.plane_begin(grain + 1);
+  const float m = -fmaf(5.0e-7f, fp, 4.0f * eps);
+  bool behind = ke > kb;
+  for (int k = kb; k < ke; ++k) {
+    const float4 A = G.plane(k);
+    const float s = fmaf(A.x, px, fmaf(A.y, py, A.z * pz)) - A.w;
+    behind = behind && fmaf(fp, fmaf(A.x, dx, fmaf(A.y, dy, A.z * dz)), s) < m;
+  }
+  return behind;
 }
 
 /* Buckets of the tail order: a quarter octave of the expected walk each. */

@@ -96,6 +96,9 @@ struct BlobLayout {
   int cand;         /* int[ncand]                                                    */
   int start;        /* voronoi: float4 (generatrix, grain); bricks: int2 (surf, grain) */
   int bvh_root;     /* int[ngrain_total]: root node of the grain's BVH, -1 linear scan */
+  int plane_begin;  /* int[ngrain_total+1]: a BVH grain's distinct planes (facet_planes) */
+  int plane;        /* float4: outward unit normal, offset                            */
+  int nplane;       /* planes in the blob (0: no grain has them)                      */
   int bvh_node;     /* float4[2*nnode]: (lo, a) (hi, b), see bvh.cpp                  */
   int nbvh;         /* BVH nodes in the blob (0: every grain scans linearly)          */
   int ncap;         /* capped-cylinder records in the blob                            */
@@ -115,7 +118,8 @@ struct GeoF32 {
   int node_stage;      /* else: float4 units of the BVH node region (its  */
                        /*    top levels, breadth first) copied instead    */
   int has_ext;         /* 1: a BVH or capped cylinders (kernels built for  */
-                       /*    them; the others leave both out)             */
+                       /*    them; the others leave both out), 2: a grain  */
+                       /*    with facet planes as well                    */
 };
 
 /* One geometry of a batched launch (device table, read through the cache). */
@@ -265,13 +269,13 @@ cudaError_t launch_tail64(const Geo64& g, const GeoF32& g32, const Run64& r, int
 cudaError_t launch_tail_fp32(const GeoF32& g, const RunF32& r, int grid, int block, size_t smem,
                              cudaStream_t st, int mode = MODE_FORWARD);
 cudaError_t tail_occupancy(int block, size_t smem, int* blocks_per_sm, int mode = MODE_FORWARD,
-                           bool bvh = false, bool whole = true);
+                           int ext = 0, bool whole = true);
 /* Batched launch over several geometries (geometry in global memory):
    forward, list (ids of transmitted samples as (global task << 32) |
    particle) or adjoint replay of such a list. */
 cudaError_t launch_persistent_batch(const RunF32& r, int grid, int block, cudaStream_t st,
-                                    bool bvh, int mode, bool tail);
-cudaError_t persistent_batch_occupancy(int block, int* blocks_per_sm, bool bvh, int mode, bool tail);
+                                    int ext, int mode, bool tail);
+cudaError_t persistent_batch_occupancy(int block, int* blocks_per_sm, int ext, int mode, bool tail);
 /* float4 per phonon in the tail list: the state of a phonon handed from the
    drain phase to the tail phase (position, direction, free path, MFP, the
    ball centre and radii, grain, last surface, task, omega, sample id,
@@ -301,7 +305,7 @@ cudaError_t launch_expand_chunks(const int* order, int norder, int per_task, int
 cudaError_t check_report(long long* count, int* code, int* index, bool reset);
 /* Residency of the persistent kernel for a block size and shared memory. */
 cudaError_t persistent_occupancy(int block, size_t smem, int* blocks_per_sm,
-                                 int mode = MODE_FORWARD, bool bvh = false, bool whole = true);
+                                 int mode = MODE_FORWARD, int ext = 0, bool whole = true);
 
 /* ---------------- FP64 kappa reduction ---------------------------------- */
 

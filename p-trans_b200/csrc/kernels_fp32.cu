@@ -106,6 +106,8 @@ struct GeoBatch {
   __device__ __forceinline__ int cand(int k) const { return ldi(lay.cand, k); }
   __device__ __forceinline__ float4 start(int i) const { return ld(lay.start + i); }
   __device__ __forceinline__ int bvh_root(int g) const { return ldi(lay.bvh_root, g); }
+  __device__ __forceinline__ int plane_begin(int g) const { return ldi(lay.plane_begin, g); }
+  __device__ __forceinline__ float4 plane(int i) const { return ld(lay.plane + i); }
   __device__ __forceinline__ float4 node(int i) const { return ld(lay.bvh_node + i); }
 };
 
@@ -251,7 +253,7 @@ __device__ __forceinline__ void capped_normal(float4 A, float4 E, float px, floa
 
 /* One candidate surface against the ray p + t d: updates the nearest raw
    distance tr and surface sb. */
-template <bool EXT, class G_t>
+template <int EXT, class G_t>
 __device__ __forceinline__ void test_surface(const G_t& G, int s, float px, float py, float pz,
                                              float dx, float dy, float dz, int last_geom,
                                              float eps, float zmax, float& tr, int& sb) {
@@ -301,7 +303,7 @@ __device__ __forceinline__ void test_surface(const G_t& G, int s, float px, floa
    there ends it; with none, a p-p event ends it), so the decision, and the
    trajectory, are those of the full search.  Kept out of line so the linear
    scan that every small grain uses stays compact in the instruction cache. */
-template <bool EXT, class G_t>
+template <int EXT, class G_t>
 __device__ __noinline__ void scan_bvh(const G_t& G, int root, float px, float py, float pz,
                                       float dx, float dy, float dz, int last_geom, float eps,
                                       float zmax, float tcut, float& tr, int& sb, unsigned& nbox,
@@ -361,7 +363,7 @@ __device__ __noinline__ void scan_bvh(const G_t& G, int root, float px, float py
    (the box-grain exit, >= 0) and sb are updated; tb stays >= 0.  fp is the
    flight's free path: a BVH search skips what lies beyond it (a hit farther
    away cannot end the flight). */
-template <bool EXT, class G_t>
+template <int EXT, class G_t>
 __device__ __forceinline__ void scan_grain(const G_t& G, int grain, float px, float py, float pz,
                                            float dx, float dy, float dz, int last_geom, float eps,
                                            float zmax, float fp, float& tb, int& sb, unsigned& nbox,
@@ -373,7 +375,7 @@ __device__ __forceinline__ void scan_grain(const G_t& G, int grain, float px, fl
     nsurf += (unsigned)(ke - kb);
     for (int k = kb; k < ke; ++k)
       test_surface<EXT>(G, G.cand(k), px, py, pz, dx, dy, dz, last_geom, eps, zmax, tr, sb);
-  } else {
+  } else if (EXT != 2 || !behind_planes(G, grain, px, py, pz, dx, dy, dz, fp, eps)) {
     scan_bvh<EXT>(G, root, px, py, pz, dx, dy, dz, last_geom, eps, zmax, fp, tr, sb, nbox, nsurf);
   }
   tb = fmaxf(tr, 0.0f);
@@ -402,7 +404,7 @@ __device__ __forceinline__ void slab_exit(float px, float py, float pz, float dx
 
 /* One candidate surface, where the second ball has shown it to be the only
    one a flight can reach: scan_grain's result for that flight. */
-template <bool EXT, class G_t>
+template <int EXT, class G_t>
 __device__ __forceinline__ void test_near(const G_t& G, int s, float px, float py, float pz,
                                           float dx, float dy, float dz, int last_geom, float eps,
                                           float zmax, float& tb, int& sb, unsigned& nsurf) {
@@ -446,7 +448,7 @@ __device__ __forceinline__ void warp_argmax(float v, int lane, float& vmax, int&
    led (three per entry); kind is 2 when every entry is a triangle, 1 when
    every entry is a polygon, else 0.  Warp-collective: every lane searches
    the same nodes. */
-template <bool EXT, class G_t>
+template <int EXT, class G_t>
 __device__ __noinline__ float list_bvh(const G_t& G, int root, float px, float py, float pz,
                                        float R, int lane, int* lst, float4* lpl, float4* led,
                                        int& n, int& kind) {
@@ -529,7 +531,7 @@ __device__ __noinline__ float list_bvh(const G_t& G, int root, float px, float p
 /* safety() for a point p within the radius lc.w of a local list's centre
    lc.xyz: the listed surfaces' bounds (lane k takes entry k) and
    lc.w - |p - c| for every other surface of the grain.  Warp-collective. */
-template <bool EXT, class G_t>
+template <int EXT, class G_t>
 __device__ __forceinline__ float safety_list(const G_t& G, const int* lst, int n, float4 lc,
                                              float px, float py, float pz, float X, float Y,
                                              float Z, float eps, int lane, float& dgrain,
@@ -564,7 +566,7 @@ __device__ __forceinline__ float safety_list(const G_t& G, const int* lst, int n
    path cannot end the flight, so the search stops at the float above fp:
    the nearest hit up to fp is the full scan's, and without one tb stays
    above fp, as it would. */
-template <bool EXT, class G_t>
+template <int EXT, class G_t>
 __device__ __forceinline__ void scan_list(const G_t& G, const int* lst, const float4* lpl,
                                           const float4* led, int n, int kind, float px, float py,
                                           float pz, float dx, float dy, float dz, int last_geom,
@@ -628,7 +630,7 @@ struct AdjAcc {
    the flight's Philox uniforms.  The one-lane path and the tail phase's
    rounds both take their events here, so a trajectory does not depend on
    which of them met the surface. */
-template <int MODE, bool EXT, class G_t>
+template <int MODE, int EXT, class G_t>
 __device__ __forceinline__ int surface_hit(const G_t& G, float tb, int sb, float u0, float u1,
                                            float u2, float u3, float Y, float Z, int pmask,
                                            int nmat, float omr, float lam, uint32_t flight,
@@ -927,7 +929,7 @@ constexpr float kBallCapMfp = 32.0f;
    bytes and still gains, C4 3833 -> 3677 ms, C3 735 -> 724 ms), two for the
    rest (the tail phase's rounds, and the batched and adjoint kernels, which
    would spill more). */
-template <bool SMEM, int MODE, bool BATCH, bool EXT, int PH>
+template <bool SMEM, int MODE, bool BATCH, int EXT, int PH>
 __global__ void __launch_bounds__(kBlock,
                                   (PH == PH_DRAIN && !BATCH && MODE != MODE_ADJOINT) ? 3 : 2)
     k_persistent(GeoF32 gp, RunF32 r) {
@@ -1001,7 +1003,6 @@ __global__ void __launch_bounds__(kBlock,
   int ch_task = -1, ch_next = 0, ch_left = 0;
   bool queue_done = false;
   bool tail_full = false;  /* the tail list refused this warp: stop asking */
-  int grace = r.grace_steps;  /* passes its long-MFP phonons get before a hand-over */
 
   /* lane state */
   bool alive = false;
@@ -1096,6 +1097,7 @@ __global__ void __launch_bounds__(kBlock,
           } else {
             if (c >= r.nchunk) {
               queue_done = true;
+              ch_left = r.grace_steps;  /* from here on: passes before a hand-over */
               if (lane == 0) atomicMin(r.stats + 6, globaltimer());
               break;
             }
@@ -1221,8 +1223,8 @@ __global__ void __launch_bounds__(kBlock,
     if (PH == PH_DRAIN && MODE != MODE_TRACE && queue_done && r.coop_lanes > 0 &&
         !tail_full && __popc(__ballot_sync(FULL, alive)) <= r.coop_lanes) {
       const unsigned mw =
-          __ballot_sync(FULL, alive && (lam < flmax || r.fast_steps <= 0 || grace == 0));
-      grace -= grace > 0 ? 1 : 0;
+          __ballot_sync(FULL, alive && (lam < flmax || r.fast_steps <= 0 || ch_left == 0));
+      ch_left -= ch_left > 0 ? 1 : 0;
       if (mw) {
         /* a slot is reserved from one counter of all requests (queue[5])
            before the phonon picks its end of the list: the phonons admitted
@@ -1448,8 +1450,14 @@ __global__ void __launch_bounds__(kBlock,
             /* in kernels built for BVH grains a round tests at most
                kTestWindow flights from its first one that needs the whole
                grain's search */
-            const unsigned needm = __ballot_sync(FULL, !in_ball && !in_gball && !in_g2 && !in_list);
-            const int jw = (EXT && needm) ? min(32, __ffs(needm) - 1 + kTestWindow) : 32;
+            /* (a grain with facet planes: one flight, the first that reaches
+               a plane, which is nearly always a hit) */
+            const bool planes = EXT == 2 && cgrain > 0 &&
+                                G.plane_begin(cgrain + 1) > G.plane_begin(cgrain);
+            bool walk = !in_ball && !in_gball && !in_g2 && !in_list;
+            if (planes && walk) walk = !behind_planes(G, cgrain, qx, qy, qz, sdx, sdy, sdz, sfp, eps);
+            const unsigned needm = __ballot_sync(FULL, walk);
+            const int jw = (EXT && needm) ? min(32, __ffs(needm) - 1 + (planes ? 1 : kTestWindow)) : 32;
             float tb = 3.0e38f;
             int sb = -1;
             if (!in_ball && lane < jw) {
@@ -1461,7 +1469,7 @@ __global__ void __launch_bounds__(kBlock,
                 else if (kUseList && in_list)
                   scan_list<EXT>(G, lst, lpl, led, ln, lkind, qx, qy, qz, sdx, sdy, sdz,
                                  lane == 0 ? clast : -1, eps, Z, sfp, tb, sb, my_surf_tests);
-                else
+                else if (walk)
                   scan_grain<EXT>(G, cgrain, qx, qy, qz, sdx, sdy, sdz, lane == 0 ? clast : -1, eps,
                                   Z, sfp, tb, sb, my_box_tests, my_surf_tests);
               }
@@ -1538,7 +1546,7 @@ __global__ void __launch_bounds__(kBlock,
                time the walk leaves it (the old safe ball stays valid) */
             if (!__shfl_sync(FULL, in_gball, j - 1) && r.fast_steps > 0) {
               float dg, dg2, d;
-              if (kUseList && cgrain > 0 && G.bvh_root(cgrain) >= 0) {
+              if (kUseList && cgrain > 0 && !planes && G.bvh_root(cgrain) >= 0) {
                 /* from the local list, built anew (one tree search) in
                    another grain or where the list's edge bounds the ball */
                 const int4 lm = coop_lmeta[threadIdx.x >> 5];
@@ -1879,13 +1887,13 @@ __global__ void __launch_bounds__(kBlock,
 /* Static shared memory (the adjoint accumulators, the cooperative rows) plus
    the staged blob can pass the 48 KB a launch gets without opting in, so
    every launch with a staged blob opts in to its dynamic size. */
-template <int MODE, bool EXT, int PH, bool SMEM = true>
+template <int MODE, int EXT, int PH, bool SMEM = true>
 cudaError_t allow_dynamic_smem(size_t smem) {
   return cudaFuncSetAttribute(k_persistent<SMEM, MODE, false, EXT, PH>,
                               cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
 }
 
-template <int MODE, bool EXT, int PH>
+template <int MODE, int EXT, int PH>
 cudaError_t occupancy_mode(int block, size_t smem, int* bps, bool whole) {
   if (smem > 0 && whole) {
     cudaError_t e = allow_dynamic_smem<MODE, EXT, PH>(smem);
@@ -1901,7 +1909,7 @@ cudaError_t occupancy_mode(int block, size_t smem, int* bps, bool whole) {
       bps, k_persistent<false, MODE, false, EXT, PH>, block, smem);
 }
 
-template <int MODE, bool EXT, int PH>
+template <int MODE, int EXT, int PH>
 cudaError_t launch_mode(const GeoF32& g, const RunF32& r, int grid, int block, size_t smem,
                         cudaStream_t st) {
   if (g.stage_smem && smem > 0) {
@@ -1921,54 +1929,57 @@ cudaError_t launch_mode(const GeoF32& g, const RunF32& r, int grid, int block, s
 }
 
 template <int MODE, int PH>
-cudaError_t batch_occupancy_mode(int block, int* bps, bool bvh) {
+cudaError_t batch_occupancy_mode(int block, int* bps, int ext) {
   return cudaOccupancyMaxActiveBlocksPerMultiprocessor(
       bps,
-      bvh ? k_persistent<false, MODE, true, true, PH> : k_persistent<false, MODE, true, false, PH>,
+      ext == 2   ? k_persistent<false, MODE, true, 2, PH>
+      : ext == 1 ? k_persistent<false, MODE, true, 1, PH>
+                 : k_persistent<false, MODE, true, 0, PH>,
       block, 0);
 }
 
 template <int PH>
-cudaError_t batch_occupancy_phase(int block, int* bps, bool bvh, int mode) {
-  if (mode == MODE_LIST) return batch_occupancy_mode<MODE_LIST, PH>(block, bps, bvh);
-  if (mode == MODE_ADJOINT) return batch_occupancy_mode<MODE_ADJOINT, PH>(block, bps, bvh);
+cudaError_t batch_occupancy_phase(int block, int* bps, int ext, int mode) {
+  if (mode == MODE_LIST) return batch_occupancy_mode<MODE_LIST, PH>(block, bps, ext);
+  if (mode == MODE_ADJOINT) return batch_occupancy_mode<MODE_ADJOINT, PH>(block, bps, ext);
   if (mode != MODE_FORWARD) return cudaErrorInvalidValue;
-  return batch_occupancy_mode<MODE_FORWARD, PH>(block, bps, bvh);
+  return batch_occupancy_mode<MODE_FORWARD, PH>(block, bps, ext);
 }
 
-cudaError_t persistent_batch_occupancy(int block, int* bps, bool bvh, int mode, bool tail) {
-  return tail ? batch_occupancy_phase<PH_TAIL>(block, bps, bvh, mode)
-              : batch_occupancy_phase<PH_DRAIN>(block, bps, bvh, mode);
+cudaError_t persistent_batch_occupancy(int block, int* bps, int ext, int mode, bool tail) {
+  return tail ? batch_occupancy_phase<PH_TAIL>(block, bps, ext, mode)
+              : batch_occupancy_phase<PH_DRAIN>(block, bps, ext, mode);
 }
 
 template <int MODE, int PH>
-cudaError_t launch_batch_mode(const RunF32& r, int grid, int block, cudaStream_t st, bool bvh) {
+cudaError_t launch_batch_mode(const RunF32& r, int grid, int block, cudaStream_t st, int ext) {
   GeoF32 g;
   memset(&g, 0, sizeof(g));
-  if (bvh) k_persistent<false, MODE, true, true, PH><<<grid, block, 0, st>>>(g, r);
-  else k_persistent<false, MODE, true, false, PH><<<grid, block, 0, st>>>(g, r);
+  if (ext == 2) k_persistent<false, MODE, true, 2, PH><<<grid, block, 0, st>>>(g, r);
+  else if (ext == 1) k_persistent<false, MODE, true, 1, PH><<<grid, block, 0, st>>>(g, r);
+  else k_persistent<false, MODE, true, 0, PH><<<grid, block, 0, st>>>(g, r);
   return cudaGetLastError();
 }
 
 template <int PH>
-cudaError_t launch_batch_phase(const RunF32& r, int grid, int block, cudaStream_t st, bool bvh,
+cudaError_t launch_batch_phase(const RunF32& r, int grid, int block, cudaStream_t st, int ext,
                                int mode) {
   if (block != kBlock) return cudaErrorInvalidConfiguration;
-  if (mode == MODE_LIST) return launch_batch_mode<MODE_LIST, PH>(r, grid, block, st, bvh);
-  if (mode == MODE_ADJOINT) return launch_batch_mode<MODE_ADJOINT, PH>(r, grid, block, st, bvh);
+  if (mode == MODE_LIST) return launch_batch_mode<MODE_LIST, PH>(r, grid, block, st, ext);
+  if (mode == MODE_ADJOINT) return launch_batch_mode<MODE_ADJOINT, PH>(r, grid, block, st, ext);
   if (mode != MODE_FORWARD) return cudaErrorInvalidValue;
-  return launch_batch_mode<MODE_FORWARD, PH>(r, grid, block, st, bvh);
+  return launch_batch_mode<MODE_FORWARD, PH>(r, grid, block, st, ext);
 }
 
-cudaError_t launch_persistent_batch(const RunF32& r, int grid, int block, cudaStream_t st, bool bvh,
+cudaError_t launch_persistent_batch(const RunF32& r, int grid, int block, cudaStream_t st, int ext,
                                     int mode, bool tail) {
-  return tail ? launch_batch_phase<PH_TAIL>(r, grid, block, st, bvh, mode)
-              : launch_batch_phase<PH_DRAIN>(r, grid, block, st, bvh, mode);
+  return tail ? launch_batch_phase<PH_TAIL>(r, grid, block, st, ext, mode)
+              : launch_batch_phase<PH_DRAIN>(r, grid, block, st, ext, mode);
 }
 
 /* The tail phase exists for the modes with cooperative rounds (forward,
    list, adjoint replay); a trace replay runs every flight on one lane. */
-template <bool EXT, int PH>
+template <int EXT, int PH>
 cudaError_t occupancy_bvh(int block, size_t smem, int* bps, int mode, bool whole) {
   if (mode == MODE_LIST) return occupancy_mode<MODE_LIST, EXT, PH>(block, smem, bps, whole);
   if (mode == MODE_ADJOINT) return occupancy_mode<MODE_ADJOINT, EXT, PH>(block, smem, bps, whole);
@@ -1979,17 +1990,19 @@ cudaError_t occupancy_bvh(int block, size_t smem, int* bps, int mode, bool whole
   return occupancy_mode<MODE_FORWARD, EXT, PH>(block, smem, bps, whole);
 }
 
-cudaError_t persistent_occupancy(int block, size_t smem, int* bps, int mode, bool bvh, bool whole) {
-  return bvh ? occupancy_bvh<true, PH_DRAIN>(block, smem, bps, mode, whole)
-             : occupancy_bvh<false, PH_DRAIN>(block, smem, bps, mode, whole);
+cudaError_t persistent_occupancy(int block, size_t smem, int* bps, int mode, int ext, bool whole) {
+  return ext == 2   ? occupancy_bvh<2, PH_DRAIN>(block, smem, bps, mode, whole)
+         : ext == 1 ? occupancy_bvh<1, PH_DRAIN>(block, smem, bps, mode, whole)
+                    : occupancy_bvh<0, PH_DRAIN>(block, smem, bps, mode, whole);
 }
 
-cudaError_t tail_occupancy(int block, size_t smem, int* bps, int mode, bool bvh, bool whole) {
-  return bvh ? occupancy_bvh<true, PH_TAIL>(block, smem, bps, mode, whole)
-             : occupancy_bvh<false, PH_TAIL>(block, smem, bps, mode, whole);
+cudaError_t tail_occupancy(int block, size_t smem, int* bps, int mode, int ext, bool whole) {
+  return ext == 2   ? occupancy_bvh<2, PH_TAIL>(block, smem, bps, mode, whole)
+         : ext == 1 ? occupancy_bvh<1, PH_TAIL>(block, smem, bps, mode, whole)
+                    : occupancy_bvh<0, PH_TAIL>(block, smem, bps, mode, whole);
 }
 
-template <bool EXT, int PH>
+template <int EXT, int PH>
 cudaError_t launch_bvh(const GeoF32& g, const RunF32& r, int grid, int block, size_t smem,
                        cudaStream_t st, int mode) {
   if (mode == MODE_LIST) return launch_mode<MODE_LIST, EXT, PH>(g, r, grid, block, smem, st);
@@ -2004,8 +2017,9 @@ cudaError_t launch_bvh(const GeoF32& g, const RunF32& r, int grid, int block, si
 cudaError_t launch_persistent_fp32(const GeoF32& g, const RunF32& r, int grid, int block,
                                    size_t smem, cudaStream_t st, int mode) {
   if (block > kBlock || block % 32) return cudaErrorInvalidConfiguration;
-  return g.has_ext ? launch_bvh<true, PH_DRAIN>(g, r, grid, block, smem, st, mode)
-                   : launch_bvh<false, PH_DRAIN>(g, r, grid, block, smem, st, mode);
+  return g.has_ext == 2   ? launch_bvh<2, PH_DRAIN>(g, r, grid, block, smem, st, mode)
+         : g.has_ext == 1 ? launch_bvh<1, PH_DRAIN>(g, r, grid, block, smem, st, mode)
+                          : launch_bvh<0, PH_DRAIN>(g, r, grid, block, smem, st, mode);
 }
 
 cudaError_t launch_tail_fp32(const GeoF32& g, const RunF32& r, int grid, int block, size_t smem,
@@ -2016,8 +2030,9 @@ cudaError_t launch_tail_fp32(const GeoF32& g, const RunF32& r, int grid, int blo
      copy would take that L1 from them */
   GeoF32 gt = g;
   gt.node_stage = 0;
-  return g.has_ext ? launch_bvh<true, PH_TAIL>(gt, r, grid, block, smem, st, mode)
-                   : launch_bvh<false, PH_TAIL>(gt, r, grid, block, smem, st, mode);
+  return g.has_ext == 2   ? launch_bvh<2, PH_TAIL>(gt, r, grid, block, smem, st, mode)
+         : g.has_ext == 1 ? launch_bvh<1, PH_TAIL>(gt, r, grid, block, smem, st, mode)
+                          : launch_bvh<0, PH_TAIL>(gt, r, grid, block, smem, st, mode);
 }
 
 namespace {

@@ -615,7 +615,8 @@ __device__ bool nearest64(const Geo64& g, const Geo<false>& G, float eps, const 
           best = L; *igrain = which; *isurf = k - kb0; hit = true;
         }
       }
-    } else {
+    } else if (!behind_planes(G, which, (float)pos[0], (float)pos[1], (float)pos[2], (float)dir[0],
+                              (float)dir[1], (float)dir[2], (float)fp, eps)) {
       const float px = (float)pos[0], py = (float)pos[1], pz = (float)pos[2];
       const float ix = inv_dir((float)dir[0]), iy = inv_dir((float)dir[1]),
                   iz = inv_dir((float)dir[2]);
@@ -682,7 +683,7 @@ __device__ __forceinline__ void ball64(const Geo<false>& G, const GeoF32& gp, in
   *bx = (float)pos[0]; *by = (float)pos[1]; *bz = (float)pos[2];
   float dg, dg2;
   int near;
-  const float d = safety<true>(G, which, *bx, *by, *bz, gp.box[0], gp.box[1], gp.box[2], gp.eps,
+  const float d = safety<2>(G, which, *bx, *by, *bz, gp.box[0], gp.box[1], gp.box[2], gp.eps,
                                kBallCap64 * lam, dg, dg2, near) - 1.0e-6f;
   dg -= 1.0e-6f;
   *br2 = d > 0.0f ? d * d : 0.0f;
@@ -984,7 +985,10 @@ __global__ void __launch_bounds__(256, 2) k_tail64(Geo64 g, GeoF32 gp, Run64 r) 
       const bool in_gball = se < gr2 && ss < gr2;
       const bool inbox = in_box64(g, sp);
       const bool brk = !inbox || (int64_t)flight + lane >= r.max_flights;
-      const bool walks = !in_ball && !in_gball && p.which > 0 && G.bvh_root(p.which) >= 0;
+      const bool walks =
+          !in_ball && !in_gball && p.which > 0 && G.bvh_root(p.which) >= 0 &&
+          !behind_planes(G, p.which, (float)sp[0], (float)sp[1], (float)sp[2], (float)sd[0],
+                         (float)sd[1], (float)sd[2], (float)sfp, gp.eps);
       const unsigned wm = __ballot_sync(FULL, walks);
       const int jw = wm ? min(32, __ffs(wm) - 1 + kTestWindow64) : 32;
       double distance = 1.0e10;

@@ -185,7 +185,7 @@ extern "C" int ptg_transmission_noalloc(ptg_handle* h, double mfp_nm, int32_t na
   const int block = (bs >= 32 && bs <= 256 && bs % 32 == 0) ? bs : 256;
   const size_t smem = ptg::dynamic_smem_bytes(v.g32, v.blob_bytes);
   int bps = 0;
-  if (ptg::persistent_occupancy(block, smem, &bps, ptg::MODE_FORWARD, v.g32.has_ext != 0, v.g32.stage_smem != 0) !=
+  if (ptg::persistent_occupancy(block, smem, &bps, ptg::MODE_FORWARD, v.g32.has_ext, v.g32.stage_smem != 0) !=
       cudaSuccess)
     return PTG_ERR_CUDA;
   if (v.opt.blocks_per_sm > 0 && v.opt.blocks_per_sm < bps) bps = v.opt.blocks_per_sm;
@@ -202,7 +202,7 @@ extern "C" int ptg_transmission_noalloc(ptg_handle* h, double mfp_nm, int32_t na
     if (cudaMemsetAsync(r.tail_order + r.tail_cap, 0, sizeof(int) * ptg::kTailOrderExtra, s) != cudaSuccess)
       return PTG_ERR_CUDA;
     int tbps = 0;
-    if (ptg::tail_occupancy(block, smem, &tbps, ptg::MODE_FORWARD, v.g32.has_ext != 0, v.g32.stage_smem != 0) != cudaSuccess)
+    if (ptg::tail_occupancy(block, smem, &tbps, ptg::MODE_FORWARD, v.g32.has_ext, v.g32.stage_smem != 0) != cudaSuccess)
       return PTG_ERR_CUDA;
     tgrid = v.num_sms * (tbps < 1 ? 1 : tbps);
     r.grace_steps = ptg::grace_passes(ntask * np_local, (int64_t)tgrid * (block / 32));

@@ -349,6 +349,30 @@ def test_bvh_and_linear_scan_take_the_same_trajectories(name):
         assert cur[1:] == ref[1:], leaf
 
 
+@pytest.mark.parametrize("levels", [1, 3])
+@pytest.mark.parametrize("precision", [A.PREC_FP32, A.PREC_FP64])
+@pytest.mark.parametrize("mfp", [(1e-9, 3e-8), (2e-8, 2e-6), None])
+def test_facet_planes_take_the_linear_scans_trajectories(levels, precision, mfp):
+    """Convex grains given as triangle meshes bound their balls by the planes
+    of their facets and walk the BVH only for flights that end in front of one
+    (kernels built for them); bvh_leaf = -1 scans every triangle.  Counts, lost
+    counts and flights are equal, with the tail phase and without it (FP32;
+    FP64 against its plain kernel), from short to infinite mean free paths."""
+    m = synth.voronoi_box(4, box=(120.0, 90.0, 100.0), seed=11, trans=0.5, spec=0.2, p_wall=0.3, tri_levels=levels)
+    spec = synth.spectrum(6, seed=8, **(dict(mfp_lo=mfp[0], mfp_hi=mfp[1]) if mfp else {}))
+    gb = A.GeomBuf(m)
+    run = A.make_run(kind_mfp=A.MFP_PER_MODE if mfp else A.MFP_MATTHIESSEN, nangle=5, np_=31, seed=5,
+                     precision=precision)
+    got = []
+    for opts in (dict(bvh_leaf=-1, tune_flags=8), dict(), dict(tune_flags=2), dict(bvh_leaf=1)):
+        with A.Handle(gb.view, spec, **opts) as h:
+            k = h.kappa(run, want_counts=True)
+            got.append((k["counts"], k["lost"], h.stats()["flights"]))
+    for g in got[1:]:
+        np.testing.assert_array_equal(g[0], got[0][0])
+        assert g[1:] == got[0][1:]
+
+
 def test_autotune_keeps_results_and_caches(tmp_path):
     """ptg_autotune leaves valid options on the handle, every option it tries
     gives the same counts (trajectories depend only on Philox counters), and

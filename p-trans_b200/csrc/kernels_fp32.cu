@@ -528,6 +528,52 @@ __device__ __noinline__ float list_bvh(const G_t& G, int root, float px, float p
   return R;
 }
 
+/* The smallest of the lanes' bounds e >= 0, the surface s of a lane that holds
+   it and the smallest of the rest (e2: the lane's next). */
+__device__ __forceinline__ void warp_min2(float& e, float& e2, int& s, int lane) {
+  const unsigned b = __float_as_uint(e);
+  const unsigned m = __reduce_min_sync(FULL, b);
+  const int who = __ffs(__ballot_sync(FULL, b == m)) - 1;
+  e2 = __uint_as_float(__reduce_min_sync(FULL, lane == who ? __float_as_uint(e2) : b));
+  e = __uint_as_float(m);
+  s = __shfl_sync(FULL, s, who);
+}
+
+/* safety() for a grain without a tree search (a linear candidate list, or
+   facet planes): the lanes take a surface each.  Warp-collective. */
+template <int EXT, class G_t>
+__device__ __forceinline__ float safety_warp(const G_t& G, int grain, float px, float py, float pz,
+                                             float X, float Y, float Z, float eps, int lane,
+                                             bool planes, float& dgrain, float& dgrain2, int& near) {
+  const float dbox = fminf(fminf(fminf(px, X - px), fminf(py, Y - py)), fminf(pz, Z - pz));
+  float e = 3.0e38f, e2 = 3.0e38f;
+  int s = -1;
+  if (grain > 0) {
+    if (EXT == 2 && planes) {
+      const int kb = G.plane_begin(grain), ke = G.plane_begin(grain + 1);
+      if (kb + lane < ke) {
+        const float4 A = G.plane(kb + lane);
+        e = fabsf(fmaf(A.x, px, fmaf(A.y, py, A.z * pz)) - A.w);
+      }
+    } else {
+      const int kb = G.cand_begin(grain), ke = G.cand_begin(grain + 1);
+      for (int k = kb + lane; k < ke; k += 32) {
+        const int sk = G.cand(k);
+        const float d = fabsf(surface_lb<EXT>(G, sk, px, py, pz));
+        const bool nearer = d < e;
+        e2 = nearer ? e : fminf(e2, d);
+        s = nearer ? sk : s;
+        e = nearer ? d : e;
+      }
+    }
+  }
+  warp_min2(e, e2, s, lane);
+  near = s;
+  dgrain = e - 4.0f * eps;
+  dgrain2 = (s >= 0 ? e2 : e) - 4.0f * eps;
+  return fminf(dbox, e) - 4.0f * eps;
+}
+
 /* safety() for a point p within the radius lc.w of a local list's centre
    lc.xyz: the listed surfaces' bounds (lane k takes entry k) and
    lc.w - |p - c| for every other surface of the grain.  Warp-collective. */
@@ -541,17 +587,9 @@ __device__ __forceinline__ float safety_list(const G_t& G, const int* lst, int n
   int s = -1;
   if (lane < n) {
     s = lst[lane];
-    e = surface_lb<EXT>(G, s, px, py, pz);
+    e = fabsf(surface_lb<EXT>(G, s, px, py, pz));
   }
-  /* the smallest bound, its surface and the second smallest */
-  for (int o = 16; o > 0; o >>= 1) {
-    const float oe = __shfl_xor_sync(FULL, e, o), oe2 = __shfl_xor_sync(FULL, e2, o);
-    const int os = __shfl_xor_sync(FULL, s, o);
-    const bool other = oe < e || (oe == e && os < s);
-    e2 = other ? fminf(e, oe2) : fminf(oe, e2);
-    e = other ? oe : e;
-    s = other ? os : s;
-  }
+  warp_min2(e, e2, s, lane);
   const float wx = px - lc.x, wy = py - lc.y, wz = pz - lc.z;
   const float du = lc.w - sqrt_approx(fmaf(wx, wx, fmaf(wy, wy, wz * wz)));
   near = e < du ? s : -1;
@@ -1581,8 +1619,12 @@ __global__ void __launch_bounds__(kBlock,
                                        cnear);
                 }
               } else {
-                d = safety<EXT>(G, cgrain, cpx, cpy, cpz, X, Y, Z, eps, kBallCapMfp * clam, dg, dg2,
-                                cnear);
+                if (EXT && !planes && cgrain > 0 && G.bvh_root(cgrain) >= 0)
+                  d = safety<EXT>(G, cgrain, cpx, cpy, cpz, X, Y, Z, eps, kBallCapMfp * clam, dg,
+                                  dg2, cnear);
+                else
+                  d = safety_warp<EXT>(G, cgrain, cpx, cpy, cpz, X, Y, Z, eps, lane, planes, dg, dg2,
+                                       cnear);
               }
               cbx = cpx; cby = cpy; cbz = cpz;
               cbr2 = d > 0.0f ? d * d : 0.0f;

@@ -149,7 +149,7 @@ struct RunF32 {
   uint32_t max_flights;
   int32_t ref_quirks;
   int32_t regen_threshold;
-  int32_t fast_steps;         /* max safe-distance p-p flights per iteration (0: off) */
+  int32_t fast_steps;         /* a quarter of the most ball flights per iteration (0: off) */
   float fast_lambda_max;      /* tasks with a smaller MFP use the fast path           */
   int32_t coop_lanes;         /* once the queue is dry, a warp with at most this many
                                  live phonons moves them to the tail list, where

@@ -30,14 +30,14 @@
  *     one the full test gives.  A diffusive walk leaves the ball only after
  *     about (d/MFP)^2 flights, which shortens the serial chain of the longest
  *     trajectories that bound the kernel's run time.  A warp takes fast
- *     flights in groups of four, past fast_steps only while half its live
- *     lanes are still in their balls, so lanes that need a full flight are
- *     not held back.  With the ball the lane keeps a second radius about the
+ *     flights in groups of two or three, after the first only while a third
+ *     of its live lanes are still in their balls and at most 4 fast_steps of
+ *     them, so lanes that need a full flight are not held back.  With the ball the lane keeps a second radius about the
  *     same centre, over the grain's candidate surfaces alone (the grain
  *     ball): a flight inside it needs only the box-face test;
  *   - one Philox4x32-10 block per free flight supplies the four uniforms of
- *     any event; on the fast path the blocks of four flights are computed
- *     together so that four independent chains fill the issue slots; tallies
+ *     any event; on the fast path the blocks of a group's flights are
+ *     computed together so that independent chains fill the issue slots; tallies
  *     are integer, aggregated per warp by task (match_any) before one atomic;
  *   - two phases: the drain phase runs the work queue one lane per phonon
  *     and, once the queue is dry, hands its live phonons to a tail list;
@@ -971,6 +971,17 @@ template <bool SMEM, int MODE, bool BATCH, int EXT, int PH>
 __global__ void __launch_bounds__(kBlock,
                                   (PH == PH_DRAIN && !BATCH && MODE != MODE_ADJOINT) ? 3 : 2)
     k_persistent(GeoF32 gp, RunF32 r) {
+  /* Ball flights drawn together, and the share of its live lanes (a third)
+     that a warp needs to go on with them.  Of the four that a group used to
+     hold, a lane took 1.7 on the porous film (12.6 of its 32 lanes in the
+     group), so it drew more than it used; one alone leaves the pipes waiting.
+     Groups of 4 by halves / 3 by thirds / 2 by thirds / 1 by halves: film
+     16.06 / 15.67 / 15.72 / 16.65 ms, polycrystal 9.08 / 8.81 / 8.91 / 9.84,
+     64 films 22.4 / 21.1 / 21.1 / 21.8; with a BVH or capped cylinders 4 by
+     halves / 2 by thirds / 1 by thirds: 222.6 / 217.5 / 216.9 ms, their
+     adjoint 10.2 / 9.75 / 10.4. */
+  constexpr int kFastGroup = EXT ? 2 : 3;
+  constexpr int kFastShare = 3;
   typename std::conditional<BATCH, GeoBatch, Geo<SMEM>>::type G;
   G.lay = gp.lay;
   G.base = gp.blob;
@@ -1678,49 +1689,46 @@ __global__ void __launch_bounds__(kBlock,
     bool paused = false;  /* stopped by the step limit while still in its ball */
     {
       /* ---- safe-ball p-p flights: the segment to the next p-p point stays
-         inside the safe ball (convex), so no surface is crossed.  Four
+         inside the safe ball (convex), so no surface is crossed.  kFastGroup
          flights at a time: their Philox blocks, new directions and free
          paths do not depend on the phonon state and are computed together;
          only the position / ball test chain is serial.  Every lane takes
-         part in the loop control (the ballots): past fast_steps flights the
-         warp goes on only while at least half of its live lanes are still in
-         their balls, and never past 4 x fast_steps, so a few lanes deep in
-         large balls do not hold the others' full flights back. ---- */
+         part in the loop control (the ballots), so a few lanes deep in large
+         balls do not hold the others' full flights back. ---- */
       bool fast_more = alive && MODE != MODE_TRACE && br2 > 0.0f && !coop;
       const int nalive = __popc(__ballot_sync(FULL, alive));
-      for (int g = 0;; g += 4) {
-        const bool go = fast_more && flight + 4u <= r.max_flights;
-        const unsigned gm = __ballot_sync(FULL, go);
+      for (int g = 0;; g += kFastGroup) {
+        /* does the next flight end inside the ball? */
+        float qx = fmaf(fp, dx, px), qy = fmaf(fp, dy, py), qz = fmaf(fp, dz, pz);
+        {
+          const float ex = qx - bx, ey = qy - by, ez = qz - bz;
+          fast_more = fast_more && fmaf(ex, ex, fmaf(ey, ey, ez * ez)) < br2 &&
+                      flight + (unsigned)kFastGroup <= r.max_flights;
+        }
+        const unsigned gm = __ballot_sync(FULL, fast_more);
         if (!gm) break;
-        if (g >= r.fast_steps && (g >= 4 * r.fast_steps || 2 * __popc(gm) < nalive)) {
-          paused = go;
+        if (g > 0 && (g >= 4 * r.fast_steps || kFastShare * __popc(gm) < nalive)) {
+          paused = fast_more;
           break;
         }
-        if (!go) continue;
-        uint4 B[4];
+        if (!fast_more) continue;
+        uint4 B[kFastGroup];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) B[j] = philox10(flight + 1u + j, c1, slo, shi, key);
-        float nx[4], ny[4], nz[4], nf[4];
+        for (int j = 0; j < kFastGroup; ++j) B[j] = philox10(flight + 1u + j, c1, slo, shi, key);
+        float nx[kFastGroup], ny[kFastGroup], nz[kFastGroup], nf[kFastGroup];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const float ct = fmaf(u23f(B[j].x), 2.0f, -1.0f);
-          const float st = sqrt_approx(fmaxf(0.0f, fmaf(-ct, ct, 1.0f)));
-          float sp, cp;
-          sincos2pi(u23f(B[j].y), &sp, &cp);
-          nx[j] = ct;
-          ny[j] = st * cp;
-          nz[j] = st * sp;
-          nf[j] = -lam * __logf(u23f(B[j].z));
-        }
+        for (int j = 0; j < kFastGroup; ++j) pp_dir(B[j], lam, nx[j], ny[j], nz[j], nf[j]);
         /* the position advances with the same rounding as a full flight's
            p-p event, so the trajectory does not depend on which path took
            a flight */
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
+        for (int j = 0; j < kFastGroup; ++j) {
           /* predicated: no branch per step */
-          const float qx = fmaf(fp, dx, px), qy = fmaf(fp, dy, py), qz = fmaf(fp, dz, pz);
+          if (j > 0) {
+            qx = fmaf(fp, dx, px); qy = fmaf(fp, dy, py); qz = fmaf(fp, dz, pz);
+          }
           const float ex = qx - bx, ey = qy - by, ez = qz - bz;
-          const bool acc = fast_more && (fmaf(ex, ex, fmaf(ey, ey, ez * ez)) < br2);
+          const bool acc = j == 0 || (fast_more && fmaf(ex, ex, fmaf(ey, ey, ez * ez)) < br2);
           if (MODE == MODE_ADJOINT) {
             adj_len += acc ? fp : 0.0f;
             adj_npp += acc ? 1u : 0u;

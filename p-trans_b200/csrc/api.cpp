@@ -99,18 +99,18 @@ struct ptg_handle {
   DevBuf blob;
   ptg::GeoF32 g32;
   size_t blob_bytes = 0;
-  /* work buffers */
-  DevBuf task, chunk, counts, lost, stats, queue, order;
-  /* pinned staging of the FP32 task table and queue order; h2d_done marks
-     the end of their last copy */
-  PinBuf pin_task, pin_order;
-  cudaEvent_t h2d_done = nullptr;
-  bool h2d_pending = false;
+  /* what a call clears and reads back (CallLayout), its tables (tasks, then
+     the queue order) and their pinned staging.  The staging is free again once
+     the stream has been waited for; busy: it has not since the last use */
+  DevBuf call, in;
+  PinBuf pin_in, pin_out, pin_const;
+  bool busy = false;
+  /* launch shape of the last mode and block size (0: none yet) */
+  int occ_key = 0, occ_bps = 0, occ_tail = 0;
   /* FP32 tail phase: phonons the drain phase hands over */
   DevBuf tail;
-  /* reduction */
-  DevBuf red_coef, red_K, red_W, red_mfp, red_bin, red_grid, red_tc, red_kv, red_bw, red_bv,
-      red_emfp, red_trans, red_result;
+  /* reduction: constants, scratch, results (result, then EMFPs), transmissions */
+  DevBuf red_in, red_tmp, red_out, red_trans;
   /* adjoint: list of transmitted samples, per-sample weights, accumulators */
   DevBuf adj_list, adj_w, adj_acc;
   /* trace replay: position offsets, counts, exit sides, positions */
@@ -120,16 +120,14 @@ struct ptg_handle {
   int tail_cap = 0;          /* its tail-list capacity (0: no tail phase)       */
   ~ptg_handle() {
     for (DevBuf* b : owned) { b->release(); delete b; }
-    DevBuf* all[] = {&blob, &task, &chunk, &counts, &lost, &stats, &queue, &red_coef, &red_K,
-                     &red_W, &red_mfp, &red_bin, &red_grid, &red_tc, &red_kv, &red_bw, &red_bv,
-                     &red_emfp, &red_trans, &red_result, &adj_list, &adj_w, &adj_acc,
-                     &tr_off, &tr_npos, &tr_end, &tr_pos, &tail, &order};
+    DevBuf* all[] = {&blob, &call, &in, &red_in, &red_tmp, &red_out, &red_trans, &adj_list, &adj_w,
+                     &adj_acc, &tr_off, &tr_npos, &tr_end, &tr_pos, &tail};
     for (DevBuf* b : all) b->release();
     if (stream) cudaStreamSynchronize(stream);
-    pin_task.release();
-    pin_order.release();
+    pin_in.release();
+    pin_out.release();
+    pin_const.release();
     for (cudaEvent_t e : ev) if (e) cudaEventDestroy(e);
-    if (h2d_done) cudaEventDestroy(h2d_done);
     if (stream) cudaStreamDestroy(stream);
   }
 };
@@ -478,6 +476,7 @@ int build_blob(ptg_handle* h) {
   int st = ptg::blob_from_geometry(G, h->opt.bvh_leaf, &blob, &L, &why);
   if (st != PTG_OK) { h->last_error = why; return st; }
   h->blob_bytes = blob.size() * 16;
+  h->occ_key = 0;
   CU(h->blob.ensure(h->blob_bytes));
   CU(cudaMemcpy(h->blob.p, blob.data(), h->blob_bytes, cudaMemcpyHostToDevice));
   ptg::GeoF32& g32 = h->g32;
@@ -591,6 +590,24 @@ struct Transport {
   int* trace_end = nullptr;
 };
 
+/* ptg_handle::call: statistics, queue and the tail order's buckets, then the
+   transmitted and lost counts of the tasks: one clear before a run, one copy
+   of the front (and the counts) after it. */
+struct CallLayout {
+  static constexpr size_t kQueue = sizeof(unsigned long long) * ptg::kStatSlots;
+  static constexpr size_t kHist = kQueue + sizeof(int) * 16;
+  static constexpr size_t kCounts = kHist + sizeof(int) * ptg::kTailOrderExtra;
+  static size_t lost(int64_t ntask) { return kCounts + sizeof(unsigned long long) * ntask; }
+  static size_t total(int64_t ntask) { return kCounts + 2 * sizeof(unsigned long long) * ntask; }
+};
+
+/* Waits for the pinned staging of a call that ended early. */
+int staging_free(ptg_handle* h) {
+  if (h->busy) CU(cudaStreamSynchronize(h->stream));
+  h->busy = false;
+  return PTG_OK;
+}
+
 int run_transport(ptg_handle* h, const Transport& T) {
   ptg::NvtxRange nvtx(T.mode == ptg::MODE_LIST      ? "ptg transport: list"
                       : T.mode == ptg::MODE_ADJOINT ? "ptg transport: adjoint replay"
@@ -598,47 +615,41 @@ int run_transport(ptg_handle* h, const Transport& T) {
                                                     : "ptg transport");
   const int64_t ntask = T.ntask;
   CU(cudaSetDevice(h->device));
-  CU(h->counts.ensure(sizeof(unsigned long long) * ntask));
-  CU(h->lost.ensure(sizeof(unsigned long long) * ntask));
-  CU(h->stats.ensure(sizeof(unsigned long long) * ptg::kStatSlots));
-  CU(h->queue.ensure(sizeof(int) * 8));
-  CU(cudaMemsetAsync(h->counts.p, 0, sizeof(unsigned long long) * ntask, h->stream));
-  CU(cudaMemsetAsync(h->lost.p, 0, sizeof(unsigned long long) * ntask, h->stream));
-  CU(cudaMemsetAsync(h->stats.p, 0, sizeof(unsigned long long) * ptg::kStatSlots, h->stream));
-  /* stats[5], stats[6] collect minima of the global timer */
-  CU(cudaMemsetAsync(h->stats.as<unsigned long long>() + 5, 0xFF, sizeof(unsigned long long) * 2,
-                     h->stream));
-  CU(cudaMemsetAsync(h->queue.p, 0, sizeof(int) * 8, h->stream));
+  CU(h->call.ensure(CallLayout::total(ntask)));
+  CU(cudaMemsetAsync(h->call.p, 0, CallLayout::total(ntask), h->stream));
+  char* const call = h->call.as<char>();
+  unsigned long long* const d_stats = reinterpret_cast<unsigned long long*>(call);
+  int* const d_queue = reinterpret_cast<int*>(call + CallLayout::kQueue);
+  int* const d_hist = reinterpret_cast<int*>(call + CallLayout::kHist);
+  unsigned long long* const d_counts = reinterpret_cast<unsigned long long*>(call + CallLayout::kCounts);
+  unsigned long long* const d_lost = d_counts + ntask;
   const int64_t maxf = h->opt.max_flights > 0 ? h->opt.max_flights : 10000000LL;
   memset(&h->last, 0, sizeof(h->last));
   const bool fp64 = T.precision == PTG_PREC_FP64;
   const bool plain = fp64 && (h->opt.tune_flags & 8);
   /* the task table and the queue order (longest expected trajectories first:
      ascending MFP) are written to pinned staging and copied without a host
-     wait; the chunk table (task, first local particle, count) is expanded
-     from the order on the device.  The MFP depends on (mode, grid point)
-     only, so those pairs are sorted and every angle's task follows its pair;
-     equal MFPs keep index order. */
-  if (h->h2d_pending) {
-    CU(cudaEventSynchronize(h->h2d_done));
-    h->h2d_pending = false;
-  }
+     wait.  The MFP depends on (mode, grid point) only, so those pairs are
+     sorted and every angle's task follows its pair; equal MFPs keep index
+     order. */
+  int rc = staging_free(h);
+  if (rc != PTG_OK) return rc;
   const size_t task_bytes = (fp64 ? sizeof(ptg::Task64) : sizeof(float4)) * (size_t)ntask;
-  CU(h->pin_task.ensure(task_bytes > 0 ? task_bytes : 1));
-  CU(h->pin_order.ensure(sizeof(int) * (ntask > 0 ? ntask : 1)));
-  int* order = h->pin_order.as<int>();
+  CU(h->pin_in.ensure(task_bytes + sizeof(int) * (size_t)(ntask > 0 ? ntask : 1)));
+  ptg::Task64* const t64 = h->pin_in.as<ptg::Task64>();
+  float4* const t32 = h->pin_in.as<float4>();
+  int* order = reinterpret_cast<int*>(h->pin_in.as<char>() + task_bytes);
   const int64_t npair = T.npair > 0 ? std::min<int64_t>(ntask, T.npair) : ntask;
   std::vector<int64_t> pairs;
   pairs.reserve(npair);
   for (int64_t i = 0; i < ntask; ++i) {
     const ptg::TaskHost& th = (*T.tasks)[i];
     if (fp64) {
-      h->pin_task.as<ptg::Task64>()[i] = {th.lambda, th.cth, th.sth, th.omega};
+      t64[i] = {th.lambda, th.cth, th.sth, th.omega};
     } else {
       float lam = th.lambda == 1.0e10 ? INFINITY : (float)th.lambda;
       if (!(th.lambda > 0.0)) lam = 0.0f;
-      h->pin_task.as<float4>()[i] = make_float4(lam, (float)th.cth, (float)th.sth,
-                                                (float)(th.omega / h->spec.max_omega));
+      t32[i] = make_float4(lam, (float)th.cth, (float)th.sth, (float)(th.omega / h->spec.max_omega));
     }
     if (i < npair && th.lambda > 0.0) pairs.push_back(i);
   }
@@ -661,21 +672,20 @@ int run_transport(ptg_handle* h, const Transport& T) {
   }
   const int64_t nchunk = plain ? 0 : norder * per_task;
   if (nchunk > 2147483647LL) { h->last_error = "too many chunks"; return PTG_ERR_INVALID; }
-  CU(h->task.ensure(task_bytes));
-  CU(h->order.ensure(sizeof(int) * (norder > 0 ? norder : 1)));
-  CU(h->chunk.ensure(sizeof(int4) * (nchunk + 1)));
-  CU(cudaMemcpyAsync(h->task.p, h->pin_task.p, task_bytes, cudaMemcpyHostToDevice, h->stream));
-  if (norder > 0)
-    CU(cudaMemcpyAsync(h->order.p, order, sizeof(int) * norder, cudaMemcpyHostToDevice, h->stream));
-  CU(cudaEventRecord(h->h2d_done, h->stream));
-  h->h2d_pending = true;
-  /* the timed transport starts here, with the tables resident: the chunk
-     expansion is part of it */
+  const size_t in_bytes = task_bytes + sizeof(int) * norder;
+  CU(h->in.ensure(in_bytes > 0 ? in_bytes : 1));
+  if (in_bytes > 0) {
+    CU(cudaMemcpyAsync(h->in.p, h->pin_in.p, in_bytes, cudaMemcpyHostToDevice, h->stream));
+    h->busy = true;
+  }
+  ptg::ChunkQueue chunks;
+  chunks.order = reinterpret_cast<const int*>(h->in.as<char>() + task_bytes);
+  chunks.per_task = (int32_t)std::max<int64_t>(per_task, 1);
+  chunks.size = (int32_t)std::min<int64_t>(csz, std::max<int64_t>(T.np_local, 1));
+  chunks.np_local = (int32_t)T.np_local;
+  /* the timed transport starts here, with the tables resident */
   CU(cudaEventRecord(h->ev[0], h->stream));
-  if (nchunk > 0)
-    CU(ptg::launch_expand_chunks(h->order.as<const int>(), (int)norder, (int)per_task, (int)csz,
-                                 (int)T.np_local, h->chunk.as<int4>(), h->stream));
-  h->last.h2d_bytes += task_bytes + sizeof(int) * norder;
+  h->last.h2d_bytes += in_bytes;
   /* scheduling of both persistent kernels.  A lane that loops longer on the
      fast path holds its warp's other lanes: 16 steps cost 13.6 ms of drain on
      the thin film against 11.1 ms for 8. */
@@ -692,7 +702,7 @@ int run_transport(ptg_handle* h, const Transport& T) {
   if (fp64) {
     ptg::Run64 r;
     memset(&r, 0, sizeof(r));
-    r.task = h->task.as<const ptg::Task64>();
+    r.task = h->in.as<const ptg::Task64>();
     r.ntask = ntask;
     r.np = T.np;
     r.np_local = T.np_local;
@@ -703,9 +713,9 @@ int run_transport(ptg_handle* h, const Transport& T) {
     r.c1 = ((uint32_t)T.stream) << 8;
     r.max_flights = maxf;
     r.ref_quirks = h->opt.ref_quirks;
-    r.counts = h->counts.as<unsigned long long>();
-    r.lost = h->lost.as<unsigned long long>();
-    r.stats = h->stats.as<unsigned long long>();
+    r.counts = d_counts;
+    r.lost = d_lost;
+    r.stats = d_stats;
     r.replay_task = -1;
     int grid = 0, pblock = block;
     h->last.launches = 0;
@@ -713,37 +723,41 @@ int run_transport(ptg_handle* h, const Transport& T) {
       CU(ptg::launch_plain_fp64(h->g64, r, h->stream, &grid, &pblock));
       h->last.launches = 1;
     } else if (nchunk > 0) {
-      r.chunk = h->chunk.as<const int4>();
+      r.chunks = chunks;
       r.nchunk = (int32_t)nchunk;
-      r.queue = h->queue.as<int>();
+      r.queue = d_queue;
+    r.tail_hist = d_hist;
       r.regen_threshold = regen_threshold;
       r.fast_steps = fast_steps;
       r.fast_lambda_max = fast_lambda_max;
       r.round_lambda_max = (float)lmin;
       r.coop_lanes = coop_lanes;
       r.max_flights = std::min<int64_t>(maxf, 4294967295LL);
-      int bps = 0, tbps = 0;
-      CU(ptg::drain64_occupancy(block, &bps));
+      const int key = -1 - block;
+      if (h->occ_key != key) {
+        h->occ_key = 0;
+        CU(ptg::drain64_occupancy(block, &h->occ_bps));
+        CU(ptg::tail64_occupancy(block, &h->occ_tail));
+        h->occ_key = key;
+      }
+      int bps = h->occ_bps;
       if (h->opt.blocks_per_sm > 0 && h->opt.blocks_per_sm < bps) bps = h->opt.blocks_per_sm;
-      CU(ptg::tail64_occupancy(block, &tbps));
       grid = h->num_sms * std::max(bps, 1);
-      const int tgrid = h->num_sms * std::max(tbps, 1);
+      const int tgrid = h->num_sms * std::max(h->occ_tail, 1);
       if (coop_lanes > 0) {
         r.tail_cap = grid * block;
-        CU(h->tail.ensure((sizeof(float4) * ptg::kTail64Units + sizeof(int)) * (size_t)r.tail_cap +
-                          sizeof(int) * ptg::kTailOrderExtra));
+        CU(h->tail.ensure((sizeof(float4) * ptg::kTail64Units + sizeof(int)) * (size_t)r.tail_cap));
         r.tail = h->tail.as<float4>();
         r.tail_order = reinterpret_cast<int*>(r.tail + (size_t)ptg::kTail64Units * r.tail_cap);
-        CU(cudaMemsetAsync(r.tail_order + r.tail_cap, 0, sizeof(int) * ptg::kTailOrderExtra, h->stream));
         r.grace_steps = ptg::grace_passes(norder * T.np_local, (int64_t)tgrid * (block / 32));
       }
       CU(ptg::launch_drain64(h->g64, h->g32, r, grid, block, h->stream));
       if (coop_lanes > 0) {
         CU(ptg::launch_tail_order(r.tail, ptg::kTail64Units, r.tail_cap, r.queue, r.tail_order,
-                                  h->stream));
+                                  r.tail_hist, h->stream));
         CU(ptg::launch_tail64(h->g64, h->g32, r, tgrid, block, h->stream));
       }
-      h->last.launches = coop_lanes > 0 ? 4 : 2;
+      h->last.launches = coop_lanes > 0 ? 3 : 1;
     }
     CU(cudaEventRecord(h->ev[1], h->stream));
     h->last.grid = grid;
@@ -752,8 +766,8 @@ int run_transport(ptg_handle* h, const Transport& T) {
   } else {
     ptg::RunF32 r;
     memset(&r, 0, sizeof(r));
-    r.task = h->task.as<const float4>();
-    r.chunk = h->chunk.as<const int4>();
+    r.task = h->in.as<const float4>();
+    r.chunks = chunks;
     r.nchunk = (int32_t)nchunk;
     r.np = T.np;
     r.rank = T.rank;
@@ -768,10 +782,11 @@ int run_transport(ptg_handle* h, const Transport& T) {
     r.fast_lambda_max = fast_lambda_max;
     r.coop_lanes = coop_lanes;
     r.stage_test = (h->opt.tune_flags & 4) ? 1 : 0;
-    r.counts = h->counts.as<unsigned long long>();
-    r.lost = h->lost.as<unsigned long long>();
-    r.stats = h->stats.as<unsigned long long>();
-    r.queue = h->queue.as<int>();
+    r.counts = d_counts;
+    r.lost = d_lost;
+    r.stats = d_stats;
+    r.queue = d_queue;
+    r.tail_hist = d_hist;
     r.tlist = T.tlist;
     r.tlist_cap = T.tlist_cap;
     r.alist = T.alist;
@@ -784,8 +799,16 @@ int run_transport(ptg_handle* h, const Transport& T) {
     r.trace_end = T.trace_end;
     r.nsurf = h->geom.nsurf();
     const size_t smem = ptg::dynamic_smem_bytes(h->g32, h->blob_bytes);
-    int bps = 0;
-    CU(ptg::persistent_occupancy(block, smem, &bps, T.mode, h->g32.has_ext, h->g32.stage_smem != 0));
+    const int key = 1 + T.mode + 4 * block;
+    if (h->occ_key != key) {
+      h->occ_key = 0;
+      CU(ptg::persistent_occupancy(block, smem, &h->occ_bps, T.mode, h->g32.has_ext, h->g32.stage_smem != 0));
+      h->occ_tail = 0;
+      if (T.mode != ptg::MODE_TRACE)
+        CU(ptg::tail_occupancy(block, smem, &h->occ_tail, T.mode, h->g32.has_ext, h->g32.stage_smem != 0));
+      h->occ_key = key;
+    }
+    int bps = h->occ_bps;
     if (h->opt.blocks_per_sm > 0 && h->opt.blocks_per_sm < bps) bps = h->opt.blocks_per_sm;
     if (bps < 1) bps = 1;
     const int grid = h->num_sms * bps;
@@ -794,18 +817,14 @@ int run_transport(ptg_handle* h, const Transport& T) {
     const bool tail = r.coop_lanes > 0 && T.mode != ptg::MODE_TRACE;
     if (tail) {
       /* the list, then the order the tail phase takes it in */
-      CU(h->tail.ensure((sizeof(float4) * ptg::kTailUnits + sizeof(int)) * (size_t)grid * block +
-                        sizeof(int) * ptg::kTailOrderExtra));
+      CU(h->tail.ensure((sizeof(float4) * ptg::kTailUnits + sizeof(int)) * (size_t)grid * block));
       r.tail = h->tail.as<float4>();
       r.tail_cap = grid * block;
       r.tail_order = reinterpret_cast<int*>(r.tail + (size_t)ptg::kTailUnits * r.tail_cap);
-      CU(cudaMemsetAsync(r.tail_order + r.tail_cap, 0, sizeof(int) * ptg::kTailOrderExtra, h->stream));
     }
     int tgrid = 0;
     if (tail) {
-      int tbps = 0;
-      CU(ptg::tail_occupancy(block, smem, &tbps, T.mode, h->g32.has_ext, h->g32.stage_smem != 0));
-      tgrid = h->num_sms * (tbps < 1 ? 1 : tbps);
+      tgrid = h->num_sms * std::max(h->occ_tail, 1);
       if (T.mode == ptg::MODE_FORWARD)
         r.grace_steps = ptg::grace_passes(norder * T.np_local, (int64_t)tgrid * (block / 32));
     }
@@ -816,29 +835,42 @@ int run_transport(ptg_handle* h, const Transport& T) {
       CU(cudaEventRecord(h->ev[4], h->stream));
       if (tail) {
         CU(ptg::launch_tail_order(r.tail, ptg::kTailUnits, r.tail_cap, r.queue, r.tail_order,
-                                  h->stream));
+                                  r.tail_hist, h->stream));
         CU(ptg::launch_tail_fp32(h->g32, r, tgrid, block, smem, h->stream, T.mode));
       }
     }
     CU(cudaEventRecord(h->ev[1], h->stream));
     h->last.grid = grid;
     h->last.block = block;
-    h->last.launches = (work ? (tail ? 3 : 1) : 0) + (r.nchunk > 0 ? 1 : 0);
+    h->last.launches = work ? (tail ? 3 : 1) : 0;
     h->fp32_split = work;
     h->tail_cap = tail ? r.tail_cap : 0;
   }
   return PTG_OK;
 }
 
-int finish_stats(ptg_handle* h) {
+/* Reads the call's front back, with the counts of its first ncount tasks
+   (*counts, in pinned staging until the next call), and `extra` bytes from
+   dextra (*hextra), in pinned staging as well; waits for the stream. */
+int finish_stats(ptg_handle* h, int64_t ncount = 0, const unsigned long long** counts = nullptr,
+                 const void* dextra = nullptr, size_t extra = 0, const double** hextra = nullptr) {
+  const size_t front = CallLayout::kCounts + sizeof(unsigned long long) * ncount;
+  CU(h->pin_out.ensure(front + extra));
+  char* const pin = h->pin_out.as<char>();
+  h->busy = true;
+  CU(cudaMemcpyAsync(pin, h->call.p, front, cudaMemcpyDeviceToHost, h->stream));
+  if (extra > 0) CU(cudaMemcpyAsync(pin + front, dextra, extra, cudaMemcpyDeviceToHost, h->stream));
+  CU(cudaStreamSynchronize(h->stream));
+  h->busy = false;
+  if (counts) *counts = reinterpret_cast<const unsigned long long*>(pin + CallLayout::kCounts);
+  if (hextra) *hextra = reinterpret_cast<const double*>(pin + front);
   unsigned long long st[ptg::kStatSlots];
   int qerr[8];
-  CU(cudaMemcpyAsync(st, h->stats.p, sizeof(st), cudaMemcpyDeviceToHost, h->stream));
-  CU(cudaMemcpyAsync(qerr, h->queue.p, sizeof(qerr), cudaMemcpyDeviceToHost, h->stream));
-  CU(cudaStreamSynchronize(h->stream));
+  memcpy(st, pin, sizeof(st));
+  memcpy(qerr, pin + CallLayout::kQueue, sizeof(qerr));
   float ms = 0.f;
   CU(cudaEventElapsedTime(&ms, h->ev[0], h->ev[1]));
-  h->last.d2h_bytes += sizeof(st) + sizeof(qerr);
+  h->last.d2h_bytes += front + extra;
   h->last.flights = st[0];
   h->last.lost = st[1];
   h->last.capped = st[2];
@@ -863,9 +895,11 @@ int finish_stats(ptg_handle* h) {
   }
   h->list_n = st[10];
   h->mismatch = st[11];
-  if (st[5] != ~0ull && st[7] >= st[5]) {
-    const unsigned long long drain = st[6] != ~0ull ? st[6] : st[7];
-    h->last.drain_ms = (double)(drain - st[5]) * 1e-6;
+  /* start and dry queue are kept as the largest complement (0: none) */
+  const unsigned long long start = ~st[5];
+  if (st[5] != 0 && st[7] >= start) {
+    const unsigned long long drain = st[6] != 0 ? ~st[6] : st[7];
+    h->last.drain_ms = (double)(drain - start) * 1e-6;
     h->last.tail_ms = (double)(st[7] - drain) * 1e-6;
   }
   if (qerr[1] != 0) { h->last_error = "shared-memory staging wait timed out"; return PTG_ERR_TIMEOUT; }
@@ -1088,10 +1122,6 @@ int ptg_create(const ptg_geometry* geom, const ptg_spectrum* spec, const ptg_opt
     }
     for (auto& e : h->ev)
       if (cudaEventCreate(&e) != cudaSuccess) { delete h; return PTG_ERR_CUDA; }
-    if (cudaEventCreateWithFlags(&h->h2d_done, cudaEventDisableTiming) != cudaSuccess) {
-      delete h;
-      return PTG_ERR_CUDA;
-    }
     st = build_geo64(h);
     if (st == PTG_OK) st = build_blob(h);
     if (st != PTG_OK) { delete h; return st; }
@@ -1176,10 +1206,10 @@ int ptg_transmission(ptg_handle* h, double mfp_nm, int32_t nangle, int64_t np, i
     const int64_t ntask = nm * (nangle - 1);
     std::vector<ptg::TaskHost> tasks(ntask);
     const double half_pi = 3.14159265358979323846 * 0.5;
-    for (int64_t t = 0; t < ntask; ++t) {
-      const int64_t m = t % nm, ia = t / nm;
+    for (int64_t ia = 0; ia < nangle - 1; ++ia) {
       const double theta = 0.0 + (double)ia / (double)(nangle - 1) * half_pi;
-      tasks[t] = {mfp_nm, cos(theta), sin(theta), h->spec.omega[m]};
+      const double ct = cos(theta), sn = sin(theta);
+      for (int64_t m = 0; m < nm; ++m) tasks[ia * nm + m] = {mfp_nm, ct, sn, h->spec.omega[m]};
     }
     Transport T;
     T.ntask = ntask;
@@ -1194,11 +1224,8 @@ int ptg_transmission(ptg_handle* h, double mfp_nm, int32_t nangle, int64_t np, i
     T.npair = h->spec.nmode();
     int st = run_transport(h, T);
     if (st != PTG_OK) return st;
-    std::vector<unsigned long long> cnt(ntask);
-    CU(cudaMemcpyAsync(cnt.data(), h->counts.p, sizeof(unsigned long long) * ntask,
-                       cudaMemcpyDeviceToHost, h->stream));
-    h->last.d2h_bytes += sizeof(unsigned long long) * ntask;
-    st = finish_stats(h);
+    const unsigned long long* cnt = nullptr;
+    st = finish_stats(h, ntask, &cnt);
     if (st != PTG_OK) return st;
     for (int64_t t = 0; t < nm * nangle; ++t) {
       double v = 0.0;
@@ -1247,32 +1274,32 @@ int ptg_kappa(ptg_handle* h, const ptg_run* run, ptg_kappa_out* out) {
     double dS = 0.0;
     ptg::simpson_weights(run->nangle, h->geom.box[0], &coef, &dS);
     const int nbins = run->nbins;
-    CU(h->red_coef.ensure(sizeof(double) * coef.size()));
-    CU(h->red_K.ensure(sizeof(double) * nm));
-    CU(h->red_W.ensure(sizeof(double) * nm));
-    CU(h->red_mfp.ensure(sizeof(double) * nm));
-    CU(h->red_bin.ensure(sizeof(int) * nm));
-    CU(h->red_grid.ensure(sizeof(double) * ns));
-    CU(h->red_tc.ensure(sizeof(double) * nm));
-    CU(h->red_kv.ensure(sizeof(double) * nm));
-    CU(h->red_bw.ensure(sizeof(double) * nm));
-    CU(h->red_bv.ensure(sizeof(double) * nm));
-    CU(h->red_emfp.ensure(sizeof(double) * nm));
+    /* constants in one copy: coef, K, W, MFPs, grid, then the bins */
+    const size_t na = coef.size(), nconst = na + 3 * (size_t)nm + ns;
+    const size_t const_bytes = sizeof(double) * nconst + sizeof(int) * (size_t)nm;
+    CU(h->pin_const.ensure(const_bytes));
+    CU(h->red_in.ensure(const_bytes));
+    CU(h->red_tmp.ensure(sizeof(double) * 4 * nm));
+    const size_t nres = 2 + 3 * (size_t)nbins;
+    CU(h->red_out.ensure(sizeof(double) * (nres + nm)));
     CU(h->red_trans.ensure(sizeof(double) * nm * ns * run->nangle));
-    CU(h->red_result.ensure(sizeof(double) * (2 + 3 * (size_t)nbins)));
     cudaStream_t s = h->stream;
-    CU(cudaMemcpyAsync(h->red_coef.p, coef.data(), sizeof(double) * coef.size(), cudaMemcpyHostToDevice, s));
-    CU(cudaMemcpyAsync(h->red_K.p, mc.K.data(), sizeof(double) * nm, cudaMemcpyHostToDevice, s));
-    CU(cudaMemcpyAsync(h->red_W.p, mc.W.data(), sizeof(double) * nm, cudaMemcpyHostToDevice, s));
-    CU(cudaMemcpyAsync(h->red_mfp.p, mc.mfp_m.data(), sizeof(double) * nm, cudaMemcpyHostToDevice, s));
-    CU(cudaMemcpyAsync(h->red_bin.p, mc.bin.data(), sizeof(int) * nm, cudaMemcpyHostToDevice, s));
-    if (run->kind_mfp == PTG_MFP_GRID)
-      CU(cudaMemcpyAsync(h->red_grid.p, run->mfp_grid_nm, sizeof(double) * ns, cudaMemcpyHostToDevice, s));
-    h->last.h2d_bytes += sizeof(double) * (coef.size() + 3 * (size_t)nm) + sizeof(int) * nm +
-                         (run->kind_mfp == PTG_MFP_GRID ? sizeof(double) * ns : 0);
+    double* const pc = h->pin_const.as<double>();
+    std::copy(coef.begin(), coef.end(), pc);
+    std::copy(mc.K.begin(), mc.K.end(), pc + na);
+    std::copy(mc.W.begin(), mc.W.end(), pc + na + nm);
+    std::copy(mc.mfp_m.begin(), mc.mfp_m.end(), pc + na + 2 * nm);
+    for (int k = 0; k < ns; ++k)
+      pc[na + 3 * nm + k] = run->kind_mfp == PTG_MFP_GRID ? run->mfp_grid_nm[k] : 0.0;
+    std::copy(mc.bin.begin(), mc.bin.end(), reinterpret_cast<int*>(pc + nconst));
+    CU(cudaMemcpyAsync(h->red_in.p, pc, const_bytes, cudaMemcpyHostToDevice, s));
+    h->last.h2d_bytes += const_bytes;
+    const double* const dc = h->red_in.as<const double>();
+    double* const dt = h->red_tmp.as<double>();
+    double* const dres = h->red_out.as<double>();
     ptg::ReduceIn in;
     memset(&in, 0, sizeof(in));
-    in.counts = h->counts.as<const unsigned long long>();
+    in.counts = reinterpret_cast<const unsigned long long*>(h->call.as<char>() + CallLayout::kCounts);
     in.nmode = nm;
     in.nangle = run->nangle;
     in.ns = ns;
@@ -1281,40 +1308,37 @@ int ptg_kappa(ptg_handle* h, const ptg_run* run, ptg_kappa_out* out) {
     in.np = (double)run->np;
     in.dS = dS;
     in.tnorm = 0.75 * h->geom.box[0];
-    in.coef = h->red_coef.as<const double>();
-    in.K = h->red_K.as<const double>();
-    in.W = h->red_W.as<const double>();
-    in.mfp_m = h->red_mfp.as<const double>();
-    in.bin = h->red_bin.as<const int>();
-    in.grid = h->red_grid.as<const double>();
-    in.tc = h->red_tc.as<double>();
-    in.kv = h->red_kv.as<double>();
-    in.bw = h->red_bw.as<double>();
-    in.bv = h->red_bv.as<double>();
-    in.emfp_nm = h->red_emfp.as<double>();
+    in.coef = dc;
+    in.K = dc + na;
+    in.W = dc + na + nm;
+    in.mfp_m = dc + na + 2 * nm;
+    in.grid = dc + na + 3 * nm;
+    in.bin = reinterpret_cast<const int*>(dc + nconst);
+    in.tc = dt;
+    in.kv = dt + nm;
+    in.bw = dt + 2 * nm;
+    in.bv = dt + 3 * nm;
+    in.result = dres;
+    in.emfp_nm = dres + nres;
     in.transmit = h->red_trans.as<double>();
-    in.result = h->red_result.as<double>();
     {
       ptg::NvtxRange nvtx("ptg kappa reduction");
       CU(cudaEventRecord(h->ev[2], s));
       CU(ptg::launch_kappa_reduce(in, s));
       CU(cudaEventRecord(h->ev[3], s));
     }
-    std::vector<double> res(2 + 3 * (size_t)nbins);
-    CU(cudaMemcpyAsync(res.data(), h->red_result.p, sizeof(double) * res.size(), cudaMemcpyDeviceToHost, s));
-    if (out->emfp_nm)
-      CU(cudaMemcpyAsync(out->emfp_nm, h->red_emfp.p, sizeof(double) * nm, cudaMemcpyDeviceToHost, s));
-    if (out->transmit)
+    if (out->transmit) {
       CU(cudaMemcpyAsync(out->transmit, h->red_trans.p, sizeof(double) * nm * ns * run->nangle,
                          cudaMemcpyDeviceToHost, s));
-    if (out->counts)
-      CU(cudaMemcpyAsync(out->counts, h->counts.p, sizeof(unsigned long long) * T.ntask,
-                         cudaMemcpyDeviceToHost, s));
-    h->last.d2h_bytes += sizeof(double) * res.size() + (out->emfp_nm ? sizeof(double) * nm : 0) +
-                         (out->transmit ? sizeof(double) * nm * ns * run->nangle : 0) +
-                         (out->counts ? sizeof(unsigned long long) * T.ntask : 0);
-    st = finish_stats(h);
+      h->last.d2h_bytes += sizeof(double) * nm * ns * run->nangle;
+    }
+    const unsigned long long* cnt = nullptr;
+    const double* res = nullptr;
+    st = finish_stats(h, out->counts ? T.ntask : 0, &cnt, dres,
+                      sizeof(double) * (nres + (out->emfp_nm ? nm : 0)), &res);
     if (st != PTG_OK) return st;
+    if (out->counts) memcpy(out->counts, cnt, sizeof(unsigned long long) * T.ntask);
+    if (out->emfp_nm) memcpy(out->emfp_nm, res + nres, sizeof(double) * nm);
     float rms = 0.f;
     CU(cudaEventElapsedTime(&rms, h->ev[2], h->ev[3]));
     h->last.reduce_ms = rms;
@@ -1502,11 +1526,10 @@ int ptg_adjoint(ptg_handle* h, const ptg_run* run, ptg_adjoint_out* out) {
     T.tlist = h->adj_list.as<unsigned long long>();
     int st = run_transport(h, T);
     if (st != PTG_OK) return st;
-    std::vector<uint64_t> counts(ntask);
-    CU(cudaMemcpyAsync(counts.data(), h->counts.p, sizeof(uint64_t) * ntask, cudaMemcpyDeviceToHost,
-                       h->stream));
-    st = finish_stats(h);
+    const unsigned long long* cnt = nullptr;
+    st = finish_stats(h, ntask, &cnt);
     if (st != PTG_OK) return st;
+    const std::vector<uint64_t> counts(cnt, cnt + ntask);
     const double fwd_ms = h->last.kernel_ms;
     const uint64_t fwd_flights = h->last.flights;
     const unsigned long long nlist = h->list_n;

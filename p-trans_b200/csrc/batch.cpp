@@ -107,12 +107,13 @@ static cudaError_t launch_phases(ptg_batch* b, ptg::RunF32 r, int mode) {
   r.grace_steps =
       mode == ptg::MODE_FORWARD ? ptg::grace_passes(b->samples, (int64_t)tgrid * (block / 32)) : 0;
   cudaError_t e = cudaMemsetAsync(b->queue.p, 0, sizeof(int) * 8, b->stream);
+  r.tail_hist = r.tail_order + r.tail_cap;
   if (e == cudaSuccess && tgrid > 0)
-    e = cudaMemsetAsync(r.tail_order + r.tail_cap, 0, sizeof(int) * ptg::kTailOrderExtra, b->stream);
+    e = cudaMemsetAsync(r.tail_hist, 0, sizeof(int) * ptg::kTailOrderExtra, b->stream);
   if (e == cudaSuccess)
     e = ptg::launch_persistent_batch(r, b->drain_grid[mode], block, b->stream, b->ext, mode, false);
   if (e == cudaSuccess && tgrid > 0)
-    e = ptg::launch_tail_order(r.tail, ptg::kTailUnits, r.tail_cap, r.queue, r.tail_order, b->stream);
+    e = ptg::launch_tail_order(r.tail, ptg::kTailUnits, r.tail_cap, r.queue, r.tail_order, r.tail_hist, b->stream);
   if (e == cudaSuccess && tgrid > 0)
     e = ptg::launch_persistent_batch(r, tgrid, block, b->stream, b->ext, mode, true);
   return e;
@@ -356,16 +357,12 @@ extern "C" int ptg_batch_create(const ptg_batch_item* items, int32_t nitems,
                       sizeof(int) * ptg::kTailOrderExtra));
 
     /* capture: clear tallies, transport, reduction, results to pinned memory */
-    const unsigned long long init[16] = {0, 0, 0, 0, 0, ~0ull, ~0ull, 0, 0, 0, 0, 0, 0, 0, 0, 0};
-    static_assert(sizeof(init) == 16 * sizeof(unsigned long long), "stats layout");
     unsigned long long* dstats = b->stats.as<unsigned long long>();
-    BCU(cudaMemcpy(b->host_stats, init, sizeof(init), cudaMemcpyHostToHost));
     BCU(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
     cudaError_t ce = cudaMemsetAsync(b->counts.p, 0, sizeof(unsigned long long) * ntot, b->stream);
     if (ce == cudaSuccess) ce = cudaMemsetAsync(b->lost.p, 0, sizeof(unsigned long long) * ntot, b->stream);
     if (ce == cudaSuccess)
       ce = cudaMemsetAsync(dstats, 0, sizeof(unsigned long long) * ptg::kStatSlots, b->stream);
-    if (ce == cudaSuccess) ce = cudaMemsetAsync(dstats + 5, 0xFF, sizeof(unsigned long long) * 2, b->stream);
     if (ce == cudaSuccess && r.nchunk > 0) ce = launch_phases(b, r, ptg::MODE_FORWARD);
     if (ce == cudaSuccess) ce = ptg::launch_kappa_reduce_batch(rb, b->stream);
     if (ce == cudaSuccess)
@@ -441,7 +438,6 @@ static int batch_launch(ptg_batch* b, const ptg::RunF32& r, int mode, unsigned l
   if (cudaMemsetAsync(b->counts.p, 0, sizeof(unsigned long long) * ntot, b->stream) != cudaSuccess ||
       cudaMemsetAsync(b->lost.p, 0, sizeof(unsigned long long) * ntot, b->stream) != cudaSuccess ||
       cudaMemsetAsync(dstats, 0, sizeof(unsigned long long) * ptg::kStatSlots, b->stream) != cudaSuccess ||
-      cudaMemsetAsync(dstats + 5, 0xFF, sizeof(unsigned long long) * 2, b->stream) != cudaSuccess ||
       cudaEventRecord(b->ev0, b->stream) != cudaSuccess)
     return PTG_ERR_CUDA;
   const bool work = mode == ptg::MODE_ADJOINT ? r.alist_n > 0 : r.nchunk > 0;

@@ -279,6 +279,13 @@ __device__ __forceinline__ int order_bucket(float x, float x_len, float lam) {
   return w > 1.0f ? min(kOrderBuckets - 1, (int)(4.0f * __log2f(w))) : 0;
 }
 
+/* Chunk c of the work queue: (task, first local particle, count). */
+__device__ __forceinline__ int3 queue_chunk(const ChunkQueue& q, int c) {
+  const int k = c / q.per_task;
+  const int j = (c - k * q.per_task) * q.size;
+  return make_int3(__ldg(q.order + k), j, min(q.size, q.np_local - j));
+}
+
 __device__ __forceinline__ unsigned lanemask_lt() {
   unsigned m;
   asm volatile("mov.u32 %0, %%lanemask_lt;" : "=r"(m));

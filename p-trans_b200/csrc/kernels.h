@@ -47,6 +47,13 @@ struct Task64 {
   double lambda, cth, sth, omega;
 };
 
+/* Work queue of a run: chunk c is particles [j, j + size), j = (c % per_task)
+   size, of task order[c / per_task], clipped to np_local. */
+struct ChunkQueue {
+  const int* order;          /* tasks, longest expected trajectories first      */
+  int32_t per_task, size, np_local;
+};
+
 struct Run64 {
   const Task64* task;
   int64_t ntask;
@@ -66,7 +73,7 @@ struct Run64 {
   double* final_pos;
   /* persistent kernels: the work queue, scheduling and tail list of RunF32
      (kTail64Units float4 per phonon; queue[4] phonons on the list) */
-  const int4* chunk;
+  ChunkQueue chunks;
   int32_t nchunk;
   int* queue;
   int32_t regen_threshold, fast_steps, coop_lanes, grace_steps;
@@ -75,6 +82,7 @@ struct Run64 {
   float4* tail;
   int32_t tail_cap;
   int32_t* tail_order;
+  int32_t* tail_hist;
 };
 
 cudaError_t launch_plain_fp64(const Geo64& g, const Run64& r, cudaStream_t st, int* grid,
@@ -142,6 +150,7 @@ struct GeoEntry {
 struct RunF32 {
   const float4* task;
   const int4* chunk;          /* (task, first local particle, count, 0) in LPT order */
+  ChunkQueue chunks;          /* ... or, chunk NULL, what they follow from          */
   int32_t nchunk;
   int64_t np;
   int32_t rank, nranks;
@@ -162,13 +171,16 @@ struct RunF32 {
   int32_t tail_cap;           /* its capacity in phonons                           */
   int32_t* tail_order;        /* the tail phase takes list slots in this order
                                  (launch_tail_order), else front then back         */
+  int32_t* tail_hist;         /* order buckets' histogram and cursors
+                                 (kTailOrderExtra ints, zeroed before the drain)   */
   int32_t stage_test;         /* test only: set up the shared-memory staging
                                  barrier without issuing the copy, so its
                                  bounded wait runs out (PTG_ERR_TIMEOUT)          */
   unsigned long long* counts;
   unsigned long long* lost;
   /* flights, lost, capped, samples, max trajectory flights,
-     t_start (min), t_drain (min), t_end (max) in globaltimer ns,
+     t_start and t_drain (the largest complement, 0: none), t_end (max) in
+     globaltimer ns,
      flights taken with the intersection test, safe balls built */
   unsigned long long* stats;
   int* queue;                 /* [0] next chunk, [1] error flags, [2] / [4] phonons
@@ -251,13 +263,13 @@ cudaError_t launch_persistent_fp32(const GeoF32& g, const RunF32& r, int grid, i
 /* The tail phase after it (forward, list and adjoint modes): the phonons
    the drain phase left in r.tail, one per warp. */
 /* Orders the tail list for the tail phase, longest expected remaining walk
-   first: tail_cap ints, then kTailOrderExtra for the buckets' histogram, which
-   the drain phase fills as it hands phonons over, and their cursors (both
-   zeroed by the caller before the drain).  One kernel between the drain and
-   the tail launch on the same stream. */
+   first, into order (tail_cap ints) from the buckets' histogram that the drain
+   phase fills as it hands phonons over (hist: kTailOrderExtra ints with the
+   buckets' cursors, zeroed by the caller before the drain).  One kernel between
+   the drain and the tail launch on the same stream. */
 constexpr int kTailOrderExtra = 256;
 cudaError_t launch_tail_order(const float4* tail, int units, int tail_cap, const int* queue,
-                              int32_t* order, cudaStream_t st);
+                              int32_t* order, int32_t* hist, cudaStream_t st);
 /* The FP64 pair: the same queue and list, FP64 flights; the blob of g32 gives
    the bounds for balls and BVH walks. */
 cudaError_t drain64_occupancy(int block, int* blocks_per_sm);
@@ -296,10 +308,6 @@ inline size_t dynamic_smem_bytes(const GeoF32& g, size_t blob_bytes) {
   if (g.stage_smem) return blob_bytes;
   return (size_t)g.node_stage * 16u;
 }
-/* Fills the chunk table (task, first local particle, count, 0): per_task
-   chunks of csz particles for each task of `order`, in that order. */
-cudaError_t launch_expand_chunks(const int* order, int norder, int per_task, int csz, int np_local,
-                                 int4* chunks, cudaStream_t st);
 /* Violations recorded by the bounds-checked build (PT_CHECK); other builds
    return cudaErrorNotSupported. */
 cudaError_t check_report(long long* count, int* code, int* index, bool reset);

@@ -987,7 +987,7 @@ __global__ void __launch_bounds__(kBlock,
   typename std::conditional<BATCH, GeoBatch, Geo<SMEM>>::type G;
   G.lay = gp.lay;
   G.base = gp.blob;
-  if (PH == PH_DRAIN && threadIdx.x == 0) atomicMin(r.stats + 5, globaltimer());
+  if (PH == PH_DRAIN && threadIdx.x == 0) atomicMax(r.stats + 5, ~globaltimer());
   if (SMEM) {
     /* on a timeout the block records the error and takes no work: the host
        reports it */
@@ -1140,7 +1140,7 @@ __global__ void __launch_bounds__(kBlock,
             /* the replay list in chunks of 32 sample ids */
             if ((long long)c * 32 >= r.alist_n) {
               queue_done = true;
-              if (lane == 0) atomicMin(r.stats + 6, globaltimer());
+              if (lane == 0) atomicMax(r.stats + 6, ~globaltimer());
               break;
             }
             ch_next = c * 32;
@@ -1149,11 +1149,16 @@ __global__ void __launch_bounds__(kBlock,
             if (c >= r.nchunk) {
               queue_done = true;
               ch_left = r.grace_steps;  /* from here on: passes before a hand-over */
-              if (lane == 0) atomicMin(r.stats + 6, globaltimer());
+              if (lane == 0) atomicMax(r.stats + 6, ~globaltimer());
               break;
             }
-            const int4 q = r.chunk[c];
-            ch_task = q.x; ch_next = q.y; ch_left = q.z;
+            if (r.chunk) {
+              const int4 q = r.chunk[c];
+              ch_task = q.x; ch_next = q.y; ch_left = q.z;
+            } else {
+              const int3 q = queue_chunk(r.chunks, c);
+              ch_task = q.x; ch_next = q.y; ch_left = q.z;
+            }
           }
         }
         const int take = min(__popc(idle), ch_left);
@@ -1312,7 +1317,7 @@ __global__ void __launch_bounds__(kBlock,
                              gr2);
           const int bucket = order_bucket(px, X, lam);
           e[6] = make_float4(g2r2, __int_as_float(gnear), __int_as_float(bucket), 0.0f);
-          atomicAdd(r.tail_order + r.tail_cap + bucket, 1);
+          atomicAdd(r.tail_hist + bucket, 1);
           if (MODE == MODE_ADJOINT)
             e[5] = make_float4(adj_w, adj_len, __uint_as_float(adj_npp), __int_as_float(adj_b));
           atomicAdd(r.stats + 16, (unsigned long long)flight);
@@ -1943,6 +1948,8 @@ __global__ void __launch_bounds__(kBlock,
    every launch with a staged blob opts in to its dynamic size. */
 template <int MODE, int EXT, int PH, bool SMEM = true>
 cudaError_t allow_dynamic_smem(size_t smem) {
+  /* at most 27 KB of any kernel here is static */
+  if (smem <= 20 * 1024) return cudaSuccess;
   return cudaFuncSetAttribute(k_persistent<SMEM, MODE, false, EXT, PH>,
                               cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
 }
@@ -2090,19 +2097,6 @@ cudaError_t launch_tail_fp32(const GeoF32& g, const RunF32& r, int grid, int blo
 }
 
 namespace {
-/* Chunk table of a run: chunk c is particles [j, j + count) of task
-   order[c / per_task], j = (c % per_task) * csz, in the queue's order. */
-__global__ void k_expand_chunks(const int* __restrict__ order, int norder, int per_task, int csz,
-                                int np_local, int4* __restrict__ chunks) {
-  const long long n = (long long)norder * per_task;
-  for (long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x; c < n;
-       c += (long long)gridDim.x * blockDim.x) {
-    const int k = (int)(c / per_task);
-    const int j = (int)(c - (long long)k * per_task) * csz;
-    chunks[c] = make_int4(__ldg(order + k), j, min(csz, np_local - j), 0);
-  }
-}
-
 /* Hand-over c of the tail list: its slot (front list, then back list). */
 __device__ __forceinline__ int tail_slot(int c, int nlong, int tail_cap) {
   return c < nlong ? c : tail_cap - 1 - (c - nlong);
@@ -2137,21 +2131,10 @@ __global__ void k_order_scatter(const float4* __restrict__ tail, int units, int 
 }  // namespace
 
 cudaError_t launch_tail_order(const float4* tail, int units, int tail_cap, const int* queue,
-                              int32_t* order, cudaStream_t st) {
-  int* hist = order + tail_cap;
+                              int32_t* order, int32_t* hist, cudaStream_t st) {
   const unsigned blocks = (unsigned)((tail_cap + 255) / 256);
   k_order_scatter<<<blocks, 256, 0, st>>>(tail, units, tail_cap, queue, hist, hist + kOrderBuckets,
                                           order);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_expand_chunks(const int* order, int norder, int per_task, int csz, int np_local,
-                                 int4* chunks, cudaStream_t st) {
-  const long long n = (long long)norder * per_task;
-  if (n <= 0) return cudaSuccess;
-  const long long blocks = (n + 255) / 256;
-  k_expand_chunks<<<(unsigned)(blocks < 4096 ? blocks : 4096), 256, 0, st>>>(order, norder, per_task, csz,
-                                                                            np_local, chunks);
   return cudaGetLastError();
 }
 

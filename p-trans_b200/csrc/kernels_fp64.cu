@@ -757,7 +757,7 @@ __global__ void __launch_bounds__(256, 2) k_drain64(Geo64 g, GeoF32 gp, Run64 r)
           if (lane == 0) c = atomicAdd(r.queue, 1);
           c = __shfl_sync(FULL, c, 0);
           if (c >= r.nchunk) { queue_done = true; break; }
-          const int4 q = r.chunk[c];
+          const int3 q = queue_chunk(r.chunks, c);
           ch_task = q.x; ch_next = q.y; ch_left = q.z;
         }
         const int take = min(__popc(idle), ch_left);
@@ -814,7 +814,7 @@ __global__ void __launch_bounds__(256, 2) k_drain64(Geo64 g, GeoF32 gp, Run64 r)
           const int bucket = order_bucket((float)p.pos[0], gp.box[0], lam);
           e[6] = make_float4(__int_as_float(p.igrain), __int_as_float(p.isurf),
                              __int_as_float(bucket), __int_as_float(p.which));
-          atomicAdd(r.tail_order + r.tail_cap + bucket, 1);
+          atomicAdd(r.tail_hist + bucket, 1);
           e[7] = make_float4(__int_as_float(task), __uint_as_float((uint32_t)sample),
                              __uint_as_float((uint32_t)(sample >> 32)), __uint_as_float(flight));
           alive = false;

@@ -143,7 +143,6 @@ extern "C" int ptg_transmission_noalloc(ptg_handle* h, double mfp_nm, int32_t na
   unsigned long long* lost = reinterpret_cast<unsigned long long*>(base + kOffLost);
   /* clear what the kernel accumulates into; the tables are rewritten */
   if (cudaMemsetAsync(stats, 0, ptg::kStatSlots * sizeof(unsigned long long), s) != cudaSuccess ||
-      cudaMemsetAsync(stats + 5, 0xFF, 2 * sizeof(unsigned long long), s) != cudaSuccess ||
       cudaMemsetAsync(queue, 0, 8 * sizeof(int), s) != cudaSuccess ||
       cudaMemsetAsync(counts, 0, sizeof(unsigned long long) * ntask, s) != cudaSuccess ||
       cudaMemsetAsync(lost, 0, sizeof(unsigned long long) * ntask, s) != cudaSuccess ||
@@ -199,7 +198,8 @@ extern "C" int ptg_transmission_noalloc(ptg_handle* h, double mfp_nm, int32_t na
     r.tail = reinterpret_cast<float4*>(base + kOffTail);
     r.tail_cap = std::min(kMaxTail, grid * block);
     r.tail_order = reinterpret_cast<int*>(base + kOffOrder);
-    if (cudaMemsetAsync(r.tail_order + r.tail_cap, 0, sizeof(int) * ptg::kTailOrderExtra, s) != cudaSuccess)
+    r.tail_hist = r.tail_order + kMaxTail;
+    if (cudaMemsetAsync(r.tail_hist, 0, sizeof(int) * ptg::kTailOrderExtra, s) != cudaSuccess)
       return PTG_ERR_CUDA;
     int tbps = 0;
     if (ptg::tail_occupancy(block, smem, &tbps, ptg::MODE_FORWARD, v.g32.has_ext, v.g32.stage_smem != 0) != cudaSuccess)
@@ -210,7 +210,7 @@ extern "C" int ptg_transmission_noalloc(ptg_handle* h, double mfp_nm, int32_t na
   if (r.nchunk > 0) {
     if (ptg::launch_persistent_fp32(v.g32, r, grid, block, smem, s) != cudaSuccess)
       return PTG_ERR_CUDA;
-    if (tgrid > 0 && (ptg::launch_tail_order(r.tail, ptg::kTailUnits, r.tail_cap, r.queue, r.tail_order, s) != cudaSuccess ||
+    if (tgrid > 0 && (ptg::launch_tail_order(r.tail, ptg::kTailUnits, r.tail_cap, r.queue, r.tail_order, r.tail_hist, s) != cudaSuccess ||
                       ptg::launch_tail_fp32(v.g32, r, tgrid, block, smem, s) != cudaSuccess))
       return PTG_ERR_CUDA;
   }

@@ -899,11 +899,15 @@ __global__ void __launch_bounds__(256, 2) k_drain64(Geo64 g, GeoF32 gp, Run64 r)
 
 /* flights a round tests from its first one that walks a BVH */
 constexpr int kTestWindow64 = 4;
+/* flights in a row that have to be drawn for a round to go without drawing:
+   at 4 / 8 / 16 / 24 the 300 nm wire takes 9.60 / 9.51 / 9.43 / 9.62 ms, and
+   10.2 where every round draws all of its flights */
+constexpr int kReady64 = 16;
 /* double2 between the rows of a warp's round */
 constexpr int kRow64 = 33;
 
 /* Tail phase: one phonon per warp, 32 flights a round, one per lane.  Every
-   lane holds the phonon.  Lane j draws what flight f+1+j ends with if it ends
+   lane holds the phonon.  A lane draws what its flight ends with if it ends
    in an intrinsic event (the blocks depend on the counter alone); the moves
    fp d and the nudges are products of those draws, so only their sums run one
    after the other: lane c < 3 adds coordinate c's, two additions a flight,
@@ -941,17 +945,34 @@ __global__ void __launch_bounds__(256, 2) k_tail64(Geo64 g, GeoF32 gp, Run64 r) 
     const double omega = r.task[task].omega;
     int end_side = -1;
     bool capped = false;
+    double nd[3] = {0.0, 0.0, 0.0}, nf = 0.0;
+    uint32_t drawn = 0;  /* the flight that the lane's draws are for */
     while (end_side < 0) {
-      double nd[3], nf;
-      pp_draw64(rng, lambda, flight + 1u + (uint32_t)lane, nd, &nf);
-      /* flight `lane` starts with what the previous one drew */
-      double sfp = __shfl_up_sync(FULL, nf, 1), sd[3];
-      if (lane == 0) sfp = p.fp;
+      /* the lane's flight is the next whose number is `lane` modulo 32, so
+         what it drew serves later rounds too; the lanes whose flight has
+         passed draw again once fewer than kReady64 flights in a row are ready */
+      const int base = (int)((flight + 1u) & 31u);
+      const int off = (lane - base) & 31;
+      const uint32_t mine = flight + 1u + (uint32_t)off;
+      unsigned ready = __ballot_sync(FULL, drawn == mine);
+      ready = __funnelshift_r(ready, ready, base);
+      int nready = ready == FULL ? 32 : __ffs(~ready) - 1;
+      if (nready < kReady64) {
+        if (drawn != mine) {
+          pp_draw64(rng, lambda, mine, nd, &nf);
+          drawn = mine;
+        }
+        nready = 32;
+        __syncwarp();
+      }
+      /* flight `off` starts with what the previous one drew */
+      double sfp = __shfl_sync(FULL, nf, (lane - 1) & 31), sd[3];
+      if (off == 0) sfp = p.fp;
 #pragma unroll
       for (int d = 0; d < 3; ++d) {
-        sd[d] = __shfl_up_sync(FULL, nd[d], 1);
-        if (lane == 0) sd[d] = p.dir[d];
-        row[d * kRow64 + lane] = make_double2(sfp * sd[d], 1.0e-7 * nd[d]);
+        sd[d] = __shfl_sync(FULL, nd[d], (lane - 1) & 31);
+        if (off == 0) sd[d] = p.dir[d];
+        row[d * kRow64 + off] = make_double2(sfp * sd[d], 1.0e-7 * nd[d]);
       }
       __syncwarp();
       if (lane < 3) {
@@ -977,63 +998,67 @@ __global__ void __launch_bounds__(256, 2) k_tail64(Geo64 g, GeoF32 gp, Run64 r) 
       double sp[3], sq[3];
 #pragma unroll
       for (int d = 0; d < 3; ++d) {
-        sq[d] = row[d * kRow64 + lane].x;
-        sp[d] = lane == 0 ? p.pos[d] : row[d * kRow64 + (lane > 0 ? lane - 1 : 0)].y;
+        sq[d] = row[d * kRow64 + off].x;
+        sp[d] = off == 0 ? p.pos[d] : row[d * kRow64 + (off > 0 ? off - 1 : 0)].y;
       }
       const float se = off2(sq, bx, by, bz), ss = off2(sp, bx, by, bz);
       const bool in_ball = se < br2 && ss < br2;
       const bool in_gball = se < gr2 && ss < gr2;
       const bool inbox = in_box64(g, sp);
-      const bool brk = !inbox || (int64_t)flight + lane >= r.max_flights;
+      const bool brk = !inbox || (int64_t)flight + off >= r.max_flights;
       const bool walks =
           !in_ball && !in_gball && p.which > 0 && G.bvh_root(p.which) >= 0 &&
           !behind_planes(G, p.which, (float)sp[0], (float)sp[1], (float)sp[2], (float)sd[0],
                          (float)sd[1], (float)sd[2], (float)sfp, gp.eps);
-      const unsigned wm = __ballot_sync(FULL, walks);
-      const int jw = wm ? min(32, __ffs(wm) - 1 + kTestWindow64) : 32;
+      unsigned wm = __ballot_sync(FULL, walks);
+      wm = __funnelshift_r(wm, wm, base);
+      const int jw = wm ? min(nready, __ffs(wm) - 1 + kTestWindow64) : nready;
       double distance = 1.0e10;
-      int ig = lane == 0 ? p.igrain : 0, is = lane == 0 ? p.isurf : -1;
+      int ig = off == 0 ? p.igrain : 0, is = off == 0 ? p.isurf : -1;
       bool stop = brk;
-      if (!brk && !in_ball && lane < jw) {
+      if (!brk && !in_ball && off < jw) {
         const bool hit = nearest64(g, G, gp.eps, sp, sd, sfp, p.which, in_gball, &distance, &ig, &is);
         stop = hit || !(sfp < 1.0e10);
       }
-      const unsigned sm = __ballot_sync(FULL, stop && lane < jw);
+      unsigned sm = __ballot_sync(FULL, stop && off < jw);
+      sm = __funnelshift_r(sm, sm, base);
       const int j = sm ? __ffs(sm) - 1 : jw;
+      const int jl = (base + j) & 31;      /* the lane of flight j ... */
+      const int jp = (base + j - 1) & 31;  /* ... and of the one before */
       flight += (uint32_t)j;
       if (j < 32) {
         /* the state at the start of flight j */
 #pragma unroll
         for (int d = 0; d < 3; ++d) {
-          p.pos[d] = __shfl_sync(FULL, sp[d], j);
-          p.dir[d] = __shfl_sync(FULL, sd[d], j);
+          p.pos[d] = __shfl_sync(FULL, sp[d], jl);
+          p.dir[d] = __shfl_sync(FULL, sd[d], jl);
         }
-        p.fp = __shfl_sync(FULL, sfp, j);
+        p.fp = __shfl_sync(FULL, sfp, jl);
       } else {
 #pragma unroll
         for (int d = 0; d < 3; ++d) {
           p.pos[d] = row[d * kRow64 + 31].y;
-          p.dir[d] = __shfl_sync(FULL, nd[d], 31);
+          p.dir[d] = __shfl_sync(FULL, nd[d], jp);
         }
-        p.fp = __shfl_sync(FULL, nf, 31);
+        p.fp = __shfl_sync(FULL, nf, jp);
       }
       __syncwarp();  /* the next round rewrites the rows */
       if (j > 0) { p.igrain = 0; p.isurf = -1; }
       if (sm) {
-        if (__shfl_sync(FULL, (int)brk, j)) {
-          capped = __shfl_sync(FULL, (int)inbox, j) != 0;
+        if (__shfl_sync(FULL, (int)brk, jl)) {
+          capped = __shfl_sync(FULL, (int)inbox, jl) != 0;
           end_side = 0;
           break;
         }
-        const double L = __shfl_sync(FULL, distance, j);
-        p.igrain = __shfl_sync(FULL, ig, j);
-        p.isurf = __shfl_sync(FULL, is, j);
+        const double L = __shfl_sync(FULL, distance, jl);
+        p.igrain = __shfl_sync(FULL, ig, jl);
+        p.isurf = __shfl_sync(FULL, is, jl);
         const int which = p.which;
         ++flight;
         end_side = surface_event64(g, lambda, omega, rng, flight, L, p);
         br2 = 0.0f;
         if (p.which != which) gr2 = 0.0f;
-      } else if (r.fast_steps > 0 && !__shfl_sync(FULL, (int)in_gball, j - 1)) {
+      } else if (r.fast_steps > 0 && !__shfl_sync(FULL, (int)in_gball, jp)) {
         /* a new ball where the walk left the grain ball */
         ball64(G, gp, p.which, p.pos, (float)lambda, &bx, &by, &bz, &br2, &gr2);
       }

@@ -329,25 +329,38 @@ __device__ __forceinline__ bool in_box64(const Geo64& g, const double* pos) {
          pos[1] <= g.box[1] + kSmall && pos[2] >= 0.0 - kSmall && pos[2] <= g.box[2] + kSmall;
 }
 
-/* Isotropic direction and free path of an intrinsic event from flight fl's
-   blocks 0 and 1 (what a used-up free path draws). */
-__device__ __forceinline__ void pp_draw64(const Draw& rng, double lambda, uint32_t fl, double* dir,
-                                          double* fp) {
-  double d0, d1, r0, r1;
-  rng.block(fl, 0, &d0, &d1);
-  rng.block(fl, 1, &r0, &r1);
-  const double ct = d0 * 2.0 - 1.0;
-  double sp, cp;
-  dsincos_2pi(d1, &sp, &cp);
-  const double st = sqrt(1.0 - ct * ct);
-  dir[0] = ct; dir[1] = st * cp; dir[2] = st * sp;
-  *fp = -lambda * dlog_pos(r0);
+/* What an event of a flight draws: blocks 0 and 1, and the sine and cosine of
+   its azimuth (an intrinsic event: from d1, a diffuse wall: from f0). */
+struct Drawn64 {
+  double d0, d1, f0, f1, sp, cp;
+};
+
+__device__ __forceinline__ void draw64(const Draw& rng, uint32_t fl, bool pp, Drawn64& w) {
+  rng.block(fl, 0, &w.d0, &w.d1);
+  rng.block(fl, 1, &w.f0, &w.f1);
+  dsincos_2pi(pp ? w.d1 : w.f0, &w.sp, &w.cp);
 }
 
-/* Flight fl ends in an intrinsic event after its whole free path. */
-__device__ __forceinline__ void pp_event64(const Draw& rng, double lambda, uint32_t fl, Ph64& p) {
+/* Isotropic direction and free path of an intrinsic event (a used-up free
+   path draws from block 1). */
+__device__ __forceinline__ void pp_dir64(const Drawn64& w, double lambda, double* dir, double* fp) {
+  const double ct = w.d0 * 2.0 - 1.0;
+  const double st = sqrt(1.0 - ct * ct);
+  dir[0] = ct; dir[1] = st * w.cp; dir[2] = st * w.sp;
+  *fp = -lambda * dlog_pos(w.f0);
+}
+
+__device__ __forceinline__ void pp_draw64(const Draw& rng, double lambda, uint32_t fl, double* dir,
+                                          double* fp) {
+  Drawn64 w;
+  draw64(rng, fl, true, w);
+  pp_dir64(w, lambda, dir, fp);
+}
+
+/* A flight ends in an intrinsic event after its whole free path. */
+__device__ __forceinline__ void pp_event64(const Drawn64& w, double lambda, Ph64& p) {
   for (int d = 0; d < 3; ++d) p.pos[d] = p.pos[d] + p.fp * p.dir[d];
-  pp_draw64(rng, lambda, fl, p.dir, &p.fp);
+  pp_dir64(w, lambda, p.dir, &p.fp);
   for (int d = 0; d < 3; ++d) p.pos[d] = p.pos[d] + 1.0e-7 * p.dir[d];
   p.igrain = 0;
   p.isurf = -1;
@@ -355,9 +368,11 @@ __device__ __forceinline__ void pp_event64(const Draw& rng, double lambda, uint3
 
 /* Flight fl ends after `distance` at surface p.isurf of grain p.igrain:
    bath, periodic face, reflection or transmission (src/RTMCphon.f90:1744-1792,
-   2225-2413).  Returns EndSide (0 lost, 1 x-, 2 x+), -1 while it goes on. */
+   2225-2413).  Returns EndSide (0 lost, 1 x-, 2 x+), -1 while it goes on.
+   DRAWN: the caller has drawn w, else it is drawn here, where it is needed. */
+template <bool DRAWN>
 __device__ int surface_event64(const Geo64& g, double lambda, double omega, const Draw& rng,
-                               uint32_t fl, double distance, Ph64& p) {
+                               uint32_t fl, double distance, const Drawn64& w, Ph64& p) {
   double* const pos = p.pos;
   double* const dir = p.dir;
   int end_side = -1, Jreflect = 1;
@@ -377,7 +392,8 @@ __device__ int surface_event64(const Geo64& g, double lambda, double omega, cons
     else pos[2] = pos[2] + sg;
   } else {
     const int k = g.grain_begin[p.igrain] + p.isurf;
-    rng.block(fl, 0, &d0, &d1);
+    if (DRAWN) { d0 = w.d0; d1 = w.d1; }
+    else rng.block(fl, 0, &d0, &d1);
     double od = 0.0;
     if (g.nmaterial != 1 && (g.kind_trans[k] == 2 || g.kind_trans[k] == 3)) {
       double x;
@@ -400,12 +416,15 @@ __device__ int surface_event64(const Geo64& g, double lambda, double omega, cons
       surface_normal(g, k, pos, N);
       if (dot3(N, dir) < 0.0) for (int d = 0; d < 3; ++d) N[d] = -1.0 * N[d];
       surface_rotation(g, k, pos, Rm);
-      double f0, f1;
-      rng.block(fl, 1, &f0, &f1);
+      double f0, f1, sp, cp;
+      if (DRAWN) {
+        f1 = w.f1; sp = w.sp; cp = w.cp;
+      } else {
+        rng.block(fl, 1, &f0, &f1);
+        dsincos_2pi(f0, &sp, &cp);
+      }
       const double sint = sqrt(d1);
       const double cost = sqrt(1.0 - sint * sint);
-      double sp, cp;
-      dsincos_2pi(f0, &sp, &cp);
       const double td[3] = {sint * cp, sint * sp, cost};
       double v[3];
       for (int i = 0; i < 3; ++i) v[i] = Rm[i] * td[0] + Rm[3 + i] * td[1] + Rm[6 + i] * td[2];
@@ -467,11 +486,14 @@ __device__ int trace(const Geo64& g, const Task64& t, const Draw& rng, int64_t m
       }
     }
     if (p.fp < distance) {
-      pp_event64(rng, t.lambda, (uint32_t)flight, p);
+      Drawn64 w;
+      draw64(rng, (uint32_t)flight, true, w);
+      pp_event64(w, t.lambda, p);
     } else {
       p.igrain = ig_min;
       p.isurf = is_min;
-      const int e = surface_event64(g, t.lambda, t.omega, rng, (uint32_t)flight, distance, p);
+      const int e = surface_event64<false>(g, t.lambda, t.omega, rng, (uint32_t)flight, distance,
+                                           Drawn64(), p);
       if (e == 0) break;
       if (e > 0) EndSide = e;
     }
@@ -843,7 +865,9 @@ __global__ void __launch_bounds__(256, 2) k_drain64(Geo64 g, GeoF32 gp, Run64 r)
         }
         if (fast) {
           ++flight;
-          pp_event64(rng, lambda, flight, p);
+          Drawn64 w;
+          draw64(rng, flight, true, w);
+          pp_event64(w, lambda, p);
         }
       }
     }
@@ -860,14 +884,18 @@ __global__ void __launch_bounds__(256, 2) k_drain64(Geo64 g, GeoF32 gp, Run64 r)
         const bool box_only = off2(q, bx, by, bz) < gr2 && off2(p.pos, bx, by, bz) < gr2;
         const bool hit = nearest64(g, G, gp.eps, p.pos, p.dir, p.fp, p.which, box_only, &distance,
                                    &p.igrain, &p.isurf);
-        if (!hit && p.fp < 1.0e10) {
-          pp_event64(rng, lambda, flight, p);
+        /* both kinds of event draw alike, before the lanes part */
+        const bool pp = !hit && p.fp < 1.0e10;
+        Drawn64 w;
+        draw64(rng, flight, pp, w);
+        if (pp) {
+          pp_event64(w, lambda, p);
           br2 = 0.0f;
           if (r.fast_steps > 0 && (float)lambda < r.fast_lambda_max)
             ball64(G, gp, p.which, p.pos, (float)lambda, &bx, &by, &bz, &br2, &gr2);
         } else {
           const int which = p.which;
-          end_side = surface_event64(g, lambda, r.task[task].omega, rng, flight, distance, p);
+          end_side = surface_event64<true>(g, lambda, r.task[task].omega, rng, flight, distance, w, p);
           br2 = 0.0f;
           if (p.which != which) gr2 = 0.0f;
         }
@@ -1055,7 +1083,7 @@ __global__ void __launch_bounds__(256, 2) k_tail64(Geo64 g, GeoF32 gp, Run64 r) 
         p.isurf = __shfl_sync(FULL, is, jl);
         const int which = p.which;
         ++flight;
-        end_side = surface_event64(g, lambda, omega, rng, flight, L, p);
+        end_side = surface_event64<false>(g, lambda, omega, rng, flight, L, Drawn64(), p);
         br2 = 0.0f;
         if (p.which != which) gr2 = 0.0f;
       } else if (r.fast_steps > 0 && !__shfl_sync(FULL, (int)in_gball, jp)) {

@@ -736,8 +736,8 @@ int run_transport(ptg_handle* h, const Transport& T) {
       const int key = -1 - block;
       if (h->occ_key != key) {
         h->occ_key = 0;
-        CU(ptg::drain64_occupancy(block, &h->occ_bps));
-        CU(ptg::tail64_occupancy(block, &h->occ_tail));
+        CU(ptg::drain64_occupancy(block, &h->occ_bps, h->g32.has_ext));
+        CU(ptg::tail64_occupancy(block, &h->occ_tail, h->g32.has_ext));
         h->occ_key = key;
       }
       int bps = h->occ_bps;

@@ -272,8 +272,8 @@ cudaError_t launch_tail_order(const float4* tail, int units, int tail_cap, const
                               int32_t* order, int32_t* hist, cudaStream_t st);
 /* The FP64 pair: the same queue and list, FP64 flights; the blob of g32 gives
    the bounds for balls and BVH walks. */
-cudaError_t drain64_occupancy(int block, int* blocks_per_sm);
-cudaError_t tail64_occupancy(int block, int* blocks_per_sm);
+cudaError_t drain64_occupancy(int block, int* blocks_per_sm, int ext);
+cudaError_t tail64_occupancy(int block, int* blocks_per_sm, int ext);
 cudaError_t launch_drain64(const Geo64& g, const GeoF32& g32, const Run64& r, int grid, int block,
                            cudaStream_t st);
 cudaError_t launch_tail64(const Geo64& g, const GeoF32& g32, const Run64& r, int grid, int block,

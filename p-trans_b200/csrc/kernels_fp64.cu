@@ -141,8 +141,9 @@ __device__ void capped_normal(const Geo64& g, int k, const double* R, double* N)
 
 /* calcSurfaceDistance dispatch, src/RTMCphon.f90:2883-3088.  CULL: a polygon
    whose plane is crossed beyond lim is left before the division and the edge
-   test (the product's 1e-6 is far above the rounding of either side). */
-template <bool CULL>
+   test (the product's 1e-6 is far above the rounding of either side).  EXT: as
+   in the FP32 kernels, 0 without BVH and capped cylinders. */
+template <bool CULL, int EXT>
 __device__ bool surface_distance(const Geo64& g, int k, const double* R0, const double* D,
                                  double lim, double* L) {
   const int sh = g.shape[k];
@@ -163,7 +164,7 @@ __device__ bool surface_distance(const Geo64& g, int k, const double* R0, const 
     *L = Lh;
     return true;
   }
-  if (sh == 4) return capped_distance(g, k, R0, D, L);
+  if (EXT && sh == 4) return capped_distance(g, k, R0, D, L);
   const double* C = g.center + 3 * k;
   const double r = g.radius[k];
   const double r2 = r * r;
@@ -208,13 +209,14 @@ __device__ bool surface_distance(const Geo64& g, int k, const double* R0, const 
 }
 
 /* calcSurfaceNormal*, src/RTMCphon.f90:3119-3179 */
+template <int EXT>
 __device__ void surface_normal(const Geo64& g, int k, const double* R, double* N) {
   const int sh = g.shape[k];
   if (sh == 1) {
     N[0] = g.normal[3 * k]; N[1] = g.normal[3 * k + 1]; N[2] = g.normal[3 * k + 2];
     return;
   }
-  if (sh == 4) {
+  if (EXT && sh == 4) {
     capped_normal(g, k, R, N);
     return;
   }
@@ -233,6 +235,7 @@ __device__ void surface_normal(const Geo64& g, int k, const double* R, double* N
 }
 
 /* calcSurfaceRotation*, src/RTMCphon.f90:3181-3301 (column-major) */
+template <int EXT>
 __device__ void surface_rotation(const Geo64& g, int k, const double* R, double* Rm) {
   const int sh = g.shape[k];
   if (sh == 1) {
@@ -241,7 +244,7 @@ __device__ void surface_rotation(const Geo64& g, int k, const double* R, double*
   }
   const double* C = g.center + 3 * k;
   double n[3];
-  if (sh == 4) {
+  if (EXT && sh == 4) {
     capped_normal(g, k, R, n);
   } else if (sh == 2) {
     double Rcs[3] = {R[0] - C[0], R[1] - C[1], R[2] - C[2]};
@@ -370,7 +373,7 @@ __device__ __forceinline__ void pp_event64(const Drawn64& w, double lambda, Ph64
    bath, periodic face, reflection or transmission (src/RTMCphon.f90:1744-1792,
    2225-2413).  Returns EndSide (0 lost, 1 x-, 2 x+), -1 while it goes on.
    DRAWN: the caller has drawn w, else it is drawn here, where it is needed. */
-template <bool DRAWN>
+template <bool DRAWN, int EXT>
 __device__ int surface_event64(const Geo64& g, double lambda, double omega, const Draw& rng,
                                uint32_t fl, double distance, const Drawn64& w, Ph64& p) {
   double* const pos = p.pos;
@@ -405,7 +408,7 @@ __device__ int surface_event64(const Geo64& g, double lambda, double omega, cons
         Jreflect = 0;
       } else {
         double N[3];
-        surface_normal(g, k, pos, N);
+        surface_normal<EXT>(g, k, pos, N);
         if (dot3(N, dir) < 0) for (int d = 0; d < 3; ++d) N[d] = -1.0 * N[d];
         const double dn = dot3(N, dir);
         for (int d = 0; d < 3; ++d) dir[d] = dir[d] - 2.0 * N[d] * dn;
@@ -413,9 +416,9 @@ __device__ int surface_event64(const Geo64& g, double lambda, double omega, cons
       }
     } else {
       double N[3], Rm[9];
-      surface_normal(g, k, pos, N);
+      surface_normal<EXT>(g, k, pos, N);
       if (dot3(N, dir) < 0.0) for (int d = 0; d < 3; ++d) N[d] = -1.0 * N[d];
-      surface_rotation(g, k, pos, Rm);
+      surface_rotation<EXT>(g, k, pos, Rm);
       double f0, f1, sp, cp;
       if (DRAWN) {
         f1 = w.f1; sp = w.sp; cp = w.cp;
@@ -478,7 +481,7 @@ __device__ int trace(const Geo64& g, const Task64& t, const Draw& rng, int64_t m
       for (int k = kb; k < ke; ++k) {
         if (!g.internal[k]) continue;
         double L;
-        if (surface_distance<false>(g, k, p.pos, p.dir, 0.0, &L) && distance > L) {
+        if (surface_distance<false, 2>(g, k, p.pos, p.dir, 0.0, &L) && distance > L) {
           distance = L;
           ig_min = ig;
           is_min = k - kb;
@@ -492,7 +495,7 @@ __device__ int trace(const Geo64& g, const Task64& t, const Draw& rng, int64_t m
     } else {
       p.igrain = ig_min;
       p.isurf = is_min;
-      const int e = surface_event64<false>(g, t.lambda, t.omega, rng, (uint32_t)flight, distance,
+      const int e = surface_event64<false, 2>(g, t.lambda, t.omega, rng, (uint32_t)flight, distance,
                                            Drawn64(), p);
       if (e == 0) break;
       if (e > 0) EndSide = e;
@@ -591,6 +594,7 @@ __global__ void __launch_bounds__(128) k_plain_fp64(Geo64 g, Run64 r) {
        and positions rounded by 2^-24 of the box, so no node that holds the
        hit is skipped.
    Returns whether there is a hit; box_only leaves the grain's surfaces out. */
+template <int EXT>
 __device__ bool nearest64(const Geo64& g, const Geo<false>& G, float eps, const double* pos,
                           const double* dir, double fp, int which, bool box_only, double* dist,
                           int* igrain, int* isurf) {
@@ -620,24 +624,24 @@ __device__ bool nearest64(const Geo64& g, const Geo<false>& G, float eps, const 
   } else {
     for (int k = 0; k < g.grain_begin[1]; ++k) {
       double L;
-      if (g.internal[k] && surface_distance<true>(g, k, pos, dir, best, &L) && best > L) {
+      if (g.internal[k] && surface_distance<true, EXT>(g, k, pos, dir, best, &L) && best > L) {
         best = L; *igrain = 0; *isurf = k; hit = true;
       }
     }
   }
   if (which > 0 && !box_only) {
     const int kb0 = g.grain_begin[which];
-    const int root = G.bvh_root(which);
+    const int root = EXT ? G.bvh_root(which) : -1;
     if (root < 0) {
       const int kb = G.cand_begin(which), ke = G.cand_begin(which + 1);
       for (int i = kb; i < ke; ++i) {
         const int k = G.cand(i);
         double L;
-        if (surface_distance<true>(g, k, pos, dir, best, &L) && best > L) {
+        if (surface_distance<true, EXT>(g, k, pos, dir, best, &L) && best > L) {
           best = L; *igrain = which; *isurf = k - kb0; hit = true;
         }
       }
-    } else if (!behind_planes(G, which, (float)pos[0], (float)pos[1], (float)pos[2], (float)dir[0],
+    } else if (EXT && !behind_planes(G, which, (float)pos[0], (float)pos[1], (float)pos[2], (float)dir[0],
                               (float)dir[1], (float)dir[2], (float)fp, eps)) {
       const float px = (float)pos[0], py = (float)pos[1], pz = (float)pos[2];
       const float ix = inv_dir((float)dir[0]), iy = inv_dir((float)dir[1]),
@@ -656,7 +660,7 @@ __device__ bool nearest64(const Geo64& g, const Geo<false>& G, float eps, const 
           for (int i = a; i < a + cnt; ++i) {
             const int k = G.cand(i);
             double L;
-            if (surface_distance<true>(g, k, pos, dir, best, &L) &&
+            if (surface_distance<true, EXT>(g, k, pos, dir, best, &L) &&
                 (best > L || (mine && best == L && k - kb0 < *isurf))) {
               best = L; *igrain = which; *isurf = k - kb0; hit = true; mine = true;
             }
@@ -699,13 +703,14 @@ __device__ bool nearest64(const Geo64& g, const Geo<false>& G, float eps, const 
 /* Safe ball and grain ball about pos from the FP32 bounds (kernels_fp32.cu),
    less the rounding of the centre, the 1e-7 nudges and the few 1e-8 of the
    box by which an FP64 root can be off: radius squared, 0 for none. */
+template <int EXT>
 __device__ __forceinline__ void ball64(const Geo<false>& G, const GeoF32& gp, int which,
                                        const double* pos, float lam, float* bx, float* by,
                                        float* bz, float* br2, float* gr2) {
   *bx = (float)pos[0]; *by = (float)pos[1]; *bz = (float)pos[2];
   float dg, dg2;
   int near;
-  const float d = safety<2>(G, which, *bx, *by, *bz, gp.box[0], gp.box[1], gp.box[2], gp.eps,
+  const float d = safety<EXT>(G, which, *bx, *by, *bz, gp.box[0], gp.box[1], gp.box[2], gp.eps,
                                kBallCap64 * lam, dg, dg2, near) - 1.0e-6f;
   dg -= 1.0e-6f;
   *br2 = d > 0.0f ? d * d : 0.0f;
@@ -751,6 +756,7 @@ __device__ __forceinline__ void unpack2(float4 v, double* a, double* b) {
    the warp's chunk; flights that stay in the safe ball are taken without a
    scan; once the queue is dry the live phonons go to the tail list
    (grace_passes). */
+template <int EXT>
 __global__ void __launch_bounds__(256, 2) k_drain64(Geo64 g, GeoF32 gp, Run64 r) {
   Geo<false> G;
   G.base = gp.blob;
@@ -882,7 +888,7 @@ __global__ void __launch_bounds__(256, 2) k_drain64(Geo64 g, GeoF32 gp, Run64 r)
         double q[3], distance;
         for (int d = 0; d < 3; ++d) q[d] = p.pos[d] + p.fp * p.dir[d];
         const bool box_only = off2(q, bx, by, bz) < gr2 && off2(p.pos, bx, by, bz) < gr2;
-        const bool hit = nearest64(g, G, gp.eps, p.pos, p.dir, p.fp, p.which, box_only, &distance,
+        const bool hit = nearest64<EXT>(g, G, gp.eps, p.pos, p.dir, p.fp, p.which, box_only, &distance,
                                    &p.igrain, &p.isurf);
         /* both kinds of event draw alike, before the lanes part */
         const bool pp = !hit && p.fp < 1.0e10;
@@ -892,10 +898,10 @@ __global__ void __launch_bounds__(256, 2) k_drain64(Geo64 g, GeoF32 gp, Run64 r)
           pp_event64(w, lambda, p);
           br2 = 0.0f;
           if (r.fast_steps > 0 && (float)lambda < r.fast_lambda_max)
-            ball64(G, gp, p.which, p.pos, (float)lambda, &bx, &by, &bz, &br2, &gr2);
+            ball64<EXT>(G, gp, p.which, p.pos, (float)lambda, &bx, &by, &bz, &br2, &gr2);
         } else {
           const int which = p.which;
-          end_side = surface_event64<true>(g, lambda, r.task[task].omega, rng, flight, distance, w, p);
+          end_side = surface_event64<true, EXT>(g, lambda, r.task[task].omega, rng, flight, distance, w, p);
           br2 = 0.0f;
           if (p.which != which) gr2 = 0.0f;
         }
@@ -941,6 +947,7 @@ constexpr int kRow64 = 33;
    after the other: lane c < 3 adds coordinate c's, two additions a flight,
    through shared memory.  The first flight that meets a surface, leaves the
    box or reaches the cap ends the round, and every lane takes its event. */
+template <int EXT>
 __global__ void __launch_bounds__(256, 2) k_tail64(Geo64 g, GeoF32 gp, Run64 r) {
   __shared__ double2 rows[8][3 * kRow64];
   double2* const row = rows[threadIdx.x >> 5];
@@ -1035,7 +1042,7 @@ __global__ void __launch_bounds__(256, 2) k_tail64(Geo64 g, GeoF32 gp, Run64 r) 
       const bool inbox = in_box64(g, sp);
       const bool brk = !inbox || (int64_t)flight + off >= r.max_flights;
       const bool walks =
-          !in_ball && !in_gball && p.which > 0 && G.bvh_root(p.which) >= 0 &&
+          EXT && !in_ball && !in_gball && p.which > 0 && G.bvh_root(p.which) >= 0 &&
           !behind_planes(G, p.which, (float)sp[0], (float)sp[1], (float)sp[2], (float)sd[0],
                          (float)sd[1], (float)sd[2], (float)sfp, gp.eps);
       unsigned wm = __ballot_sync(FULL, walks);
@@ -1045,7 +1052,7 @@ __global__ void __launch_bounds__(256, 2) k_tail64(Geo64 g, GeoF32 gp, Run64 r) 
       int ig = off == 0 ? p.igrain : 0, is = off == 0 ? p.isurf : -1;
       bool stop = brk;
       if (!brk && !in_ball && off < jw) {
-        const bool hit = nearest64(g, G, gp.eps, sp, sd, sfp, p.which, in_gball, &distance, &ig, &is);
+        const bool hit = nearest64<EXT>(g, G, gp.eps, sp, sd, sfp, p.which, in_gball, &distance, &ig, &is);
         stop = hit || !(sfp < 1.0e10);
       }
       unsigned sm = __ballot_sync(FULL, stop && off < jw);
@@ -1083,12 +1090,12 @@ __global__ void __launch_bounds__(256, 2) k_tail64(Geo64 g, GeoF32 gp, Run64 r) 
         p.isurf = __shfl_sync(FULL, is, jl);
         const int which = p.which;
         ++flight;
-        end_side = surface_event64<false>(g, lambda, omega, rng, flight, L, Drawn64(), p);
+        end_side = surface_event64<false, EXT>(g, lambda, omega, rng, flight, L, Drawn64(), p);
         br2 = 0.0f;
         if (p.which != which) gr2 = 0.0f;
       } else if (r.fast_steps > 0 && !__shfl_sync(FULL, (int)in_gball, jp)) {
         /* a new ball where the walk left the grain ball */
-        ball64(G, gp, p.which, p.pos, (float)lambda, &bx, &by, &bz, &br2, &gr2);
+        ball64<EXT>(G, gp, p.which, p.pos, (float)lambda, &bx, &by, &bz, &br2, &gr2);
       }
     }
     my_flights += flight;
@@ -1121,25 +1128,31 @@ cudaError_t launch_plain_fp64(const Geo64& g, const Run64& r, cudaStream_t st, i
   return cudaGetLastError();
 }
 
-cudaError_t drain64_occupancy(int block, int* bps) {
-  return cudaOccupancyMaxActiveBlocksPerMultiprocessor(bps, k_drain64, block, 0);
+/* Kernels without BVH and capped cylinders, or with both: a round's or pass's
+   instructions are fetched again and again, and the shorter code stalls less
+   for them (gray wire, 3e4 phonons: 2.25 -> 2.09 ms; porous film 3.19 -> 2.89,
+   wire 300 x 60 nm 9.43 -> 8.97). */
+cudaError_t drain64_occupancy(int block, int* bps, int ext) {
+  return cudaOccupancyMaxActiveBlocksPerMultiprocessor(bps, ext ? k_drain64<2> : k_drain64<0>, block, 0);
 }
 
-cudaError_t tail64_occupancy(int block, int* bps) {
-  return cudaOccupancyMaxActiveBlocksPerMultiprocessor(bps, k_tail64, block, 0);
+cudaError_t tail64_occupancy(int block, int* bps, int ext) {
+  return cudaOccupancyMaxActiveBlocksPerMultiprocessor(bps, ext ? k_tail64<2> : k_tail64<0>, block, 0);
 }
 
 cudaError_t launch_drain64(const Geo64& g, const GeoF32& gp, const Run64& r, int grid, int block,
                            cudaStream_t st) {
   if (block > 256 || block % 32) return cudaErrorInvalidConfiguration;
-  k_drain64<<<grid, block, 0, st>>>(g, gp, r);
+  if (gp.has_ext) k_drain64<2><<<grid, block, 0, st>>>(g, gp, r);
+  else k_drain64<0><<<grid, block, 0, st>>>(g, gp, r);
   return cudaGetLastError();
 }
 
 cudaError_t launch_tail64(const Geo64& g, const GeoF32& gp, const Run64& r, int grid, int block,
                           cudaStream_t st) {
   if (block > 256 || block % 32) return cudaErrorInvalidConfiguration;
-  k_tail64<<<grid, block, 0, st>>>(g, gp, r);
+  if (gp.has_ext) k_tail64<2><<<grid, block, 0, st>>>(g, gp, r);
+  else k_tail64<0><<<grid, block, 0, st>>>(g, gp, r);
   return cudaGetLastError();
 }
 

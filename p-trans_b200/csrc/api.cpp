@@ -102,7 +102,7 @@ struct ptg_handle {
   /* what a call clears and reads back (CallLayout), its tables (tasks, then
      the queue order) and their pinned staging.  The staging is free again once
      the stream has been waited for; busy: it has not since the last use */
-  DevBuf call, in;
+  DevBuf call, in, chunk;
   PinBuf pin_in, pin_out, pin_const;
   bool busy = false;
   /* launch shape of the last mode and block size (0: none yet) */
@@ -120,7 +120,7 @@ struct ptg_handle {
   int tail_cap = 0;          /* its tail-list capacity (0: no tail phase)       */
   ~ptg_handle() {
     for (DevBuf* b : owned) { b->release(); delete b; }
-    DevBuf* all[] = {&blob, &call, &in, &red_in, &red_tmp, &red_out, &red_trans, &adj_list, &adj_w,
+    DevBuf* all[] = {&blob, &call, &in, &chunk, &red_in, &red_tmp, &red_out, &red_trans, &adj_list, &adj_w,
                      &adj_acc, &tr_off, &tr_npos, &tr_end, &tr_pos, &tail};
     for (DevBuf* b : all) b->release();
     if (stream) cudaStreamSynchronize(stream);
@@ -828,6 +828,11 @@ int run_transport(ptg_handle* h, const Transport& T) {
       if (T.mode == ptg::MODE_FORWARD)
         r.grace_steps = ptg::grace_passes(norder * T.np_local, (int64_t)tgrid * (block / 32));
     }
+    if (h->g32.has_ext == ptg::kChunkTableExt && nchunk > 0) {
+      CU(h->chunk.ensure(sizeof(int4) * nchunk));
+      r.chunk = h->chunk.as<const int4>();
+      CU(ptg::launch_expand_chunks(chunks, (int)nchunk, h->chunk.as<int4>(), h->stream));
+    }
     const bool work = (T.mode == ptg::MODE_ADJOINT || T.mode == ptg::MODE_TRACE) ? T.alist_n > 0
                                                                                    : r.nchunk > 0;
     if (work) {
@@ -842,7 +847,7 @@ int run_transport(ptg_handle* h, const Transport& T) {
     CU(cudaEventRecord(h->ev[1], h->stream));
     h->last.grid = grid;
     h->last.block = block;
-    h->last.launches = work ? (tail ? 3 : 1) : 0;
+    h->last.launches = work ? (tail ? 3 : 1) + (r.chunk ? 1 : 0) : 0;
     h->fp32_split = work;
     h->tail_cap = tail ? r.tail_cap : 0;
   }

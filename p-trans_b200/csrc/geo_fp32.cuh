@@ -283,7 +283,7 @@ __device__ __forceinline__ int order_bucket(float x, float x_len, float lam) {
 __device__ __forceinline__ int3 queue_chunk(const ChunkQueue& q, int c) {
   const int k = c / q.per_task;
   const int j = (c - k * q.per_task) * q.size;
-  return make_int3(__ldg(q.order + k), j, min(q.size, q.np_local - j));
+  return make_int3(q.order ? __ldg(q.order + k) : k, j, min(q.size, q.np_local - j));
 }
 
 __device__ __forceinline__ unsigned lanemask_lt() {

@@ -47,10 +47,14 @@ struct Task64 {
   double lambda, cth, sth, omega;
 };
 
+/* GeoF32.has_ext of the FP32 kernels that read a chunk table. */
+constexpr int kChunkTableExt = 1;
+
 /* Work queue of a run: chunk c is particles [j, j + size), j = (c % per_task)
    size, of task order[c / per_task], clipped to np_local. */
 struct ChunkQueue {
   const int* order;          /* tasks, longest expected trajectories first      */
+                             /* (NULL: as they are numbered)                    */
   int32_t per_task, size, np_local;
 };
 
@@ -149,8 +153,10 @@ struct GeoEntry {
 /* Per task (FP32): lambda (inf = ballistic, <= 0 skipped), cos, sin, omega/max_omega */
 struct RunF32 {
   const float4* task;
-  const int4* chunk;          /* (task, first local particle, count, 0) in LPT order */
-  ChunkQueue chunks;          /* ... or, chunk NULL, what they follow from          */
+  ChunkQueue chunks;          /* the chunks, longest expected trajectories first   */
+  const int4* chunk;          /* their table (task, first local particle, count, 0),
+                                 read instead by batches and behind a BVH or with
+                                 capped cylinders (kChunkTableExt) */
   int32_t nchunk;
   int64_t np;
   int32_t rank, nranks;
@@ -262,6 +268,8 @@ cudaError_t launch_persistent_fp32(const GeoF32& g, const RunF32& r, int grid, i
                                    size_t smem, cudaStream_t st, int mode = MODE_FORWARD);
 /* The tail phase after it (forward, list and adjoint modes): the phonons
    the drain phase left in r.tail, one per warp. */
+/* Fills the chunk table of the queue's nchunk chunks. */
+cudaError_t launch_expand_chunks(const ChunkQueue& q, int nchunk, int4* chunks, cudaStream_t st);
 /* Orders the tail list for the tail phase, longest expected remaining walk
    first, into order (tail_cap ints) from the buckets' histogram that the drain
    phase fills as it hands phonons over (hist: kTailOrderExtra ints with the

@@ -1152,7 +1152,12 @@ __global__ void __launch_bounds__(kBlock,
               if (lane == 0) atomicMax(r.stats + 6, ~globaltimer());
               break;
             }
-            if (r.chunk) {
+            /* the table where it is there anyway (a batch) or where the
+               arithmetic costs the kernel registers: with it behind a BVH
+               the spills of the drain grow from 104 to 120 bytes read, and
+               64 spheres with 16 capped cylinders, 2e7 phonons, take 107.0
+               ms of drain against 104.1 */
+            if (BATCH || EXT == kChunkTableExt) {
               const int4 q = r.chunk[c];
               ch_task = q.x; ch_next = q.y; ch_left = q.z;
             } else {
@@ -2129,6 +2134,22 @@ __global__ void k_order_scatter(const float4* __restrict__ tail, int units, int 
   order[h[b] + atomicAdd(&cursor[b], 1)] = slot;
 }
 }  // namespace
+
+/* Chunk table of a run whose kernels read one (kChunkTableExt). */
+__global__ void k_expand_chunks(const ChunkQueue q, int nchunk, int4* __restrict__ chunks) {
+  for (long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x; c < nchunk;
+       c += (long long)gridDim.x * blockDim.x) {
+    const int3 v = queue_chunk(q, (int)c);
+    chunks[c] = make_int4(v.x, v.y, v.z, 0);
+  }
+}
+
+cudaError_t launch_expand_chunks(const ChunkQueue& q, int nchunk, int4* chunks, cudaStream_t st) {
+  if (nchunk <= 0) return cudaSuccess;
+  const int blocks = (nchunk + 255) / 256;
+  k_expand_chunks<<<blocks < 4096 ? blocks : 4096, 256, 0, st>>>(q, nchunk, chunks);
+  return cudaGetLastError();
+}
 
 cudaError_t launch_tail_order(const float4* tail, int units, int tail_cap, const int* queue,
                               int32_t* order, int32_t* hist, cudaStream_t st) {

@@ -155,7 +155,11 @@ extern "C" int ptg_transmission_noalloc(ptg_handle* h, double mfp_nm, int32_t na
   ptg::RunF32 r;
   memset(&r, 0, sizeof(r));
   r.task = reinterpret_cast<const float4*>(base + kOffTasks);
+  /* one mean free path: the tasks run as they are numbered */
   r.chunk = reinterpret_cast<const int4*>(base + kOffChunks);
+  r.chunks.per_task = (int32_t)std::max<int64_t>(per_task, 1);
+  r.chunks.size = (int32_t)std::min(chunk, std::max<int64_t>(np_local, 1));
+  r.chunks.np_local = (int32_t)np_local;
   r.nchunk = (int32_t)(ntask * per_task);
   r.np = np;
   r.rank = rank;

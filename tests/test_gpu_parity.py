@@ -173,6 +173,37 @@ def test_ballistic_specular_duct_transmits_everything(prec):
     assert k["lost"] == 0
 
 
+@pytest.mark.parametrize("np_,nranks,chunk", [(1, 1, 0), (1, 3, 0), (63, 1, 0), (65, 2, 0), (130, 1, 7),
+                                              (130, 4, 1000)])
+@pytest.mark.parametrize("capped", [False, True])
+def test_queue_chunks_cover_every_particle_once(capped, np_, nranks, chunk):
+    """Chunks that the kernel computes (spheres) or reads from a table (capped
+    cylinders): tasks of one particle, ranks without one, last chunks of one
+    particle, chunks longer than a task.  Every particle is flown once, and
+    the counts are those of single-particle chunks on one rank, in both
+    precisions and without allocation."""
+    model = synth.spheres_cylinders_box(n_spheres=3, n_cylinders=3 if capped else 0, l=300.0, seed=3,
+                                        r_sphere=(15.0, 35.0), r_cylinder=20.0, length=(50.0, 150.0),
+                                        trans=0.3, p_wall=0.2)
+    spec = synth.spectrum(5, seed=2)
+    gb = A.GeomBuf(model)
+    for prec in (A.PREC_FP32, A.PREC_FP64):
+        with A.Handle(gb.view, spec, chunk=1) as h:
+            want, _ = h.transmission(40.0, 4, np_, seed=8, precision=prec)
+        with A.Handle(gb.view, spec, chunk=chunk) as h:
+            calls = [lambda r: h.transmission(40.0, 4, np_, rank=r, nranks=nranks, seed=8, precision=prec)[0]]
+            if prec == A.PREC_FP32:
+                calls.append(lambda r: h.transmission_noalloc(40.0, 4, np_, rank=r, nranks=nranks, seed=8))
+            for call in calls:
+                total, flown = np.zeros_like(want), 0
+                for r in range(nranks):
+                    got = call(r)
+                    flown += h.stats()["samples"]
+                    total += np.rint(got * np_)
+                assert flown == 5 * 3 * np_
+                np.testing.assert_array_equal(total, np.rint(want * np_))
+
+
 @pytest.mark.parametrize("prec", [A.PREC_FP32, A.PREC_FP64])
 def test_lost_phonons_with_flight_cap(orc, prec):
     m, spec, gb = setup("nanowire_diffuse", nmode=3)

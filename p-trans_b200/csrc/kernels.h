@@ -245,7 +245,7 @@ inline int default_fast_steps(const GeoF32& g) {
    3500 for 32 of them.  So they stay where the tail phase would get many per
    warp (120 000 phonons, MFP 150 nm in a 200 nm cube: 432 -> 209 us; 3.6e6
    ballistic ones among spheres: 1107 -> 710 us) and go at once where it gets
-   few (2400 phonons in a porous film, MFP 100 nm: 229 us against 248 with 16
+   few (3200 phonons in a porous film, MFP 100 nm: 229 us against 248 with 16
    passes, 260 with 32).  The two are equal at 4 to 8 phonons per warp, and
    16 and 32 passes at about 40; behind a BVH too (64 spheres and 16 capped
    cylinders, 2e5 phonons, MFP 150 nm: 6.0 -> 3.1 ms).  The adjoint's two

@@ -241,3 +241,29 @@ def test_adjoint_per_surface_matches_central_differences(orc):
     mo, so = ofd.mean(0), ofd.std(0, ddof=1) / 2.0
     zo = (ma - mo) / np.hypot(sa, so)
     assert np.all(np.abs(zo[resolved]) < 3.0), (zo, table)
+
+
+# dk_dscale by (structure, seed), as the replay sums it up: a sample's path
+# length in FP32, a round's flights by warp shuffles, the sum taken over at
+# every surface.  The score is a small difference of two large numbers, so
+# another grouping of the same flights moves it by 5e-6 to 2e-5 of itself.
+_DSCALE = {("wire", 4): 1.3476224, ("wire", 6): -1.8050285, ("film", 1): -7.0445188, ("film", 2): -2.6002088,
+           ("film", 3): 2.5241594, ("film", 6): -5.9722795}
+
+
+@pytest.mark.parametrize("name", ["wire", "film"])
+def test_scale_derivative_keeps_its_summation(name):
+    """The median of five runs lies within 3e-6 of the recorded value: runs of
+    one build differ by up to 2e-6 (where the drain phase hands a phonon over
+    depends on timing)."""
+    model = {"wire": synth.nanowire(length=300.0, width=80.0, height=80.0, p_side=0.3),
+             "film": synth.film_with_holes(nholes=2, seed=4, p_hole=0.5, p_z=0.3)}[name]
+    spec = synth.spectrum(24, seed=5, mfp_lo=4e-9, mfp_hi=1e-6)
+    gb = A.GeomBuf(model)
+    with A.Handle(gb.view, spec) as h:
+        for (s, seed), want in _DSCALE.items():
+            if s != name:
+                continue
+            run = A.make_run(kind_mfp=A.MFP_PER_MODE, nangle=7, np_=40, seed=seed)
+            got = np.median([h.adjoint(run)["dk_dscale"] for _ in range(5)])
+            assert abs(got - want) <= 3e-6 * abs(want), (seed, got)

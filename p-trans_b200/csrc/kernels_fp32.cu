@@ -1406,7 +1406,10 @@ __global__ void __launch_bounds__(kBlock,
           float cbx = s2.x, cby = s2.y, cbz = s2.z, cbr2 = s2.w, cgr2 = s4.w;
           float cg2r2 = s5.x;
           int cnear = __float_as_int(s5.y);
-          float clen = 0.0f;
+          /* path length of the replay's flights: a single structure's adds up
+             by rounds, a batch's goes on flight by flight from the drain's
+             sum, so that it does not depend on where a phonon was handed over */
+          float clen = BATCH && MODE == MODE_ADJOINT ? __shfl_sync(FULL, adj_len, 0) : 0.0f;
           unsigned cnpp = 0, ctaken = 0, crounds = 0;
           int stop = 0;  /* 0 round limit, 1 surface hit, 2 lost or capped */
           uint4 sR = make_uint4(0u, 0u, 0u, 0u);
@@ -1553,9 +1556,14 @@ __global__ void __launch_bounds__(kBlock,
                 __ballot_sync(FULL, lane < jw && (brk || (!in_ball && !(sfp < tb))));
             const int j = sm ? __ffs(sm) - 1 : jw;
             if (MODE == MODE_ADJOINT) {
-              float l = lane < j ? sfp : 0.0f;
-              for (int o = 16; o > 0; o >>= 1) l += __shfl_xor_sync(FULL, l, o);
-              clen += l;
+              if (BATCH) {
+                for (int k = 0; k < j; ++k) clen += frow[k];
+                __syncwarp();
+              } else {
+                float l = lane < j ? sfp : 0.0f;
+                for (int o = 16; o > 0; o >>= 1) l += __shfl_xor_sync(FULL, l, o);
+                clen += l;
+              }
               cnpp += (unsigned)j;
             }
             ctaken += (unsigned)j;
@@ -1678,7 +1686,7 @@ __global__ void __launch_bounds__(kBlock,
             park[4] = make_float4(s4.x, s4.y, __uint_as_float(cfl), cgr2);
             park[5] = make_float4(cg2r2, __int_as_float(cnear), 0.0f, 0.0f);
             if (MODE == MODE_ADJOINT) {
-              adj_len += clen;
+              adj_len = BATCH ? clen : adj_len + clen;
               adj_npp += cnpp;
             }
             coop = true;

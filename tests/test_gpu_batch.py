@@ -114,3 +114,33 @@ def test_batched_tail_phase_takes_the_same_trajectories(kind, cap):
     np.testing.assert_array_equal(got[1][0], got[0][0])
     assert got[1][1:] == got[0][1:]
     assert got[0][5] == 0
+
+
+def _unlike():
+    """A porous film, a convex mesh with a BVH and facet planes, capped
+    cylinders and a cube lattice with a BVH alone."""
+    return [synth.film_with_holes(nholes=2, seed=4, p_hole=0.5, p_z=0.3),
+            synth.voronoi_box(4, box=(300.0, 250.0, 250.0), seed=5, trans=0.5, p_wall=0.3, tri_levels=2),
+            synth.spheres_cylinders_box(n_spheres=4, n_cylinders=5, l=300.0, seed=3, r_sphere=(15.0, 35.0),
+                                        r_cylinder=20.0, length=(50.0, 150.0), trans=0.3, p_wall=0.2),
+            synth.cube_lattice(n=4, l=300.0, fill=0.4, trans=0.3, spec=0.2, p_wall=0.3)]
+
+
+def test_batched_scale_derivative_does_not_depend_on_the_tail_phase():
+    """A replayed sample's path length is one running sum, whichever phase flies
+    it: the derivatives with and without a tail phase (tune_flags bit 1) differ
+    by the order of the FP64 sums over samples alone.  Each score is below 1e3
+    standard errors, so 1e-10 of the error leaves room for 1e3 roundings."""
+    spec = synth.spectrum(12, seed=5, mfp_lo=1e-9, mfp_hi=1e-7)
+    bufs = [A.GeomBuf(m) for m in _unlike()]
+    nps, n = [37, 90, 44, 61], len(bufs)
+    run = A.make_run(kind_mfp=A.MFP_PER_MODE, nangle=5, np_=1)
+    got = []
+    for flags in (2, 0):
+        with A.Batch([b.view for b in bufs], nps, [9 + i for i in range(n)], [0] * n, spec, run,
+                     tune_flags=flags) as bt:
+            got.append(bt.adjoint())
+    se = got[0]["dk_dscale_stderr"]
+    assert np.all(se > 0.0)
+    assert np.all(np.abs(got[1]["dk_dscale"] - got[0]["dk_dscale"]) <= 1e-10 * se)
+    np.testing.assert_allclose(got[1]["dk_dscale_stderr"], se, rtol=1e-10)

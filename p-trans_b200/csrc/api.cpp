@@ -95,6 +95,7 @@ struct ptg_handle {
   /* FP64 geometry */
   std::vector<DevBuf*> owned;
   ptg::Geo64 g64;
+  bool persistent64 = false;  /* the bounds of the persistent FP64 kernels hold */
   /* FP32 blob */
   DevBuf blob;
   ptg::GeoF32 g32;
@@ -528,6 +529,22 @@ bool box_is_axis_aligned(const ptg::GeomSoA& G) {
   return true;
 }
 
+/* Whether the planes of the grains' polygons bound them: unit normals, every
+   vertex within eps of the plane through the first (the BVH's boxes hold the
+   vertices, padded by 4 eps).  The plain FP64 kernel's hits need neither. */
+bool polygons_are_flat(const ptg::GeomSoA& G) {
+  const double eps = std::max(G.box[0], std::max(G.box[1], G.box[2])) / 1048576.0;
+  for (int s = G.grain_begin[1]; s < G.nsurf(); ++s) {
+    if (G.shape[s] != PTG_SHAPE_POLYGON || !G.internal[s]) continue;
+    const double* n = &G.normal[3 * s];
+    const double* v = &G.vertex[3 * (size_t)G.vertex_begin[s]];
+    if (!(fabs(n[0] * n[0] + n[1] * n[1] + n[2] * n[2] - 1.0) <= 1e-6)) return false;
+    for (int k = 3; k < 3 * G.nvertex[s]; k += 3)
+      if (!(fabs(n[0] * (v[k] - v[0]) + n[1] * (v[k + 1] - v[1]) + n[2] * (v[k + 2] - v[2])) <= eps)) return false;
+  }
+  return true;
+}
+
 int build_geo64(ptg_handle* h) {
   const ptg::GeomSoA& G = h->geom;
   ptg::Geo64& g = h->g64;
@@ -558,7 +575,7 @@ int build_geo64(ptg_handle* h) {
   g.igrain_fill = G.igrain_fill;
   g.nmaterial = G.nmaterial;
   g.max_omega = h->spec.max_omega;
-  g.box_axis = box_is_axis_aligned(G) ? 1 : 0;
+  h->persistent64 = box_is_axis_aligned(G) && polygons_are_flat(G);
   return PTG_OK;
 }
 
@@ -626,7 +643,9 @@ int run_transport(ptg_handle* h, const Transport& T) {
   const int64_t maxf = h->opt.max_flights > 0 ? h->opt.max_flights : 10000000LL;
   memset(&h->last, 0, sizeof(h->last));
   const bool fp64 = T.precision == PTG_PREC_FP64;
-  const bool plain = fp64 && (h->opt.tune_flags & 8);
+  /* the persistent FP64 kernels leave out what their bounds exclude; a caller's
+     geometry that the bounds do not describe runs as it is */
+  const bool plain = fp64 && ((h->opt.tune_flags & 8) || !h->persistent64);
   /* the task table and the queue order (longest expected trajectories first:
      ascending MFP) are written to pinned staging and copied without a host
      wait.  The MFP depends on (mode, grid point) only, so those pairs are

@@ -37,8 +37,6 @@ struct Geo64 {
   int face_kind[6];
   int kind_grain, ngrain, igrain_fill, nmaterial;
   double max_omega;
-  int box_axis;              /* grain 0 is the six axis-aligned rectangles of
-                                the box, every one internal                 */
 };
 
 /* Per task: lambda [nm] (1e10 ballistic, <= 0 skipped), cos/sin of the

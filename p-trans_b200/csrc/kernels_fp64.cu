@@ -585,10 +585,10 @@ __global__ void __launch_bounds__(128) k_plain_fp64(Geo64 g, Run64 r) {
    distance and tie (box before grain, then the lower index) as the linear
    scan.  What the scan does for every surface is left out where it cannot
    matter:
-     - box faces that the host found to be the axis-aligned rectangles they
-       are meant to be (Geo64.box_axis) are met at (face - x) / d, which is
-       the general formula's value with a normal of +-1 and zeros, and a hit
-       well inside the rectangle needs no edge test;
+     - the box faces, which the host found to be axis-aligned rectangles
+       (box_is_axis_aligned), are met at (face - x) / d, which is the general
+       formula's value with a normal of +-1 and zeros, and a hit well inside
+       the rectangle needs no edge test;
      - a plane crossed beyond the nearest hit so far is left early;
      - a grain with a BVH is walked in FP32: the node boxes are padded by 4 eps
        and positions rounded by 2^-24 of the box, so no node that holds the
@@ -600,34 +600,25 @@ __device__ bool nearest64(const Geo64& g, const Geo<false>& G, float eps, const 
                           int* igrain, int* isurf) {
   double best = fp < 1.0e10 ? __longlong_as_double(__double_as_longlong(fp) + 1) : 1.0e10;
   bool hit = false;
-  if (g.box_axis) {
-    const double m = (double)eps;
+  const double m = (double)eps;
 #pragma unroll
-    for (int ax = 0; ax < 3; ++ax) {
-      const double d = dir[ax];
-      const double w = (d > 0.0 ? g.box[ax] : 0.0) - pos[ax];
-      if (d == 0.0) continue;
-      if (d > 0.0 ? (w < 0.0 || w > best * d * 1.000001) : (w > 0.0 || w < best * d * 1.000001))
-        continue;
-      const double L = w / d;
-      if (!(best > L)) continue;
-      const int b = ax == 0 ? 1 : 0, c = ax == 2 ? 1 : 2;
-      const double hb = pos[b] + dir[b] * L, hc = pos[c] + dir[c] * L;
-      const int k = 2 * ax + (d > 0.0 ? 1 : 0);
-      bool in = hb > m && hb < g.box[b] - m && hc > m && hc < g.box[c] - m;
-      if (!in) {
-        const double Rh[3] = {pos[0] + dir[0] * L, pos[1] + dir[1] * L, pos[2] + dir[2] * L};
-        in = in_polygon(g.vertex + 3 * (size_t)g.vbegin[k], 4, Rh);
-      }
-      if (in) { best = L; *igrain = 0; *isurf = k; hit = true; }
+  for (int ax = 0; ax < 3; ++ax) {
+    const double d = dir[ax];
+    const double w = (d > 0.0 ? g.box[ax] : 0.0) - pos[ax];
+    if (d == 0.0) continue;
+    if (d > 0.0 ? (w < 0.0 || w > best * d * 1.000001) : (w > 0.0 || w < best * d * 1.000001))
+      continue;
+    const double L = w / d;
+    if (!(best > L)) continue;
+    const int b = ax == 0 ? 1 : 0, c = ax == 2 ? 1 : 2;
+    const double hb = pos[b] + dir[b] * L, hc = pos[c] + dir[c] * L;
+    const int k = 2 * ax + (d > 0.0 ? 1 : 0);
+    bool in = hb > m && hb < g.box[b] - m && hc > m && hc < g.box[c] - m;
+    if (!in) {
+      const double Rh[3] = {pos[0] + dir[0] * L, pos[1] + dir[1] * L, pos[2] + dir[2] * L};
+      in = in_polygon(g.vertex + 3 * (size_t)g.vbegin[k], 4, Rh);
     }
-  } else {
-    for (int k = 0; k < g.grain_begin[1]; ++k) {
-      double L;
-      if (g.internal[k] && surface_distance<true, EXT>(g, k, pos, dir, best, &L) && best > L) {
-        best = L; *igrain = 0; *isurf = k; hit = true;
-      }
-    }
+    if (in) { best = L; *igrain = 0; *isurf = k; hit = true; }
   }
   if (which > 0 && !box_only) {
     const int kb0 = g.grain_begin[which];

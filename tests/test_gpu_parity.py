@@ -315,6 +315,41 @@ def test_persistent_fp64_takes_the_plain_kernels_trajectories(k, mfp):
         assert got[1][1:] == got[0][1:], (name, opts)
 
 
+def _callers_geometries():
+    """Geometries of a caller's own that the FP32 bounds do not describe: the
+    x+ bath inside the box, facet normals of length 2, and facets behind a BVH
+    with a vertex 2 nm off their plane."""
+    bath = A.GeomBuf(synth.nanowire(length=100.0, width=80.0, height=80.0, p_side=0.3)).numpy()
+    v, b = bath["vertex"], int(bath["vertex_begin"][1])
+    v[3 * b:3 * (b + 5)].reshape(5, 3)[:, 0] *= 0.6
+    normals = A.GeomBuf(synth.cube_lattice(n=3, l=300.0, fill=0.4, trans=0.3, spec=0.0, p_wall=0.3)).numpy()
+    normals["normal"][3 * 6:] *= 2.0
+    bent = A.GeomBuf(synth.voronoi_box(4, box=(300.0, 250.0, 250.0), seed=5, trans=0.5, p_wall=0.3, tri_levels=2)).numpy()
+    for s in range(6, int(bent["nsurf"])):
+        k = int(bent["vertex_begin"][s]) + 2
+        bent["vertex"][3 * k:3 * k + 3] -= 2.0 * bent["normal"][3 * s:3 * s + 3]
+    return {"bath": bath, "normals": normals, "bent": bent}
+
+
+@pytest.mark.parametrize("name", ["bath", "normals", "bent"])
+def test_fp64_runs_of_a_callers_geometry_take_the_plain_kernels_trajectories(name):
+    """ptg_create takes any geometry whose records are in range.  Where the
+    bounds that the persistent FP64 kernels leave surfaces out by do not hold,
+    the counts are the plain kernel's (tune_flags bit 3) all the same."""
+    geom = A.numpy_to_geometry(_callers_geometries()[name])
+    spec = synth.spectrum(12, seed=3, mfp_lo=3e-9, mfp_hi=1e-7)
+    run = A.make_run(kind_mfp=A.MFP_PER_MODE, nangle=5, np_=200, seed=8, precision=A.PREC_FP64)
+    got = []
+    for flags in (8, 0):
+        with A.Handle(geom, spec, tune_flags=flags, max_flights=20000) as h:
+            k = h.kappa(run, want_counts=True)
+            st = h.stats()
+        got.append((k["counts"], st["lost"], st["flights"], st["capped"]))
+    np.testing.assert_array_equal(got[1][0], got[0][0])
+    assert got[1][1:] == got[0][1:]
+    assert got[0][0].sum() > 0
+
+
 @pytest.mark.parametrize("name", ["film_periodic", "brick_tris", "capped"])
 @pytest.mark.parametrize("np_", [3, 355, 356, 2400])
 @pytest.mark.parametrize("cap", [0, 17])

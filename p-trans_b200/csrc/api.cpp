@@ -847,7 +847,9 @@ int run_transport(ptg_handle* h, const Transport& T) {
       if (T.mode == ptg::MODE_FORWARD)
         r.grace_steps = ptg::grace_passes(norder * T.np_local, (int64_t)tgrid * (block / 32));
     }
-    if (h->g32.has_ext == ptg::kChunkTableExt && nchunk > 0) {
+    /* (the replays walk a list) */
+    if (h->g32.has_ext == ptg::kChunkTableExt && nchunk > 0 &&
+        (T.mode == ptg::MODE_FORWARD || T.mode == ptg::MODE_LIST)) {
       CU(h->chunk.ensure(sizeof(int4) * nchunk));
       r.chunk = h->chunk.as<const int4>();
       CU(ptg::launch_expand_chunks(chunks, (int)nchunk, h->chunk.as<int4>(), h->stream));

@@ -267,3 +267,17 @@ def test_scale_derivative_keeps_its_summation(name):
             run = A.make_run(kind_mfp=A.MFP_PER_MODE, nangle=7, np_=40, seed=seed)
             got = np.median([h.adjoint(run)["dk_dscale"] for _ in range(5)])
             assert abs(got - want) <= 3e-6 * abs(want), (seed, got)
+
+
+def test_replay_expands_no_chunk_table():
+    """Behind capped cylinders the listing pass expands a chunk table (a launch
+    of its own); the replay walks the list and launches drain, order and tail."""
+    m = synth.spheres_cylinders_box(n_spheres=4, n_cylinders=5, l=300.0, seed=3, r_sphere=(15.0, 35.0),
+                                    r_cylinder=20.0, length=(50.0, 150.0), trans=0.3, p_wall=0.2)
+    gb = A.GeomBuf(m)
+    run = A.make_run(kind_mfp=A.MFP_PER_MODE, nangle=5, np_=50, seed=2)
+    with A.Handle(gb.view, synth.spectrum(8, seed=1, mfp_lo=20e-9, mfp_hi=2e-6)) as h:
+        assert h.adjoint(run)["replayed"] > 0
+        assert h.stats()["launches"] == 3
+        h.kappa(run)
+        assert h.stats()["launches"] == 6  # and two for the reduction

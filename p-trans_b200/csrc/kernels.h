@@ -45,6 +45,9 @@ struct Task64 {
   double lambda, cth, sth, omega;
 };
 
+/* Most facet planes of a grain: the tail phase's balls take one a lane. */
+constexpr int kMaxPlanes = 32;
+
 /* GeoF32.has_ext of the FP32 kernels that read a chunk table. */
 constexpr int kChunkTableExt = 1;
 

@@ -541,6 +541,7 @@ __device__ __forceinline__ void warp_min2(float& e, float& e2, int& s, int lane)
 
 /* safety() for a grain without a tree search (a linear candidate list, or
    facet planes): the lanes take a surface each.  Warp-collective. */
+static_assert(kMaxPlanes <= 32, "a facet plane per lane");
 template <int EXT, class G_t>
 __device__ __forceinline__ float safety_warp(const G_t& G, int grain, float px, float py, float pz,
                                              float X, float Y, float Z, float eps, int lane,

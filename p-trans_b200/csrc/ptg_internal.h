@@ -124,7 +124,6 @@ inline void tail_counts(const int* queue, int cap, uint64_t* handed, uint64_t* r
    (bvh_leaf < 0: none, linear candidate scans everywhere). */
 constexpr int kBvhMinCand = 32;
 constexpr int kBvhDefaultLeaf = 4;
-constexpr int kMaxPlanes = 32;
 int blob_from_geometry(const GeomSoA& G, int bvh_leaf, std::vector<float4>* out, BlobLayout* lay,
                        std::string* why);
 /* Binned-SAH BVH over boxes lo/hi (3 floats each): nodes (2 float4 each,

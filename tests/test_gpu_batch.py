@@ -144,3 +144,25 @@ def test_batched_scale_derivative_does_not_depend_on_the_tail_phase():
     assert np.all(se > 0.0)
     assert np.all(np.abs(got[1]["dk_dscale"] - got[0]["dk_dscale"]) <= 1e-10 * se)
     np.testing.assert_allclose(got[1]["dk_dscale_stderr"], se, rtol=1e-10)
+
+
+@pytest.mark.parametrize("mfp", [(1e-9, 3e-8), (2e-8, 2e-6), None])
+def test_batch_with_facet_planes_equals_linear_scans(mfp):
+    """A convex mesh sends the whole batch to the kernels that use facet planes,
+    the film, the capped cylinders and the lattice with it: every structure gets
+    the counts of its own run without BVH and planes."""
+    spec = synth.spectrum(10, seed=6, mfp_lo=mfp[0], mfp_hi=mfp[1]) if mfp else synth.spectrum(10, seed=6)
+    kind = A.MFP_PER_MODE if mfp else A.MFP_MATTHIESSEN
+    bufs = [A.GeomBuf(m) for m in _unlike()]
+    nps, n = [37, 90, 44, 61], len(bufs)
+    run = A.make_run(kind_mfp=kind, nangle=5, np_=1)
+    with A.Batch([b.view for b in bufs], nps, [9 + i for i in range(n)], [0] * n, spec, run) as bt:
+        r = bt.run(want_counts=True)
+        replayed = bt.adjoint()["replayed"]
+    for g in range(n):
+        single = A.make_run(kind_mfp=kind, nangle=5, np_=nps[g], seed=9 + g)
+        with A.Handle(bufs[g].view, spec, bvh_leaf=-1) as h:
+            k = h.kappa(single, want_counts=True)
+        np.testing.assert_array_equal(r["counts"][g], k["counts"])
+        replayed -= int(k["counts"].sum())
+    assert replayed == 0

@@ -43,6 +43,15 @@ def test_noalloc_matches_transmission_on_consecutive_calls():
             assert np.all(want[:, :, -1] == 0.0) and want[:, :, :-1].sum() > 0
 
 
+@pytest.mark.parametrize("mfp", [3.0, 40.0, 1000.0])
+def test_noalloc_with_facet_planes_equals_the_linear_scan(mfp):
+    gb = A.GeomBuf(synth.voronoi_box(4, box=(300.0, 250.0, 250.0), seed=5, trans=0.5, p_wall=0.3, tri_levels=2))
+    spec = synth.spectrum(10, seed=2)
+    with A.Handle(gb.view, spec) as h, A.Handle(gb.view, spec, bvh_leaf=-1) as linear:
+        want, _ = linear.transmission(mfp, 7, 130, seed=3, precision=A.PREC_FP32)
+        np.testing.assert_array_equal(h.transmission_noalloc(mfp, 7, 130, seed=3), want)
+
+
 def test_noalloc_tail_list_overflow_keeps_every_phonon():
     """A strongly diffusive run (MFP 2 nm in a 145 nm film) with every lane
     refilled at once keeps more phonons alive when the work queue runs dry than

@@ -472,8 +472,8 @@ void ptg_batch_destroy(ptg_batch* b);
  * Bounds-checked build (no counterpart in the reference, whose debug aids
  * are its verbose self-checks, src/RTMCphon.f90:1695-1703, 1711-1731):
  * libptrans_b200_check.so, the same library built with -DPT_CHECK, checks
- * every geometry-blob index the FP32 kernels read (surfaces, edges,
- * candidates, BVH nodes) and that every live phonon's state is finite; a
+ * every geometry-blob index the persistent kernels of both precisions read
+ * (surfaces, edges, candidates, BVH nodes) and that every live phonon's state is finite; a
  * failed check is counted, its access redirected to a valid element, and
  * the kernel goes on (it never traps).  ptg_check_report returns, for a
  * device, the number of failed checks since the last reset, the code of the

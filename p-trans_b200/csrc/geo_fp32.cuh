@@ -21,9 +21,22 @@ extern __shared__ float4 sblob[];
 
 #ifdef PT_CHECK
 /* Bounds-checked build: [0] violations, [1] code of the first, [2] its
-   index.  A failed check is recorded and the access is redirected to a
-   valid element; the kernel never traps. */
+   index, one set per file of kernels.  A failed check is recorded and the
+   access is redirected to a valid element; the kernel never traps. */
 __device__ int g_check[3];
+cudaError_t check_read(long long* count, int* code, int* index, bool reset) {
+  int v[3] = {0, 0, 0};
+  cudaError_t e = cudaMemcpyFromSymbol(v, g_check, sizeof(v));
+  if (e != cudaSuccess) return e;
+  *count = v[0];
+  *code = v[1];
+  *index = v[2];
+  if (reset) {
+    const int z[3] = {0, 0, 0};
+    e = cudaMemcpyToSymbol(g_check, z, sizeof(z));
+  }
+  return e;
+}
 __device__ __noinline__ void check_fail(int code, int index) {
   if (atomicAdd(&g_check[0], 1) == 0) {
     g_check[1] = code;

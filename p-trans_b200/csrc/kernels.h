@@ -320,6 +320,7 @@ inline size_t dynamic_smem_bytes(const GeoF32& g, size_t blob_bytes) {
 /* Violations recorded by the bounds-checked build (PT_CHECK); other builds
    return cudaErrorNotSupported. */
 cudaError_t check_report(long long* count, int* code, int* index, bool reset);
+cudaError_t check_report_fp64(long long* count, int* code, int* index, bool reset);
 /* Residency of the persistent kernel for a block size and shared memory. */
 cudaError_t persistent_occupancy(int block, size_t smem, int* blocks_per_sm,
                                  int mode = MODE_FORWARD, int ext = 0, bool whole = true);

@@ -2179,23 +2179,21 @@ cudaError_t launch_tail_order(const float4* tail, int units, int tail_cap, const
   return cudaGetLastError();
 }
 
-/* Violations recorded by a bounds-checked build (PT_CHECK): count, code of
+/* Violations recorded by a bounds-checked build (PT_CHECK) of both
+   precisions' kernels: count, code of
    the first (1 geometry-blob index out of range, 2 non-finite phonon state)
    and its index; reset = true clears them.  Other builds return
    cudaErrorNotSupported. */
 cudaError_t check_report(long long* count, int* code, int* index, bool reset) {
 #ifdef PT_CHECK
-  int v[3] = {0, 0, 0};
-  cudaError_t e = cudaMemcpyFromSymbol(v, g_check, sizeof(v));
+  const cudaError_t e = check_read(count, code, index, reset);
   if (e != cudaSuccess) return e;
-  *count = v[0];
-  *code = v[1];
-  *index = v[2];
-  if (reset) {
-    const int z[3] = {0, 0, 0};
-    e = cudaMemcpyToSymbol(g_check, z, sizeof(z));
-  }
-  return e;
+  long long n64 = 0;
+  int code64 = 0, index64 = 0;
+  const cudaError_t e64 = check_report_fp64(&n64, &code64, &index64, reset);
+  if (*count == 0) { *code = code64; *index = index64; }
+  *count += n64;
+  return e64;
 #else
   (void)count; (void)code; (void)index; (void)reset;
   return cudaErrorNotSupported;

@@ -733,6 +733,13 @@ __device__ __forceinline__ void unpack2(float4 v, double* a, double* b) {
   *b = __hiloint2double(__float_as_int(v.w), __float_as_int(v.z));
 }
 
+#ifdef PT_CHECK
+__device__ __noinline__ void check_finite64(const Ph64& p, int task) {
+  for (int d = 0; d < 3; ++d)
+    if (!isfinite(p.pos[d]) || !isfinite(p.dir[d]) || isnan(p.fp)) { check_fail(2, task); return; }
+}
+#endif
+
 /* ---- the two phases ---------------------------------------------------------
    The plain kernel is bound by latency: one lane per phonon, every flight a
    scan of all surfaces by divergent lanes (about 4 us a flight), to the end of
@@ -898,6 +905,9 @@ __global__ void __launch_bounds__(256, 2) k_drain64(Geo64 g, GeoF32 gp, Run64 r)
         }
       }
     }
+#ifdef PT_CHECK
+    if (alive) check_finite64(p, task);
+#endif
     const bool fin = alive && end_side >= 0;
     warp_add_by_task(fin && (end_side == 2 || (end_side == 0 && r.ref_quirks)), task, r.counts);
     warp_add_by_task(fin && end_side == 0, task, r.lost);
@@ -1089,6 +1099,9 @@ __global__ void __launch_bounds__(256, 2) k_tail64(Geo64 g, GeoF32 gp, Run64 r) 
         ball64<EXT>(G, gp, p.which, p.pos, (float)lambda, &bx, &by, &bz, &br2, &gr2);
       }
     }
+#ifdef PT_CHECK
+    if (lane == 0) check_finite64(p, task);
+#endif
     my_flights += flight;
     my_capped += capped ? 1 : 0;
     my_lost += end_side == 0 ? 1 : 0;
@@ -1146,5 +1159,11 @@ cudaError_t launch_tail64(const Geo64& g, const GeoF32& gp, const Run64& r, int 
   else k_tail64<0><<<grid, block, 0, st>>>(g, gp, r);
   return cudaGetLastError();
 }
+
+#ifdef PT_CHECK
+cudaError_t check_report_fp64(long long* count, int* code, int* index, bool reset) {
+  return check_read(count, code, index, reset);
+}
+#endif
 
 }  // namespace ptg

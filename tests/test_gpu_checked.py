@@ -41,3 +41,21 @@ def test_checked_build_finds_no_violation_and_matches_the_regular_build():
         assert checked[name]["counts"] == regular[name]["counts"], name
         assert checked[name]["flights"] == regular[name]["flights"], name
         assert checked[name]["mismatched"] == 0 and regular[name]["mismatched"] == 0
+
+
+def test_checked_build_covers_fp64_runs_and_batches():
+    """The same for the persistent FP64 kernels, which read the same blob, and
+    for a batch whose warps change structure from phonon to phonon."""
+    from ptrans_b200 import abi as A
+    got = []
+    for lib in (A.LIB_PATH, A.CHECK_LIB_PATH):
+        env = dict(os.environ, PTRANS_B200_LIB=lib)
+        p = subprocess.run([sys.executable, os.path.join(HERE, "checked_run_fp64.py")], capture_output=True,
+                           text=True, env=env, timeout=900)
+        assert p.returncode == 0, p.stderr[-3000:]
+        got.append(json.loads(p.stdout.strip().splitlines()[-1]))
+    assert got[0].pop("check") == {"status": A.PTG_ERR_UNSUPPORTED}
+    rep = got[1].pop("check")
+    assert rep["violations"] == 0, rep
+    assert got[1] == got[0]
+    assert got[0]["batch"][3] == 0

@@ -309,8 +309,10 @@ constexpr int kTailUnits = 7;
 constexpr int kTail64Units = 8;
 /* Shared memory for staged BVH nodes when the whole blob is not staged:
    64 KB, the top ten or so levels of the trees, small enough that two
-   blocks of the tail kernel (28.5 KB of its own) still fit on an SM. */
+   blocks of the tail kernel (kStaticSmem of its own at most) still fit on an
+   SM. */
 constexpr int kNodeStageUnits = 4096;
+constexpr size_t kStaticSmem = 27 * 1024;
 /* Dynamic shared memory of a transport launch: the whole blob, or the
    staged BVH nodes, or none. */
 inline size_t dynamic_smem_bytes(const GeoF32& g, size_t blob_bytes) {

@@ -1041,6 +1041,9 @@ __global__ void __launch_bounds__(kBlock,
   __shared__ float4 coop_ledge[kLW][3 * kList];
   __shared__ float4 coop_lball[kLW];
   __shared__ int4 coop_lmeta[kLW];  /* count, grain, kind (list_bvh) */
+  static_assert(sizeof(adj_sh) + sizeof(coop_rowf) + sizeof(coop_park) + sizeof(coop_list) + sizeof(coop_lplane) +
+                        sizeof(coop_ledge) + sizeof(coop_lball) + sizeof(coop_lmeta) + 64 <= kStaticSmem,
+                "static shared memory of a block");
   int* const lst = coop_list[kLW > 1 ? (threadIdx.x >> 5) : 0];
   float4* const lpl = coop_lplane[kLW > 1 ? (threadIdx.x >> 5) : 0];
   float4* const led = coop_ledge[kLW > 1 ? (threadIdx.x >> 5) : 0];
@@ -1973,8 +1976,7 @@ __global__ void __launch_bounds__(kBlock,
    every launch with a staged blob opts in to its dynamic size. */
 template <int MODE, int EXT, int PH, bool SMEM = true>
 cudaError_t allow_dynamic_smem(size_t smem) {
-  /* at most 27 KB of any kernel here is static */
-  if (smem <= 20 * 1024) return cudaSuccess;
+  if (smem + kStaticSmem <= 48 * 1024) return cudaSuccess;
   return cudaFuncSetAttribute(k_persistent<SMEM, MODE, false, EXT, PH>,
                               cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
 }

@@ -664,7 +664,9 @@ __device__ __forceinline__ void scan_list(const G_t& G, const int* lst, const fl
 }
 
 /* Adjoint accumulators of the sample: dlogP/dp of surface k goes to
-   base + k, in shared memory (sh) when the block holds them, else global. */
+   base + k, in shared memory (sh) when the block holds them, else global;
+   base < 0: nowhere (a lane that takes the event along with the one that
+   accumulates). */
 struct AdjAcc {
   double* sh;
   double* gl;
@@ -762,7 +764,7 @@ __device__ __forceinline__ int surface_hit(const G_t& G, float tb, int sb, float
     if (MODE == MODE_ADJOINT) {
       /* d log P / d p of the specular (1/p) or diffuse (-1/(1-p)) choice */
       const float pk = C0.w;
-      if (pk > 0.0f && pk < 1.0f) {
+      if (pk > 0.0f && pk < 1.0f && acc.base >= 0) {
         const double sc = (u0 <= pk) ? 1.0 / (double)pk : -1.0 / (1.0 - (double)pk);
         const double v = (double)acc.w * sc;
         const int idx = acc.base + sb;
@@ -1363,8 +1365,8 @@ __global__ void __launch_bounds__(kBlock,
        safe ball.  The first flight that hits a surface, leaves the box or
        reaches the cap ends the round; the flights before it are p-p events.
        A surface or side-face event is taken by the whole warp
-       (surface_hit) and the rounds go on from it; at a bath face (and in
-       the adjoint replay at any surface) the hit flight's Philox block and
+       (surface_hit; lane 0 adds its score in the adjoint replay) and the
+       rounds go on from it; at a bath face the hit flight's Philox block and
        nearest surface are handed to the phonon's lane, which processes the
        event below. */
     bool coop = false;       /* this lane was advanced cooperatively          */
@@ -1584,16 +1586,29 @@ __global__ void __launch_bounds__(kBlock,
                 sR.z = __shfl_sync(FULL, R.z, j); sR.w = __shfl_sync(FULL, R.w, j);
                 stb = __shfl_sync(FULL, tb, j);
                 ssb = __shfl_sync(FULL, sb, j);
-                if (MODE != MODE_ADJOINT && ssb > 1) {
+                if (ssb > 1) {
                   /* a surface or a side face, not a bath: every lane takes
                      the event (the same inputs, the same result) and the
                      rounds go on from it; a bath face ends the visit */
                   ++cfl;
                   ++ctaken;
-                  const AdjAcc none{nullptr, nullptr, 0.0f, 0, false};
+                  if (MODE == MODE_ADJOINT) {
+                    /* a path length sums up as if the event had ended the
+                       visit: carried over to a visit's end it would group
+                       the same flights otherwise (2e-5 of the derivative) */
+                    if (BATCH) {
+                      clen += stb;
+                    } else {
+                      adj_len = (adj_len + clen) + stb;
+                      clen = 0.0f;
+                      round = -1;
+                    }
+                  }
+                  const AdjAcc acc{adj_sh, r.adj, adj_w,
+                                   lane == 0 ? adj_off + adj_b * adj_stride : -1, adj_in_smem};
                   surface_hit<MODE, EXT>(G, stb, ssb, u23f(sR.x), u23f(sR.y), u23f(sR.z),
                                          u23f(sR.w), Y, Z, pmask, nmat, s3.w, clam, cfl, c1, cslo,
-                                         cshi, key, none, cpx, cpy, cpz, cdx, cdy, cdz, cfp, cgrain,
+                                         cshi, key, acc, cpx, cpy, cpz, cdx, cdy, cdz, cfp, cgrain,
                                          cgr2, cg2r2, clast);
                   cbr2 = 0.0f;
                   stop = 0;

@@ -994,12 +994,13 @@ __global__ void __launch_bounds__(kBlock,
      hold, a lane took 1.7 on the porous film (12.6 of its 32 lanes in the
      group), so it drew more than it used; one alone leaves the pipes waiting.
      Groups of 4 by halves / 3 by thirds / 2 by thirds / 1 by halves: film
-     16.06 / 15.67 / 15.72 / 16.65 ms, polycrystal 9.08 / 8.81 / 8.91 / 9.84,
-     64 films 22.4 / 21.1 / 21.1 / 21.8; with a BVH or capped cylinders 4 by
-     halves / 2 by thirds / 1 by thirds: 222.6 / 217.5 / 216.9 ms, their
-     adjoint 10.2 / 9.75 / 10.4. */
-  constexpr int kFastGroup = EXT ? 2 : 3;
-  constexpr int kFastShare = 3;
+     16.06 / 15.67 / 15.72 / 16.65 ms, polycrystal 9.08 / 8.81 / 8.91 / 9.84;
+     with a BVH or capped cylinders 4 by halves / 2 by thirds / 1 by thirds:
+     222.6 / 217.5 / 216.9 ms, their adjoint 10.2 / 9.75 / 10.4.  A batch, whose
+     lanes' geometries differ, keeps groups of 4 by halves: 64 films of 1e5 to
+     1e7 samples 99.2 ms, 3 by halves 100.9, 3 by thirds 104.1 (+- 0.3). */
+  constexpr int kFastGroup = BATCH ? 4 : EXT ? 2 : 3;
+  constexpr int kFastShare = BATCH ? 2 : 3;
   typename std::conditional<BATCH, GeoBatch, Geo<SMEM>>::type G;
   G.lay = gp.lay;
   G.base = gp.blob;

@@ -998,8 +998,13 @@ __global__ void __launch_bounds__(kBlock,
      with a BVH or capped cylinders 4 by halves / 2 by thirds / 1 by thirds:
      222.6 / 217.5 / 216.9 ms, their adjoint 10.2 / 9.75 / 10.4.  A batch, whose
      lanes' geometries differ, keeps groups of 4 by halves: 64 films of 1e5 to
-     1e7 samples 99.2 ms, 3 by halves 100.9, 3 by thirds 104.1 (+- 0.3). */
-  constexpr int kFastGroup = BATCH ? 4 : EXT ? 2 : 3;
+     1e7 samples 99.2 ms, 3 by halves 100.9, 3 by thirds 104.1 (+- 0.3).
+     The tail takes few of them, but how many are written out decides how its
+     rounds compile.  Behind a BVH whose blob is not staged, 4: lattices of
+     6^3 / 8^3 / 16^3 cubes 42.9 / 48.0 / 265 ms of tail against 50.8 / 53.5 /
+     275 with 2 (+- 1 to 2); with the blob staged 2: inclusions 104 against
+     113. */
+  constexpr int kFastGroup = BATCH || (PH == PH_TAIL && EXT == 1 && !SMEM) ? 4 : EXT ? 2 : 3;
   constexpr int kFastShare = BATCH ? 2 : 3;
   typename std::conditional<BATCH, GeoBatch, Geo<SMEM>>::type G;
   G.lay = gp.lay;

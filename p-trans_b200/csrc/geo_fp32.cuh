@@ -261,12 +261,15 @@ __device__ __forceinline__ float safety(const G_t& G, int grain, float px, float
    of a BVH grain that has them: a polygon is met only from behind (along its
    outward normal), so none is met up to fp.  The margin covers the polygons'
    distance from their plane (eps / 4), the tests' eps and the rounding of the
-   direction times fp.  This and the plane bounds of the balls replace nearly
+   direction times fp.  A ballistic flight (infinite, 1e10 in FP64) ends behind
+   none: 8000 ballistic phonons in a small mesh 0.48 -> 0.44 ms without asking.
+   This and the plane bounds of the balls replace nearly
    every tree walk in a polyhedral grain: 5 Voronoi grains as 43 000 triangles,
    2.5e6 phonons: 160 -> 54 ms (drain 60 -> 22, tail 93 -> 27). */
 template <class G_t>
 __device__ __forceinline__ bool behind_planes(const G_t& G, int grain, float px, float py, float pz,
                                               float dx, float dy, float dz, float fp, float eps) {
+  if (fp >= 1.0e10f) return false;
   const int kb = G.plane_begin(grain), ke = G.plane_begin(grain + 1);
   const float m = -fmaf(5.0e-7f, fp, 4.0f * eps);
   bool behind = ke > kb;

@@ -200,12 +200,13 @@ typedef struct ptg_options {
                             /*   bit 3: FP64 runs with the plain kernel, one    */
                             /*          phonon per thread (the comparator; the  */
                             /*          same trajectories)                      */
-  int32_t fast_steps;       /* a quarter of the most fast p-p flights a warp takes   */
-                            /* per iteration (it goes on only while a third of  */
-                            /* its live lanes can; FP64: half, past fast_steps; */
-                            /* 0 = 4 for structures without BVH or capped       */
-                            /* cylinders, 20 for the others, 8 in a batched     */
-                            /* launch)                                          */
+  int32_t fast_steps;       /* a quarter of the most fast p-p flights a warp    */
+                            /* takes per iteration, rounded up to whole groups  */
+                            /* of two or three (it goes on only while a third   */
+                            /* of its live lanes can; FP64: one by one, past    */
+                            /* fast_steps while half can; 0 = 4 for structures  */
+                            /* without BVH or capped cylinders, 20 for the      */
+                            /* others, 8 in a batched launch)                   */
   int32_t coop_lanes;       /* once the work queue is dry, a warp with at most  */
                             /* this many live phonons hands them over to the    */
                             /* tail phase, a second kernel that gives           */

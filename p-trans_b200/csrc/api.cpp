@@ -684,7 +684,7 @@ int run_transport(ptg_handle* h, const Transport& T) {
     }
   int64_t csz = h->opt.chunk > 0 ? h->opt.chunk : 64;
   int64_t per_task = T.np_local > 0 ? (T.np_local + csz - 1) / csz : 0;
-  /* FP64 runs take any size: larger chunks past a table of 1 GB */
+  /* FP64 runs take any size: larger chunks past 2^26 of them */
   while (fp64 && norder * per_task > (1LL << 26) && per_task > 1) {
     csz *= 2;
     per_task = (T.np_local + csz - 1) / csz;
@@ -745,7 +745,7 @@ int run_transport(ptg_handle* h, const Transport& T) {
       r.chunks = chunks;
       r.nchunk = (int32_t)nchunk;
       r.queue = d_queue;
-    r.tail_hist = d_hist;
+      r.tail_hist = d_hist;
       r.regen_threshold = regen_threshold;
       r.fast_steps = fast_steps;
       r.fast_lambda_max = fast_lambda_max;

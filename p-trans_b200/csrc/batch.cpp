@@ -10,8 +10,9 @@
  * geometries with very uneven sample counts and mean free paths share the
  * GPU without a tail per geometry.  Set-up builds every table once; each
  * ptg_batch_run replays one graph: clear the tallies, the batched transport
- * (drain phase, order, tail phase), the batched FP64 kappa reduction (effectiveMFP + the kappa sum,
- * :2418-2451, :2645-2755) and the copy of the results to pinned memory.
+ * (drain phase, order, tail phase), the batched FP64 kappa reduction
+ * (effectiveMFP + the kappa sum, :2418-2451, :2645-2755) and the copy of the
+ * results to pinned memory.
  */
 #include <cuda_runtime.h>
 #include <math.h>

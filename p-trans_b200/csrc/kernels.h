@@ -156,8 +156,9 @@ struct RunF32 {
   const float4* task;
   ChunkQueue chunks;          /* the chunks, longest expected trajectories first   */
   const int4* chunk;          /* their table (task, first local particle, count, 0),
-                                 read instead by batches and behind a BVH or with
-                                 capped cylinders (kChunkTableExt) */
+                                 read instead by batches and by the kernels for a
+                                 BVH or capped cylinders without facet planes
+                                 (kChunkTableExt) */
   int32_t nchunk;
   int64_t np;
   int32_t rank, nranks;
@@ -165,7 +166,8 @@ struct RunF32 {
   uint32_t max_flights;
   int32_t ref_quirks;
   int32_t regen_threshold;
-  int32_t fast_steps;         /* a quarter of the most ball flights per iteration (0: off) */
+  int32_t fast_steps;         /* a quarter of the most ball flights per iteration,
+                                 but for the last group's (0: off)                 */
   float fast_lambda_max;      /* tasks with a smaller MFP use the fast path           */
   int32_t coop_lanes;         /* once the queue is dry, a warp with at most this many
                                  live phonons moves them to the tail list, where
@@ -267,8 +269,6 @@ enum { MODE_FORWARD = 0, MODE_LIST = 1, MODE_ADJOINT = 2, MODE_TRACE = 3 };
 
 cudaError_t launch_persistent_fp32(const GeoF32& g, const RunF32& r, int grid, int block,
                                    size_t smem, cudaStream_t st, int mode = MODE_FORWARD);
-/* The tail phase after it (forward, list and adjoint modes): the phonons
-   the drain phase left in r.tail, one per warp. */
 /* Fills the chunk table of the queue's nchunk chunks. */
 cudaError_t launch_expand_chunks(const ChunkQueue& q, int nchunk, int4* chunks, cudaStream_t st);
 /* Orders the tail list for the tail phase, longest expected remaining walk
@@ -287,6 +287,8 @@ cudaError_t launch_drain64(const Geo64& g, const GeoF32& g32, const Run64& r, in
                            cudaStream_t st);
 cudaError_t launch_tail64(const Geo64& g, const GeoF32& g32, const Run64& r, int grid, int block,
                           cudaStream_t st);
+/* The FP32 tail phase (forward, list and adjoint modes): the phonons the drain
+   phase left in r.tail, one per warp. */
 cudaError_t launch_tail_fp32(const GeoF32& g, const RunF32& r, int grid, int block, size_t smem,
                              cudaStream_t st, int mode = MODE_FORWARD);
 cudaError_t tail_occupancy(int block, size_t smem, int* blocks_per_sm, int mode = MODE_FORWARD,

@@ -31,10 +31,11 @@
  *     about (d/MFP)^2 flights, which shortens the serial chain of the longest
  *     trajectories that bound the kernel's run time.  A warp takes fast
  *     flights in groups of two or three, after the first only while a third
- *     of its live lanes are still in their balls and at most 4 fast_steps of
- *     them, so lanes that need a full flight are not held back.  With the ball the lane keeps a second radius about the
- *     same centre, over the grain's candidate surfaces alone (the grain
- *     ball): a flight inside it needs only the box-face test;
+ *     of its live lanes are still in their balls and no group from 4
+ *     fast_steps flights on, so lanes that need a full flight are not held
+ *     back.  With the ball the lane keeps a second radius about the same
+ *     centre, over the grain's candidate surfaces alone (the grain ball): a
+ *     flight inside it needs only the box-face test;
  *   - one Philox4x32-10 block per free flight supplies the four uniforms of
  *     any event; on the fast path the blocks of a group's flights are
  *     computed together so that independent chains fill the issue slots; tallies
@@ -590,10 +591,11 @@ __device__ __forceinline__ float safety_list(const G_t& G, const int* lst, int n
     s = lst[lane];
     e = fabsf(surface_lb<EXT>(G, s, px, py, pz));
   }
-  /* by shuffles in the kernels with EXT 1, where that measured faster: 64 spheres with 16 capped cylinders,
-     2e7 phonons, 206.8 ms (mean of 5) against 215.4 with the two minima,
-     43 008 triangles with facet planes (EXT 2) 51.0 against 52.3 the other
-     way round */
+  /* by shuffles in the kernels with EXT 1: the tails of four structures of
+     spheres and capped cylinders take 104.5, 88.2, 49.2 and 69.9 ms (means of
+     24 runs, +- 1 to 5) against 112.6, 95.5, 48.9 and 75.4 with the two
+     minima.  With EXT 2 the minima: 43 008 triangles with facet planes, which
+     take no list balls, 25.6 against 26.9 (+- 0.4) all the same */
   if (EXT == 1) {
     for (int o = 16; o > 0; o >>= 1) {
       const float oe = __shfl_xor_sync(FULL, e, o), oe2 = __shfl_xor_sync(FULL, e2, o);
@@ -1181,7 +1183,7 @@ __global__ void __launch_bounds__(kBlock,
                arithmetic costs the kernel registers: with it behind a BVH
                the spills of the drain grow from 104 to 120 bytes read, and
                64 spheres with 16 capped cylinders, 2e7 phonons, take 107.0
-               ms of drain against 104.1 */
+               ms of drain against 103.9 (+- 0.04) */
             if (BATCH || EXT == kChunkTableExt) {
               const int4 q = r.chunk[c];
               ch_task = q.x; ch_next = q.y; ch_left = q.z;

@@ -324,7 +324,14 @@ inline size_t dynamic_smem_bytes(const GeoF32& g, size_t blob_bytes) {
 /* Violations recorded by the bounds-checked build (PT_CHECK); other builds
    return cudaErrorNotSupported. */
 cudaError_t check_report(long long* count, int* code, int* index, bool reset);
+cudaError_t check_report_planes(long long* count, int* code, int* index, bool reset);
+cudaError_t check_report_batch(long long* count, int* code, int* index, bool reset);
 cudaError_t check_report_fp64(long long* count, int* code, int* index, bool reset);
+/* The part of the FP32 kernels built for facet planes, behind
+   launch_persistent_fp32, launch_tail_fp32 and their occupancies. */
+cudaError_t planes_occupancy(int block, size_t smem, int* blocks_per_sm, int mode, bool whole, bool tail);
+cudaError_t launch_planes(const GeoF32& g, const RunF32& r, int grid, int block, size_t smem, cudaStream_t st,
+                          int mode, bool tail);
 /* Residency of the persistent kernel for a block size and shared memory. */
 cudaError_t persistent_occupancy(int block, size_t smem, int* blocks_per_sm,
                                  int mode = MODE_FORWARD, int ext = 0, bool whole = true);

@@ -50,6 +50,12 @@
  *     every path (fast, full, cooperative) moves the position with the same
  *     fma and takes events with the same code, so a trajectory is the same
  *     whichever path takes its flights.
+ *
+ * Compiled three times (PT_PART): 0 single structures, 1 those with facet
+ * planes, 2 batches.  CUDA loads a file's kernels when the first of them is
+ * used, and a program seldom uses more than one of the three: the first run of
+ * a process (a gray film) takes 23 ms with all of them in one file, 6.5 ms as
+ * they are.
  */
 #include <cuda_runtime.h>
 #include <math.h>
@@ -77,6 +83,7 @@ __device__ __forceinline__ void sincos2pi(float u, float* s, float* c) {
   *c = -__cosf(a);
 }
 
+#if PT_PART == 2
 /* Geometry accessor of a batched launch: each lane reads the blob of its own
    geometry from global memory. */
 struct GeoBatch {
@@ -111,6 +118,9 @@ struct GeoBatch {
   __device__ __forceinline__ float4 plane(int i) const { return ld(lay.plane + i); }
   __device__ __forceinline__ float4 node(int i) const { return ld(lay.bvh_node + i); }
 };
+#else
+using GeoBatch = Geo<false>;  /* no batches in this part */
+#endif
 
 /* Point (x, y, z) on a polygon's plane against its edge half-spaces m
    (unit normal in the plane, pointing in, offset m.w), within eps. */
@@ -1992,8 +2002,6 @@ __global__ void __launch_bounds__(kBlock,
   }
 }
 
-}  // namespace
-
 /* Static shared memory (the adjoint accumulators, the cooperative rows) plus
    the staged blob can pass the 48 KB a launch gets without opting in, so
    every launch with a staged blob opts in to its dynamic size. */
@@ -2039,6 +2047,32 @@ cudaError_t launch_mode(const GeoF32& g, const RunF32& r, int grid, int block, s
   return cudaGetLastError();
 }
 
+/* The tail phase exists for the modes with cooperative rounds (forward,
+   list, adjoint replay); a trace replay runs every flight on one lane. */
+template <int EXT, int PH>
+cudaError_t occupancy_bvh(int block, size_t smem, int* bps, int mode, bool whole) {
+  if (mode == MODE_LIST) return occupancy_mode<MODE_LIST, EXT, PH>(block, smem, bps, whole);
+  if (mode == MODE_ADJOINT) return occupancy_mode<MODE_ADJOINT, EXT, PH>(block, smem, bps, whole);
+  if (mode == MODE_TRACE) {
+    if (PH == PH_TAIL) return cudaErrorInvalidValue;
+    return occupancy_mode<MODE_TRACE, EXT, PH_DRAIN>(block, smem, bps, whole);
+  }
+  return occupancy_mode<MODE_FORWARD, EXT, PH>(block, smem, bps, whole);
+}
+
+template <int EXT, int PH>
+cudaError_t launch_bvh(const GeoF32& g, const RunF32& r, int grid, int block, size_t smem,
+                       cudaStream_t st, int mode) {
+  if (mode == MODE_LIST) return launch_mode<MODE_LIST, EXT, PH>(g, r, grid, block, smem, st);
+  if (mode == MODE_ADJOINT) return launch_mode<MODE_ADJOINT, EXT, PH>(g, r, grid, block, smem, st);
+  if (mode == MODE_TRACE) {
+    if (PH == PH_TAIL) return cudaErrorInvalidValue;
+    return launch_mode<MODE_TRACE, EXT, PH_DRAIN>(g, r, grid, block, smem, st);
+  }
+  return launch_mode<MODE_FORWARD, EXT, PH>(g, r, grid, block, smem, st);
+}
+
+#if PT_PART == 2
 template <int MODE, int PH>
 cudaError_t batch_occupancy_mode(int block, int* bps, int ext) {
   return cudaOccupancyMaxActiveBlocksPerMultiprocessor(
@@ -2055,11 +2089,6 @@ cudaError_t batch_occupancy_phase(int block, int* bps, int ext, int mode) {
   if (mode == MODE_ADJOINT) return batch_occupancy_mode<MODE_ADJOINT, PH>(block, bps, ext);
   if (mode != MODE_FORWARD) return cudaErrorInvalidValue;
   return batch_occupancy_mode<MODE_FORWARD, PH>(block, bps, ext);
-}
-
-cudaError_t persistent_batch_occupancy(int block, int* bps, int ext, int mode, bool tail) {
-  return tail ? batch_occupancy_phase<PH_TAIL>(block, bps, ext, mode)
-              : batch_occupancy_phase<PH_DRAIN>(block, bps, ext, mode);
 }
 
 template <int MODE, int PH>
@@ -2082,55 +2111,29 @@ cudaError_t launch_batch_phase(const RunF32& r, int grid, int block, cudaStream_
   return launch_batch_mode<MODE_FORWARD, PH>(r, grid, block, st, ext);
 }
 
-cudaError_t launch_persistent_batch(const RunF32& r, int grid, int block, cudaStream_t st, int ext,
-                                    int mode, bool tail) {
-  return tail ? launch_batch_phase<PH_TAIL>(r, grid, block, st, ext, mode)
-              : launch_batch_phase<PH_DRAIN>(r, grid, block, st, ext, mode);
-}
+#endif
 
-/* The tail phase exists for the modes with cooperative rounds (forward,
-   list, adjoint replay); a trace replay runs every flight on one lane. */
-template <int EXT, int PH>
-cudaError_t occupancy_bvh(int block, size_t smem, int* bps, int mode, bool whole) {
-  if (mode == MODE_LIST) return occupancy_mode<MODE_LIST, EXT, PH>(block, smem, bps, whole);
-  if (mode == MODE_ADJOINT) return occupancy_mode<MODE_ADJOINT, EXT, PH>(block, smem, bps, whole);
-  if (mode == MODE_TRACE) {
-    if (PH == PH_TAIL) return cudaErrorInvalidValue;
-    return occupancy_mode<MODE_TRACE, EXT, PH_DRAIN>(block, smem, bps, whole);
-  }
-  return occupancy_mode<MODE_FORWARD, EXT, PH>(block, smem, bps, whole);
-}
+}  // namespace
 
+#if PT_PART == 0
 cudaError_t persistent_occupancy(int block, size_t smem, int* bps, int mode, int ext, bool whole) {
-  return ext == 2   ? occupancy_bvh<2, PH_DRAIN>(block, smem, bps, mode, whole)
-         : ext == 1 ? occupancy_bvh<1, PH_DRAIN>(block, smem, bps, mode, whole)
-                    : occupancy_bvh<0, PH_DRAIN>(block, smem, bps, mode, whole);
+  if (ext == 2) return planes_occupancy(block, smem, bps, mode, whole, false);
+  return ext == 1 ? occupancy_bvh<1, PH_DRAIN>(block, smem, bps, mode, whole)
+                  : occupancy_bvh<0, PH_DRAIN>(block, smem, bps, mode, whole);
 }
 
 cudaError_t tail_occupancy(int block, size_t smem, int* bps, int mode, int ext, bool whole) {
-  return ext == 2   ? occupancy_bvh<2, PH_TAIL>(block, smem, bps, mode, whole)
-         : ext == 1 ? occupancy_bvh<1, PH_TAIL>(block, smem, bps, mode, whole)
-                    : occupancy_bvh<0, PH_TAIL>(block, smem, bps, mode, whole);
-}
-
-template <int EXT, int PH>
-cudaError_t launch_bvh(const GeoF32& g, const RunF32& r, int grid, int block, size_t smem,
-                       cudaStream_t st, int mode) {
-  if (mode == MODE_LIST) return launch_mode<MODE_LIST, EXT, PH>(g, r, grid, block, smem, st);
-  if (mode == MODE_ADJOINT) return launch_mode<MODE_ADJOINT, EXT, PH>(g, r, grid, block, smem, st);
-  if (mode == MODE_TRACE) {
-    if (PH == PH_TAIL) return cudaErrorInvalidValue;
-    return launch_mode<MODE_TRACE, EXT, PH_DRAIN>(g, r, grid, block, smem, st);
-  }
-  return launch_mode<MODE_FORWARD, EXT, PH>(g, r, grid, block, smem, st);
+  if (ext == 2) return planes_occupancy(block, smem, bps, mode, whole, true);
+  return ext == 1 ? occupancy_bvh<1, PH_TAIL>(block, smem, bps, mode, whole)
+                  : occupancy_bvh<0, PH_TAIL>(block, smem, bps, mode, whole);
 }
 
 cudaError_t launch_persistent_fp32(const GeoF32& g, const RunF32& r, int grid, int block,
                                    size_t smem, cudaStream_t st, int mode) {
   if (block > kBlock || block % 32) return cudaErrorInvalidConfiguration;
-  return g.has_ext == 2   ? launch_bvh<2, PH_DRAIN>(g, r, grid, block, smem, st, mode)
-         : g.has_ext == 1 ? launch_bvh<1, PH_DRAIN>(g, r, grid, block, smem, st, mode)
-                          : launch_bvh<0, PH_DRAIN>(g, r, grid, block, smem, st, mode);
+  if (g.has_ext == 2) return launch_planes(g, r, grid, block, smem, st, mode, false);
+  return g.has_ext == 1 ? launch_bvh<1, PH_DRAIN>(g, r, grid, block, smem, st, mode)
+                        : launch_bvh<0, PH_DRAIN>(g, r, grid, block, smem, st, mode);
 }
 
 cudaError_t launch_tail_fp32(const GeoF32& g, const RunF32& r, int grid, int block, size_t smem,
@@ -2141,67 +2144,9 @@ cudaError_t launch_tail_fp32(const GeoF32& g, const RunF32& r, int grid, int blo
      copy would take that L1 from them */
   GeoF32 gt = g;
   gt.node_stage = 0;
-  return g.has_ext == 2   ? launch_bvh<2, PH_TAIL>(gt, r, grid, block, smem, st, mode)
-         : g.has_ext == 1 ? launch_bvh<1, PH_TAIL>(gt, r, grid, block, smem, st, mode)
-                          : launch_bvh<0, PH_TAIL>(gt, r, grid, block, smem, st, mode);
-}
-
-namespace {
-/* Hand-over c of the tail list: its slot (front list, then back list). */
-__device__ __forceinline__ int tail_slot(int c, int nlong, int tail_cap) {
-  return c < nlong ? c : tail_cap - 1 - (c - nlong);
-}
-
-/* One thread per hand-over: the bucket offsets from the top bucket down
-   (every block from the histogram), then the slot to its bucket's range. */
-__global__ void k_order_scatter(const float4* __restrict__ tail, int units, int tail_cap,
-                                const int* __restrict__ queue, const int* __restrict__ hist,
-                                int* __restrict__ cursor, int* __restrict__ order) {
-  __shared__ int h[kOrderBuckets];
-  const int nlong = min(queue[2], tail_cap);
-  const int ntail = nlong + min(queue[4], tail_cap - nlong);
-  if ((int)(blockIdx.x * blockDim.x) >= ntail) return;
-  for (int b = threadIdx.x; b < kOrderBuckets; b += blockDim.x) h[b] = hist[b];
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    int run = 0;
-    for (int b = kOrderBuckets - 1; b >= 0; --b) {
-      const int n = h[b];
-      h[b] = run;
-      run += n;
-    }
-  }
-  __syncthreads();
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= ntail) return;
-  const int slot = tail_slot(c, nlong, tail_cap);
-  const int b = reinterpret_cast<const int*>(tail + (size_t)units * slot + 6)[2];
-  order[h[b] + atomicAdd(&cursor[b], 1)] = slot;
-}
-}  // namespace
-
-/* Chunk table of a run whose kernels read one (kChunkTableExt). */
-__global__ void k_expand_chunks(const ChunkQueue q, int nchunk, int4* __restrict__ chunks) {
-  for (long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x; c < nchunk;
-       c += (long long)gridDim.x * blockDim.x) {
-    const int3 v = queue_chunk(q, (int)c);
-    chunks[c] = make_int4(v.x, v.y, v.z, 0);
-  }
-}
-
-cudaError_t launch_expand_chunks(const ChunkQueue& q, int nchunk, int4* chunks, cudaStream_t st) {
-  if (nchunk <= 0) return cudaSuccess;
-  const int blocks = (nchunk + 255) / 256;
-  k_expand_chunks<<<blocks < 4096 ? blocks : 4096, 256, 0, st>>>(q, nchunk, chunks);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_tail_order(const float4* tail, int units, int tail_cap, const int* queue,
-                              int32_t* order, int32_t* hist, cudaStream_t st) {
-  const unsigned blocks = (unsigned)((tail_cap + 255) / 256);
-  k_order_scatter<<<blocks, 256, 0, st>>>(tail, units, tail_cap, queue, hist, hist + kOrderBuckets,
-                                          order);
-  return cudaGetLastError();
+  if (g.has_ext == 2) return launch_planes(gt, r, grid, block, smem, st, mode, true);
+  return g.has_ext == 1 ? launch_bvh<1, PH_TAIL>(gt, r, grid, block, smem, st, mode)
+                        : launch_bvh<0, PH_TAIL>(gt, r, grid, block, smem, st, mode);
 }
 
 /* Violations recorded by a bounds-checked build (PT_CHECK) of both
@@ -2213,16 +2158,54 @@ cudaError_t check_report(long long* count, int* code, int* index, bool reset) {
 #ifdef PT_CHECK
   const cudaError_t e = check_read(count, code, index, reset);
   if (e != cudaSuccess) return e;
-  long long n64 = 0;
-  int code64 = 0, index64 = 0;
-  const cudaError_t e64 = check_report_fp64(&n64, &code64, &index64, reset);
-  if (*count == 0) { *code = code64; *index = index64; }
-  *count += n64;
-  return e64;
+  for (auto report : {check_report_planes, check_report_batch, check_report_fp64}) {
+    long long n = 0;
+    int c = 0, i = 0;
+    const cudaError_t er = report(&n, &c, &i, reset);
+    if (er != cudaSuccess) return er;
+    if (*count == 0) { *code = c; *index = i; }
+    *count += n;
+  }
+  return cudaSuccess;
 #else
   (void)count; (void)code; (void)index; (void)reset;
   return cudaErrorNotSupported;
 #endif
 }
+#elif PT_PART == 1
+cudaError_t planes_occupancy(int block, size_t smem, int* bps, int mode, bool whole, bool tail) {
+  return tail ? occupancy_bvh<2, PH_TAIL>(block, smem, bps, mode, whole)
+              : occupancy_bvh<2, PH_DRAIN>(block, smem, bps, mode, whole);
+}
+
+cudaError_t launch_planes(const GeoF32& g, const RunF32& r, int grid, int block, size_t smem, cudaStream_t st,
+                          int mode, bool tail) {
+  return tail ? launch_bvh<2, PH_TAIL>(g, r, grid, block, smem, st, mode)
+              : launch_bvh<2, PH_DRAIN>(g, r, grid, block, smem, st, mode);
+}
+
+#ifdef PT_CHECK
+cudaError_t check_report_planes(long long* count, int* code, int* index, bool reset) {
+  return check_read(count, code, index, reset);
+}
+#endif
+#else
+cudaError_t persistent_batch_occupancy(int block, int* bps, int ext, int mode, bool tail) {
+  return tail ? batch_occupancy_phase<PH_TAIL>(block, bps, ext, mode)
+              : batch_occupancy_phase<PH_DRAIN>(block, bps, ext, mode);
+}
+
+cudaError_t launch_persistent_batch(const RunF32& r, int grid, int block, cudaStream_t st, int ext,
+                                    int mode, bool tail) {
+  return tail ? launch_batch_phase<PH_TAIL>(r, grid, block, st, ext, mode)
+              : launch_batch_phase<PH_DRAIN>(r, grid, block, st, ext, mode);
+}
+
+#ifdef PT_CHECK
+cudaError_t check_report_batch(long long* count, int* code, int* index, bool reset) {
+  return check_read(count, code, index, reset);
+}
+#endif
+#endif
 
 }  // namespace ptg

@@ -744,11 +744,12 @@ __device__ __noinline__ void check_finite64(const Ph64& p, int task) {
    The plain kernel is bound by latency: one lane per phonon, every flight a
    scan of all surfaces by divergent lanes (about 4 us a flight), to the end of
    the longest trajectory.  Porous film, 2000 modes from 5 nm, 1e5 phonons:
-   plain 29.4 ms, here 3.4; wire 300 x 60 nm, MFPs from 2 nm, 1e5 phonons:
-   171 -> 7.9 ms; wire 1000 x 100 nm, gray MFP 150 nm, 3e4 phonons: 5.2 -> 2.9.
-   What bounds them now is the instructions of a round (about 2100 a warp, at
-   7 cycles each: fixed latencies of the FP64 chains, instruction fetch) times
-   the rounds of the longest walk. */
+   plain 27.8 ms, here 3.0; wire 300 x 60 nm, MFPs from 2 nm, 1e5 phonons:
+   141 -> 6.1 ms; wire 1000 x 100 nm, gray MFP 150 nm, 3e4 phonons: 5.2 -> 2.1.
+   What bounds them now is latency: 7 cycles a warp instruction in the tail
+   (2.6 of them fixed latencies of the FP64 chains, 1.2 instruction fetch; 22
+   lanes, SMs active for a quarter of it), times the rounds of the longest
+   walk. */
 
 /* Drain phase: the work queue, one phonon per lane, idle lanes refilled from
    the warp's chunk; flights that stay in the safe ball are taken without a

@@ -529,18 +529,24 @@ bool box_is_axis_aligned(const ptg::GeomSoA& G) {
   return true;
 }
 
-/* Whether the planes of the grains' polygons bound them: unit normals, every
-   vertex within eps of the plane through the first (the BVH's boxes hold the
-   vertices, padded by 4 eps).  The plain FP64 kernel's hits need neither. */
+/* Whether the planes of the grains' polygons bound them: unit normals, and in
+   grains that get a BVH, whose boxes hold the vertices padded by 4 eps, every
+   vertex within eps of the plane through the first.  The plain FP64 kernel's
+   hits need neither. */
 bool polygons_are_flat(const ptg::GeomSoA& G) {
   const double eps = std::max(G.box[0], std::max(G.box[1], G.box[2])) / 1048576.0;
-  for (int s = G.grain_begin[1]; s < G.nsurf(); ++s) {
-    if (G.shape[s] != PTG_SHAPE_POLYGON || !G.internal[s]) continue;
-    const double* n = &G.normal[3 * s];
-    const double* v = &G.vertex[3 * (size_t)G.vertex_begin[s]];
-    if (!(fabs(n[0] * n[0] + n[1] * n[1] + n[2] * n[2] - 1.0) <= 1e-6)) return false;
-    for (int k = 3; k < 3 * G.nvertex[s]; k += 3)
-      if (!(fabs(n[0] * (v[k] - v[0]) + n[1] * (v[k + 1] - v[1]) + n[2] * (v[k + 2] - v[2])) <= eps)) return false;
+  const int ngt = (int)G.grain_begin.size() - 1;
+  for (int g = 1; g < ngt; ++g) {
+    int ncand = 0;
+    for (int s = G.grain_begin[g]; s < G.grain_begin[g + 1]; ++s) ncand += G.internal[s] ? 1 : 0;
+    for (int s = G.grain_begin[g]; s < G.grain_begin[g + 1]; ++s) {
+      if (G.shape[s] != PTG_SHAPE_POLYGON || !G.internal[s]) continue;
+      const double* n = &G.normal[3 * s];
+      const double* v = &G.vertex[3 * (size_t)G.vertex_begin[s]];
+      if (!(fabs(n[0] * n[0] + n[1] * n[1] + n[2] * n[2] - 1.0) <= 1e-6)) return false;
+      for (int k = 3; ncand > ptg::kBvhMinCand && k < 3 * G.nvertex[s]; k += 3)
+        if (!(fabs(n[0] * (v[k] - v[0]) + n[1] * (v[k + 1] - v[1]) + n[2] * (v[k + 2] - v[2])) <= eps)) return false;
+    }
   }
   return true;
 }

@@ -440,20 +440,20 @@ def test_facet_planes_take_the_linear_scans_trajectories(levels, precision, mfp)
         assert g[1:] == got[0][1:]
 
 
-def _prism(sides, l=300.0, r=90.0):
-    """A prism of `sides` side faces in a box: quads and two fans of triangles,
-    a convex grain of sides + 2 planes behind a BVH; the matrix around it keeps
-    a BVH without planes."""
+def _prism(sides, levels=1, l=300.0, r=90.0):
+    """A prism of `sides` side faces in a box: a convex grain of sides + 2
+    planes behind a BVH (the matrix around it keeps a BVH without planes), its
+    faces as triangles `levels` times split, or as quads and fans (-1)."""
     th = 2 * math.pi * (np.arange(sides) + 0.5) / sides
     x, y = 0.5 * l + r * np.cos(th), 0.5 * l + r * np.sin(th)
-    ring = [[(x[i], y[i], z) for i in range(sides)] for z in (60.0, l - 60.0)]
-    faces = []
-    for i in range(sides):
-        k = (i + 1) % sides
-        faces.append([ring[0][i], ring[0][k], ring[1][k], ring[1][i]])
-    for i in range(1, sides - 1):
-        faces.append([ring[0][0], ring[0][i + 1], ring[0][i]])
-        faces.append([ring[1][0], ring[1][i], ring[1][i + 1]])
+    ring = [[np.array([x[i], y[i], z]) for i in range(sides)] for z in (60.0, l - 60.0)]
+    faces = [[ring[0][i], ring[0][(i + 1) % sides], ring[1][(i + 1) % sides], ring[1][i]] for i in range(sides)]
+    if levels >= 0:
+        faces += [ring[0][::-1], ring[1]]
+        faces = [t for f in faces for t in synth._triangulate(f, levels)]
+    else:
+        for i in range(1, sides - 1):
+            faces += [[ring[0][0], ring[0][i + 1], ring[0][i]], [ring[1][0], ring[1][i], ring[1][i + 1]]]
     m = synth.brick_box(l=l, t=0.4, p_wall=0.2)
     return dataclasses.replace(
         m, grain_generatrix=[0.5 * l] * 3, grain_nfacet=[len(faces)], facet_nvertex=[len(f) for f in faces],
@@ -461,13 +461,14 @@ def _prism(sides, l=300.0, r=90.0):
         surf_material_to=[A.MATERIAL_INTERNAL] * len(faces), surf_grain_to=[0] * len(faces))
 
 
-@pytest.mark.parametrize("sides,launches", [(29, 5), (30, 5), (31, 6)])
+@pytest.mark.parametrize("sides,levels,launches", [(29, 1, 5), (30, 1, 5), (31, 1, 6), (30, -1, 6), (30, 0, 6)])
 @pytest.mark.parametrize("precision", [A.PREC_FP32, A.PREC_FP64])
-def test_facet_planes_at_their_limit(sides, launches, precision):
+def test_facet_planes_at_their_limit(sides, levels, launches, precision):
     """Grains of 31 and 32 facet planes use them (the tail's balls take one a
-    lane), one of 33 keeps the tree searches alone, whose FP32 run expands a
-    chunk table: the counts of the linear scan each time."""
-    gb = A.GeomBuf(_prism(sides))
+    lane), one of 33 and one of few facets a plane keep the tree searches
+    alone, whose FP32 run expands a chunk table: the counts of the linear scan
+    each time."""
+    gb = A.GeomBuf(_prism(sides, levels))
     spec = synth.spectrum(12, seed=6, mfp_lo=2e-9, mfp_hi=3e-7)
     run = A.make_run(kind_mfp=A.MFP_PER_MODE, nangle=5, np_=61, seed=5, precision=precision)
     got = []

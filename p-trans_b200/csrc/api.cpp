@@ -726,11 +726,16 @@ int run_transport(ptg_handle* h, const Transport& T) {
   const int fast_steps = (h->opt.tune_flags & 1) ? 0 : (h->opt.fast_steps > 0 ? h->opt.fast_steps : ptg::default_fast_steps(h->g32));
   const double lmin = std::min(h->geom.box[0], std::min(h->geom.box[1], h->geom.box[2]));
   const float fast_lambda_max = (float)(0.1 * lmin);
+  const double longest = pairs.empty() ? 0.0 : (*T.tasks)[pairs.back()].lambda;
   /* tune_flags bit 1 turns the tail phase off; 0 selects 32 lanes (every
      diffusive phonon still alive when a warp finds the queue dry) */
   const int coop_lanes = (h->opt.tune_flags & 2) ? 0 : (h->opt.coop_lanes > 0 ? std::min(h->opt.coop_lanes, 32) : 32);
   const int bs = h->opt.block_size;
   const int block = (bs >= 32 && bs <= 256 && bs % 32 == 0) ? bs : 256;
+  auto grace = [&](int tail_blocks) {
+    return ptg::grace_passes(norder * T.np_local, (int64_t)tail_blocks * (block / 32), h->g32.lay.nbvh > 0, longest,
+                             lmin);
+  };
   if (fp64) {
     ptg::Run64 r;
     memset(&r, 0, sizeof(r));
@@ -781,7 +786,7 @@ int run_transport(ptg_handle* h, const Transport& T) {
         CU(h->tail.ensure((sizeof(float4) * ptg::kTail64Units + sizeof(int)) * (size_t)r.tail_cap));
         r.tail = h->tail.as<float4>();
         r.tail_order = reinterpret_cast<int*>(r.tail + (size_t)ptg::kTail64Units * r.tail_cap);
-        r.grace_steps = ptg::grace_passes(norder * T.np_local, (int64_t)tgrid * (block / 32));
+        r.grace_steps = grace(tgrid);
       }
       CU(ptg::launch_drain64(h->g64, h->g32, r, grid, block, h->stream));
       if (coop_lanes > 0) {
@@ -858,7 +863,7 @@ int run_transport(ptg_handle* h, const Transport& T) {
     if (tail) {
       tgrid = h->num_sms * std::max(h->occ_tail, 1);
       if (T.mode == ptg::MODE_FORWARD)
-        r.grace_steps = ptg::grace_passes(norder * T.np_local, (int64_t)tgrid * (block / 32));
+        r.grace_steps = grace(tgrid);
     }
     /* (the replays walk a list) */
     if (h->g32.has_ext == ptg::kChunkTableExt && nchunk > 0 &&

@@ -60,6 +60,8 @@ struct ptg_batch {
   Dev tail;
   int64_t samples = 0;
   int ext = 0;   /* which kernels its geometries need (GeoF32.has_ext) */
+  bool bvh = false;   /* one of them has a BVH */
+  double longest_mfp = 0.0, box_min = 0.0;   /* of all tasks, of all geometries */
   /* what the per-geometry adjoint needs besides the forward's tables */
   ptg::SpecSoA spec;
   ptg_run run;
@@ -106,7 +108,9 @@ static cudaError_t launch_phases(ptg_batch* b, ptg::RunF32 r, int mode) {
   const int tgrid = r.coop_lanes > 0 ? b->tail_grid[mode] : 0;
   if (tgrid == 0) r.coop_lanes = 0;
   r.grace_steps =
-      mode == ptg::MODE_FORWARD ? ptg::grace_passes(b->samples, (int64_t)tgrid * (block / 32)) : 0;
+      mode == ptg::MODE_FORWARD
+          ? ptg::grace_passes(b->samples, (int64_t)tgrid * (block / 32), b->bvh, b->longest_mfp, b->box_min)
+          : 0;
   cudaError_t e = cudaMemsetAsync(b->queue.p, 0, sizeof(int) * 8, b->stream);
   r.tail_hist = r.tail_order + r.tail_cap;
   if (e == cudaSuccess && tgrid > 0)
@@ -178,6 +182,7 @@ extern "C" int ptg_batch_create(const ptg_batch_item* items, int32_t nitems,
       ptg::GeoEntry& e = entries[g];
       memset(&e, 0, sizeof(e));
       e.lay = L;
+      b->bvh = b->bvh || L.nbvh > 0;
       if (L.nbvh > 0 || L.ncap > 0) b->ext = std::max(b->ext, L.nplane > 0 ? 2 : 1);
       for (int d = 0; d < 3; ++d) e.box[d] = (float)G.box[d];
       e.scope[0] = (float)G.scope[0];
@@ -186,6 +191,7 @@ extern "C" int ptg_batch_create(const ptg_batch_item* items, int32_t nitems,
       const double smin = std::min(G.box[0], std::min(G.box[1], G.box[2]));
       e.eps = (float)(smax * (1.0 / 1048576.0));
       e.fast_lambda_max = (float)(0.1 * smin);
+      b->box_min = g == 0 ? smin : std::min(b->box_min, smin);
       for (int f = 0; f < 6; ++f)
         if (G.face_kind[f] == PTG_FACE_PERIODIC) e.periodic_mask |= 1 << f;
       e.kind_grain = G.kind_grain;
@@ -228,6 +234,7 @@ extern "C" int ptg_batch_create(const ptg_batch_item* items, int32_t nitems,
       }
     }
     std::stable_sort(order.begin(), order.end(), [](const Order& a, const Order& c) { return a.lam < c.lam; });
+    if (!order.empty()) b->longest_mfp = order.back().lam;
     const int64_t csz = o.chunk > 0 ? o.chunk : 64;
     std::vector<int4> chunks;
     for (const Order& od : order) {

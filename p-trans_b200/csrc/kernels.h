@@ -250,13 +250,18 @@ inline int default_fast_steps(const GeoF32& g) {
    ballistic ones among spheres: 1107 -> 710 us) and go at once where it gets
    few (3200 phonons in a porous film, MFP 100 nm: 229 us against 248 with 16
    passes, 260 with 32).  The two are equal at 4 to 8 phonons per warp, and
-   16 and 32 passes at about 40; behind a BVH too (64 spheres and 16 capped
-   cylinders, 2e5 phonons, MFP 150 nm: 6.0 -> 3.1 ms).  The adjoint's two
-   passes hand over at once: their tail is a few long trajectories, which the
-   passes only delay (9.9 ms against 10.5 with 16). */
-inline int grace_passes(int64_t samples, int64_t tail_warps) {
-  if (samples < 6 * tail_warps) return 0;
-  return samples < 40 * tail_warps ? 16 : 32;
+   16 and 32 passes at about 40.  Behind a BVH a pass waits for 32 tree walks,
+   so the line lies higher (64 spheres and 16 capped cylinders, 2e5 phonons,
+   MFP 150 nm: 6.0 -> 3.1 ms, a mesh with 17 a warp, 2000 nm: 2.6 -> 2.1; but 14
+   a warp, ballistic: lattice of 5^3 cubes 2.27 ms against 2.00 without the
+   passes, a prism 0.55 against 0.46).  Below 40 the longest MFP also has to be
+   a quarter of the smallest box side: shorter ones outlive the passes (MFP 10
+   nm among a sphere and a cylinder, 14 a warp: 1.49 against 1.37 ms).  The
+   adjoint's two passes hand over at once: their tail is a few long
+   trajectories, which the passes only delay (9.9 ms against 10.5 with 16). */
+inline int grace_passes(int64_t samples, int64_t tail_warps, bool bvh, double longest_mfp, double box_min) {
+  if (samples >= 40 * tail_warps) return 32;
+  return samples >= (bvh ? 16 : 6) * tail_warps && longest_mfp >= 0.25 * box_min ? 16 : 0;
 }
 
 /* Replays are split in this many interleaved batches (sample % kAdjBatches)

@@ -209,7 +209,8 @@ extern "C" int ptg_transmission_noalloc(ptg_handle* h, double mfp_nm, int32_t na
     if (ptg::tail_occupancy(block, smem, &tbps, ptg::MODE_FORWARD, v.g32.has_ext, v.g32.stage_smem != 0) != cudaSuccess)
       return PTG_ERR_CUDA;
     tgrid = v.num_sms * (tbps < 1 ? 1 : tbps);
-    r.grace_steps = ptg::grace_passes(ntask * np_local, (int64_t)tgrid * (block / 32));
+    r.grace_steps = ptg::grace_passes(ntask * np_local, (int64_t)tgrid * (block / 32), v.g32.lay.nbvh > 0, mfp_nm,
+                                      std::min(v.g32.box[0], std::min(v.g32.box[1], v.g32.box[2])));
   }
   if (r.nchunk > 0) {
     if (ptg::launch_persistent_fp32(v.g32, r, grid, block, smem, s) != cudaSuccess)

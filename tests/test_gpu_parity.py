@@ -374,6 +374,23 @@ def test_long_mfp_phonons_end_alike_in_either_phase(name, np_, cap):
     assert got[1][1:] == got[0][1:]
 
 
+@pytest.mark.parametrize("np_,mfp", [(947, 90.0), (948, 90.0), (1000, 74.9), (1000, 75.1), (2400, 40.0)])
+@pytest.mark.parametrize("noalloc", [False, True])
+def test_long_mfp_phonons_behind_a_bvh_end_alike_in_either_phase(np_, mfp, noalloc):
+    """The same behind a BVH, where the line lies at 16 a tail warp, and on
+    either side of the MFP's, a quarter of the box: 40 tasks, a lattice of
+    triangulated cubes, T equal to the one-lane path's."""
+    gb = A.GeomBuf(geometries()["lattice_tris"])
+    spec = synth.spectrum(10, seed=8)
+    with A.Handle(gb.view, spec, tune_flags=2) as h:
+        want, _ = h.transmission(mfp, 5, np_, seed=31)
+        flights = h.stats()["flights"]
+    with A.Handle(gb.view, spec) as h:
+        got = h.transmission_noalloc(mfp, 5, np_, seed=31) if noalloc else h.transmission(mfp, 5, np_, seed=31)[0]
+        assert h.stats()["flights"] == flights
+    np.testing.assert_array_equal(got, want)
+
+
 def _many_spheres(n=40, l=400.0, seed=0):
     rng = np.random.default_rng(seed)
     c, r = [], []
